@@ -17,7 +17,9 @@
 //                         x-fwd -> y-fwd                       (z done inside CONV_FZ)
 //   signal:               x-fwd -> y-fwd -> z[fwd, (.)F, inv] -> y-inv -> x-inv(scale)
 // With the fused pass in the plan (N = 128, 256, 512), x-fwd -> y-fwd and y-inv -> x-inv
-// each run as one L2-staged launch. One cube of N <= 64 runs all of it in one cooperative
+// each run as one L2-staged launch. With the two-pass transform in the plan (N = 128, 256)
+// the passes are instead tiles of x and part of y, then tiles of the rest of y and z with the
+// product, then the mirror of the first (enqueue_tp). One cube of N <= 64 runs all of it in one cooperative
 // launch (persistent.cu: launch_small_conv).
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -197,6 +199,7 @@ static void teardown_locked() {
   release_uneven_plans();
   release_grouped_plans();
   release_xy_l2();
+  release_tp();
   g.ws.release();
   g.hfilt.release();
   for (auto &b : g.hreal) b.release();
@@ -352,7 +355,7 @@ static cudaError_t pass_xy(int n, const float2 *src, float2 *dst, int nvol, bool
     }
   }
   // the L2-staged pass is two launches: counter clear + pass
-  if (e == cudaSuccess) count_launches((tc_fused || get_pass_variant(n, kKindXy) == 1) ? 2 : 1);
+  if (e == cudaSuccess) count_launches((tc_fused || get_pass_variant(n, kKindXy) != 2) ? 2 : 1);
   return e;
 }
 
@@ -474,6 +477,104 @@ static cudaError_t enqueue_signals(int n, const float2 *sig, float2 *out, const 
   return cudaSuccess;
 }
 
+// ------------------------------------------------------------------ two-pass transform
+// True when FP32 calls of size n run the two-pass transform (plan kind kKindXy = 3).
+static bool use_tp(int n, int tc) {
+  return tp_size(n) && tma_enabled() && get_pass_variant(n, kKindXy) == kXyTwoPass && !tc_kernels(n, tc);
+}
+
+// One launch of the two-pass transform, profiled in the slot of the passes it replaces: the
+// outer passes as fused x+y passes with the bytes of an x and a y pass, the middle pass as
+// the fused z pass.
+template <class F>
+static cudaError_t pass_tp(int slot, double bytes, cudaStream_t s, F &&launch) {
+  NvtxRange nv(kSlotNames[slot]);
+  PassRec r{slot, bytes, nullptr, nullptr};
+  if (g_prof) {
+    cudaEventCreate(&r.a);
+    cudaEventCreate(&r.b);
+    cudaEventRecord(r.a, s);
+  }
+  const cudaError_t e = launch();
+  if (g_prof) {
+    cudaEventRecord(r.b, s);
+    if (e == cudaSuccess) {
+      g_prof_recs.push_back(r);
+    } else {
+      cudaEventDestroy(r.a);
+      cudaEventDestroy(r.b);
+    }
+  }
+  return e;
+}
+static cudaError_t tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, cudaStream_t s) {
+  return pass_tp(12, (real ? 28.0 : 32.0) * n * n * n * nvol, s,
+                 [&] { return launch_tp_fwd(n, src, dst, nvol, real, g.tw512, s); });
+}
+static cudaError_t tp_mid(int n, int mode, const float2 *src, float2 *dst, const float2 *filt, long long filt_vol,
+                          int nvol, cudaStream_t s) {
+  const int slot = 8 + (mode == kTpPair ? OP_CONV_FZ : (mode == kTpSpectrum ? OP_CONV : OP_FWD));
+  return pass_tp(slot, (mode == kTpFwd ? 16.0 : 24.0) * n * n * n * nvol, s,
+                 [&] { return launch_tp_mid(n, mode, src, dst, filt, filt_vol, nvol, g.tw512, s); });
+}
+static cudaError_t tp_inv(int n, const float2 *src, float2 *dst, int nvol, float scale, cudaStream_t s) {
+  return pass_tp(13, 32.0 * n * n * n * nvol, s, [&] { return launch_tp_inv(n, src, dst, nvol, scale, g.tw512, s); });
+}
+
+// Largest batch for which a shared filter's second pass runs inside every signal's middle
+// pass (TP_PAIR) instead of once before them (TP_FWD, then TP_SPECTRUM). Measured, us a
+// cube: 256^3 80 with it, 69 without and 46 once for the filter; 128^3 10, 8.1 and 6.
+constexpr unsigned kTpSharedPairMax = 3;
+
+// Convolutions by the two-pass transform. With a filter per signal and outputs of their own,
+// signals go through the outputs and back through the filters' workspace, all at once;
+// otherwise through the scratch cubes, as many at a time as there are. cudaErrorNotSupported, with
+// nothing enqueued, when an operand is not 16-byte aligned, when outputs overlap signals
+// without being them, or when there is no scratch.
+static cudaError_t enqueue_tp(int n, const float2 *sig, const float2 *filt, float2 *out, unsigned how_many,
+                              bool per_signal, bool real, float scale, float2 *ws, cudaStream_t s) {
+  const long long V = (long long)n * n * n;
+  const uintptr_t su = reinterpret_cast<uintptr_t>(sig), ou = reinterpret_cast<uintptr_t>(out),
+                  fu = reinterpret_cast<uintptr_t>(filt);
+  const uintptr_t bytes = (uintptr_t)V * how_many * sizeof(float2);
+  if ((su | ou | fu) & 15u) return cudaErrorNotSupported;
+  const bool overlap = su < ou + bytes && ou < su + bytes;
+  if (overlap && su != ou) return cudaErrorNotSupported;
+  const bool pairs = per_signal || how_many == 1;  // every filter serves one signal
+  const bool direct = pairs && !overlap;
+  float2 *scratch = tp_scratch(n, !capturing(s));
+  if (!direct && !scratch) return cudaErrorNotSupported;
+  if (direct) {
+    CG_TRY(tp_fwd(n, filt, ws, how_many, real, s));
+    CG_TRY(tp_fwd(n, sig, out, how_many, false, s));
+    CG_TRY(tp_mid(n, kTpPair, out, ws, ws, V, how_many, s));
+    CG_TRY(tp_inv(n, ws, out, how_many, scale, s));
+    return cudaSuccess;
+  }
+  const unsigned chunk = std::min<unsigned>(how_many, tp_scratch_cubes(n));
+  // Filters are read before any output is written: a caller may convolve into them.
+  const uintptr_t fbytes = (uintptr_t)V * (per_signal ? how_many : 1) * (real ? 4 : 8);
+  const bool filters_first = !per_signal || (fu < ou + bytes && ou < fu + fbytes);
+  const bool spectrum = !per_signal && how_many > kTpSharedPairMax;
+  if (filters_first) CG_TRY(tp_fwd(n, filt, ws, per_signal ? how_many : 1, real, s));
+  if (spectrum) CG_TRY(tp_mid(n, kTpFwd, ws, ws, nullptr, 0, 1, s));
+  for (unsigned i = 0; i < how_many; i += chunk) {
+    const int k = (int)std::min(chunk, how_many - i);
+    const float2 *f = ws;
+    if (per_signal) {
+      if (filters_first)
+        f = ws + i * V;
+      else
+        CG_TRY(tp_fwd(n, real ? (const void *)((const float *)(const void *)filt + i * V) : (const void *)(filt + i * V),
+                      ws, k, real, s));
+    }
+    CG_TRY(tp_fwd(n, sig + i * V, scratch, k, false, s));
+    CG_TRY(tp_mid(n, spectrum ? kTpSpectrum : kTpPair, scratch, scratch, f, per_signal ? V : 0, k, s));
+    CG_TRY(tp_inv(n, scratch, out + i * V, k, scale, s));
+  }
+  return cudaSuccess;
+}
+
 static int tc_of(unsigned flags) {
   // 0: FP32 kernels; 1 + split precision for the tensor-core path.
   return (flags & (kFlagTensorSplit | kFlagTensorBf16x3)) ? 1 + ((flags & kFlagTensorBf16x3) ? kTcBf16x3 : kTcTf32x3)
@@ -521,6 +622,11 @@ static cudaError_t enqueue_conv_device(unsigned n, const float2 *sig, const floa
     if (e != cudaSuccess) return e;
     const long long hv = (long long)n * n * half_spectrum_pitch((int)n);
     return enqueue_signals(n, sig, out, ws, per ? hv : 0, OP_CONV, how_many, scale, s, nullptr, 0, true);
+  }
+  if (use_tp((int)n, tc)) {
+    const cudaError_t e =
+        enqueue_tp((int)n, sig, filt, out, how_many, (flags & kFlagPerSignalFilter) != 0, real, scale, ws, s);
+    if (e != cudaErrorNotSupported) return e;
   }
   if (flags & kFlagPerSignalFilter) {
     cudaError_t e = enqueue_filter(n, filt, ws, how_many, true, s, tc, real);
@@ -1186,6 +1292,7 @@ struct TuneRow {
   int n;
   int choice[kPassKinds];
   double us[2][kPassKinds];
+  double us_two_pass;  // two-pass transform of a signal and its filter (N = 128, 256), else 0
 };
 static std::vector<TuneRow> g_tuned;
 
@@ -1204,6 +1311,7 @@ static bool write_plan_cache(const std::string &path) {
       for (int k = 0; k < kPassKinds; ++k) std::fprintf(f, "%.2f%s", r.us[v][k], k + 1 < kPassKinds ? ", " : "");
       std::fprintf(f, "]%s", v == 0 ? ", " : "");
     }
+    if (r.us_two_pass > 0.0) std::fprintf(f, ", \"us_two_pass\": %.2f", r.us_two_pass);
     std::fprintf(f, "}%s\n", i + 1 < g_tuned.size() ? "," : "");
   }
   std::fprintf(f, "}}\n");
@@ -1267,7 +1375,38 @@ int bridge_autotune(const unsigned *sizes, unsigned count, int write_cache) {
           }
         }
         row.choice[k] = row.us[1][k] < row.us[0][k] ? 1 : 0;
+        // The two-pass transform (variant 3) replaces all three axes: it is compared on a
+        // signal with its filter, against the faster of the others twice forward and once
+        // inverse and the fused z pass.
+        if (tp_size(n) && tma_enabled() && err == cudaSuccess) {
+          auto run = [&] {
+            cudaError_t r = launch_tp_fwd(n, data, spec, nvol, false, g.tw512, s);
+            if (r == cudaSuccess) r = launch_tp_fwd(n, data, spec, nvol, false, g.tw512, s);
+            if (r == cudaSuccess) r = launch_tp_mid(n, kTpPair, data, spec, spec, (long long)V, nvol, g.tw512, s);
+            return r == cudaSuccess ? launch_tp_inv(n, spec, data, nvol, 1.f, g.tw512, s) : r;
+          };
+          for (int w = 0; w < 2 && err == cudaSuccess; ++w) err = run();
+          cudaEventRecord(e0, s);
+          for (int t = 0; t < 5 && err == cudaSuccess; ++t) err = run();
+          cudaEventRecord(e1, s);
+          cudaEventSynchronize(e1);
+          float ms = 0.f;
+          cudaEventElapsedTime(&ms, e0, e1);
+          count_launches(28);
+          row.us_two_pass = 1000.0 * ms / 5.0;
+          if (err == cudaSuccess &&
+              row.us_two_pass < 3.0 * row.us[row.choice[k]][k] + row.us[row.choice[kKindConvFz]][kKindConvFz])
+            row.choice[k] = kXyTwoPass;
+          if (err == cudaErrorNotSupported) err = cudaSuccess;
+        }
         set_pass_variant(n, k, row.choice[k]);
+        continue;
+      }
+      if (k == kKindHalf && row.choice[kKindXy] == kXyTwoPass) {
+        // half spectra belong to the three-axis passes; not timed
+        for (int v = 0; v < 2; ++v) row.us[v][k] = 0.0;
+        row.choice[k] = 0;
+        set_pass_variant(n, k, 0);
         continue;
       }
       if (k == kKindHalf) {

@@ -3,6 +3,7 @@
 // (that header declares its own `float2`).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -47,6 +48,7 @@ cudaError_t launch_axis_pass_tc(int n, int axis, int op, const float2 *src, floa
 
 // Selects the TMA-fed y / z pass kernels (default) or the register-gather kernels.
 void set_tma_enabled(bool on);
+bool tma_enabled();
 
 // Twiddle buffer of the engine: 512 twiddles W512^j followed by the constant block of
 // the tcgen05 kernels (B operand hi / lo, W256^j), written by tc05_init_consts.
@@ -69,6 +71,41 @@ cudaError_t launch_xy_l2_tc_pass(int n, const float2 *src, float2 *dst, int npla
 int pass_kind(int axis, int op);
 void set_pass_variant(int n, int kind, int variant);
 int get_pass_variant(int n, int kind);
+// Plan kind kKindXy, variant 3 (N = 128 and 256): the two-pass 3D transform (twopass.cuh) in
+// place of the x, y and z passes, for the calls it takes; the others run variant 1.
+constexpr int kXyTwoPass = 3;
+bool tp_size(int n);
+// The middle pass's filter operand (twopass.cuh: TpMode).
+constexpr int kTpPair = 0, kTpSpectrum = 1, kTpFwd = 2;
+// Forward outer pass (cubes, or N^3 floats each with `real`, to tile order), middle pass, and
+// inverse outer pass (tile order to cubes). src and dst of the outer passes must not
+// overlap; the middle pass may write over its source or its filters. cudaErrorNotSupported
+// when an operand is not 16-byte aligned.
+cudaError_t launch_tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, const float2 *tw512,
+                          cudaStream_t s);
+cudaError_t launch_tp_mid(int n, int mode, const float2 *src, float2 *dst, const float2 *filt, long long filt_vol,
+                          int nvol, const float2 *tw512, cudaStream_t s);
+cudaError_t launch_tp_inv(int n, const float2 *src, float2 *dst, int nvol, float scale, const float2 *tw512,
+                          cudaStream_t s);
+// The same over cubes at unrelated addresses: device arrays of pointers and of tensor maps
+// (tp_encode_tiles of each cube in tile order). prepare_tp sets the kernels' attributes (call
+// it before a capture).
+bool tp_encode_tiles(CUtensorMap *m, const void *cubes, int n, int nvol);
+cudaError_t prepare_tp(int n);
+cudaError_t launch_tp_fwd_table(int n, const float2 *const *srcs, const CUtensorMap *dst_maps, int nvol,
+                                const float2 *tw512, cudaStream_t s);
+cudaError_t launch_tp_mid_table(int n, const float2 *const *srcs, float2 *const *dsts, const float2 *const *filts,
+                                int nvol, const float2 *tw512, cudaStream_t s);
+cudaError_t launch_tp_inv_table(int n, const CUtensorMap *src_maps, float2 *const *dsts, int nvol, float scale,
+                                const float2 *tw512, cudaStream_t s);
+// The process's scratch cubes in tile order, tp_scratch_cubes(n) of them (512 MiB): the
+// signals a call transforms at a time. Fewer cost more in launches than L2 gives back: a
+// call of 16 cubes of 128^3 took 403 us by 4, 357 by 8 and 339 at once. Null when not
+// allocated and not (or not to be) allocatable.
+constexpr int kTpScratchCubes128 = 32, kTpScratchCubes256 = 4;
+int tp_scratch_cubes(int n);
+float2 *tp_scratch(int n, bool may_allocate);
+void release_tp();
 // Fused x + y pass over `nplanes` planes (N = 128, 256, 512; cudaErrorNotSupported otherwise
 // or when tensor maps cannot describe the operands). Plan kind kKindXy, N = 256: variant 1
 // stages the x-transformed planes through an L2-resident scratch ring (one persistent
@@ -89,7 +126,6 @@ cudaError_t launch_axis_pass_variant(int n, int axis, int op, const float2 *src,
 // maps of the source (and, for the fused z pass, of the filter spectrum) and per-volume
 // destination bases, all in device memory. encode_table_map fills the map of one cube
 // for kind 0 (rows, x pass), 1 (y pass) or 2 (z pass) with the box of that size's kernel.
-#include <cuda.h>
 bool encode_table_map(CUtensorMap *m, const void *cube, int n, int kind);
 // Sets the kernel attributes the table-mode launches of size n need (call before a
 // stream capture that contains them).

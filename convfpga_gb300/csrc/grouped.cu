@@ -8,7 +8,10 @@
 // sequence of job sizes and replayed on every call; tensor maps are re-encoded and
 // uploaded only when a job's buffers move. When the plan fuses the x and y passes of
 // N = 256 or 128 (L2-staged pass), that class runs filter x+y, signal x+y, fused z and
-// inverse y+x instead: three table-mode launches of the fused pass around the z launch.
+// inverse y+x instead: three table-mode launches of the fused pass around the z launch. With
+// the two-pass transform in the plan (and no job of the class in place) it runs that: filters
+// and signals forward (signals through their outputs), middle pass into the spectra's
+// workspace, inverse.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -27,18 +30,20 @@ namespace convgpu {
 namespace {
 
 // rows(filter) rows(signal) rows(out) y(spec) y(out) z(out) z(spec), then the fused x+y
-// pass's rows maps (N = 256 and 128): filter, signal, out
-constexpr int kKinds = 10;
+// pass's rows maps (N = 256 and 128): filter, signal, out; then the two-pass transform's
+// maps of cubes in tile order: spectrum, out
+constexpr int kKinds = 12;
+enum XyForm { kXySeparate = 0, kXyStaged = 1, kXyTiles = 2 };
 
 struct SizeGroup {
   int n = 0;
   std::vector<int> jobs;
   CUtensorMap *d_maps = nullptr;  // [kind][job in group]
-  float2 **d_dsts = nullptr;      // [0][j] spectrum, [1][j] output
+  float2 **d_dsts = nullptr;      // [0][j] spectrum, [1][j] output, [2][j] filter, [3][j] signal
   std::vector<CUtensorMap> h_maps;
   std::vector<float2 *> h_dsts;
   unsigned *d_ctr = nullptr;  // dependency counters of the fused x+y launches
-  bool xy = false;            // this class runs the fused x+y pass
+  XyForm xy = kXySeparate;
 };
 
 struct GPlan {
@@ -65,7 +70,7 @@ struct GPlan {
 };
 
 std::mutex g_mu;
-// key: job sizes, normalize + 2 * (fused x+y: bit 0 N = 256, bit 1 N = 128)
+// key: job sizes, normalize + 2 * (form of N = 256 + 3 * form of N = 128)
 std::map<std::pair<std::vector<int>, int>, std::unique_ptr<GPlan>> g_plans;
 
 cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, cudaStream_t s) {
@@ -74,7 +79,13 @@ cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, 
   float2 *const *spec = g.d_dsts;
   float2 *const *out = g.d_dsts + k;
   cudaError_t e;
-  if (g.xy) {
+  if (g.xy == kXyTiles) {
+    if ((e = launch_tp_fwd_table(g.n, g.d_dsts + 2 * k, m + 10 * k, k, tw512, s)) != cudaSuccess) return e;
+    if ((e = launch_tp_fwd_table(g.n, g.d_dsts + 3 * k, m + 11 * k, k, tw512, s)) != cudaSuccess) return e;
+    if ((e = launch_tp_mid_table(g.n, out, spec, spec, k, tw512, s)) != cudaSuccess) return e;
+    return launch_tp_inv_table(g.n, m + 10 * k, out, k, scale, tw512, s);
+  }
+  if (g.xy == kXyStaged) {
     unsigned *st = device_status_address();
     if ((e = launch_xy_l2_table(g.n, m + 7 * k, spec, k, false, 1.f, tw512, st, g.d_ctr, s)) != cudaSuccess)
       return e;
@@ -94,8 +105,8 @@ cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, 
   return launch_axis_pass_table(g.n, 0, OP_INV, m + 2 * k, nullptr, out, k, scale, tw512, s);
 }
 
-// xy_mask: bit 0 fuses x and y for N = 256, bit 1 for N = 128.
-cudaError_t build(GPlan &p, bool normalize, int xy_mask, const float2 *tw512) {
+// f256, f128: form of the x and y passes for N = 256 and 128.
+cudaError_t build(GPlan &p, bool normalize, XyForm f256, XyForm f128, const float2 *tw512) {
   std::map<int, int> idx;
   for (int j = 0; j < (int)p.sizes.size(); ++j) {
     const int n = p.sizes[j];
@@ -119,11 +130,12 @@ cudaError_t build(GPlan &p, bool normalize, int xy_mask, const float2 *tw512) {
   for (auto &g : p.groups) {
     const size_t k = g.jobs.size();
     g.h_maps.resize(kKinds * k);
-    g.h_dsts.resize(2 * k);
+    g.h_dsts.resize(4 * k);
     if ((e = cudaMalloc(&g.d_maps, sizeof(CUtensorMap) * kKinds * k)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&g.d_dsts, sizeof(float2 *) * 2 * k)) != cudaSuccess) return e;
-    g.xy = (g.n == 256 && (xy_mask & 1)) || (g.n == 128 && (xy_mask & 2));
-    if (g.xy) {
+    if ((e = cudaMalloc(&g.d_dsts, sizeof(float2 *) * 4 * k)) != cudaSuccess) return e;
+    g.xy = g.n == 256 ? f256 : (g.n == 128 ? f128 : kXySeparate);
+    if (g.xy == kXyTiles && (e = prepare_tp(g.n)) != cudaSuccess) return e;
+    if (g.xy == kXyStaged) {
       if ((e = prepare_xy_l2(g.n)) != cudaSuccess) return e;
       if ((e = cudaMalloc(&g.d_ctr, xy_l2_counter_bytes(g.n, (int)k))) != cudaSuccess) return e;
     }
@@ -131,7 +143,7 @@ cudaError_t build(GPlan &p, bool normalize, int xy_mask, const float2 *tw512) {
   if ((e = cudaEventCreateWithFlags(&p.done, cudaEventDisableTiming)) != cudaSuccess) return e;
   for (auto &g : p.groups)
     if ((e = prepare_table_launches(g.n)) != cudaSuccess) return e;
-  // Capture: one branch per size class.
+  // Capture: one branch per size class that runs the three-axis passes.
   cudaStream_t cap;
   if ((e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)) != cudaSuccess) return e;
   std::vector<cudaStream_t> br(p.groups.size(), nullptr);
@@ -142,10 +154,16 @@ cudaError_t build(GPlan &p, bool normalize, int xy_mask, const float2 *tw512) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
+    // Classes of the two-pass transform run one after another, before the others: a CTA of
+    // theirs holds an SM and a fixed share of the tiles, so kernels beside it would leave
+    // some CTAs waiting for an SM.
+    auto scale_of = [&](int n) { return normalize ? (float)(1.0 / ((double)n * n * n)) : 1.0f; };
+    for (auto &g : p.groups)
+      if (g.xy == kXyTiles && e == cudaSuccess) e = enqueue_group(g, scale_of(g.n), tw512, cap);
     cudaEventRecord(ev.back(), cap);
     for (size_t gi = 0; gi < p.groups.size() && e == cudaSuccess; ++gi) {
-      const int n = p.groups[gi].n;
-      const float scale = normalize ? (float)(1.0 / ((double)n * n * n)) : 1.0f;
+      if (p.groups[gi].xy == kXyTiles) continue;
+      const float scale = scale_of(p.groups[gi].n);
       cudaStreamWaitEvent(br[gi], ev.back(), 0);
       e = enqueue_group(p.groups[gi], scale, tw512, br[gi]);
       cudaEventRecord(ev[gi], br[gi]);
@@ -182,14 +200,29 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
       }
   }
   std::lock_guard<std::mutex> lk(g_mu);
-  // the L2-staged variant (1) has a table mode
-  const int xy_mask = (get_pass_variant(256, kKindXy) == 1 ? 1 : 0) | (get_pass_variant(128, kKindXy) == 1 ? 2 : 0);
-  auto key = std::make_pair(sizes, (normalize ? 1 : 0) + 2 * xy_mask);
+  // The L2-staged variant (1) and the two-pass transform (3) have table modes. The latter
+  // takes signals through their outputs, so a class with a job in place (or partly so) runs
+  // the former, as does every class when tensor maps are switched off.
+  auto form = [&](int n) {
+    const int v = get_pass_variant(n, kKindXy);
+    if (v == kXyTwoPass && tma_enabled()) {
+      const uintptr_t bytes = (uintptr_t)n * n * n * sizeof(float2);
+      bool apart = true;
+      for (unsigned j = 0; j < njobs && apart; ++j) {
+        const uintptr_t su = reinterpret_cast<uintptr_t>(ptrs[3 * j]), ou = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
+        if (sizes[j] == n && su < ou + bytes && ou < su + bytes) apart = false;
+      }
+      if (apart) return kXyTiles;
+    }
+    return v == 1 || v == kXyTwoPass ? kXyStaged : kXySeparate;
+  };
+  const XyForm f256 = form(256), f128 = form(128);
+  auto key = std::make_pair(sizes, (normalize ? 1 : 0) + 2 * (f256 + 3 * f128));
   auto it = g_plans.find(key);
   if (it == g_plans.end()) {
     auto p = std::make_unique<GPlan>();
     p->sizes = sizes;
-    cudaError_t e = build(*p, normalize, xy_mask, tw512);
+    cudaError_t e = build(*p, normalize, f256, f128, tw512);
     if (e != cudaSuccess) {
       err = std::string("uneven grouped plan: ") + cudaGetErrorString(e);
       cudaGetLastError();
@@ -212,7 +245,9 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
                   encode_table_map(&g.h_maps[2 * k + v], ot, g.n, 0) && encode_table_map(&g.h_maps[3 * k + v], sp, g.n, 1) &&
                   encode_table_map(&g.h_maps[4 * k + v], ot, g.n, 1) && encode_table_map(&g.h_maps[5 * k + v], ot, g.n, 2) &&
                   encode_table_map(&g.h_maps[6 * k + v], sp, g.n, 2);
-        if (ok && g.xy)
+        if (ok && g.xy == kXyTiles)
+          ok = tp_encode_tiles(&g.h_maps[10 * k + v], sp, g.n, 1) && tp_encode_tiles(&g.h_maps[11 * k + v], ot, g.n, 1);
+        if (ok && g.xy == kXyStaged)
           ok = encode_xy_table_map(&g.h_maps[7 * k + v], ft, g.n) &&
                encode_xy_table_map(&g.h_maps[8 * k + v], sg, g.n) && encode_xy_table_map(&g.h_maps[9 * k + v], ot, g.n);
         if (!ok) {
@@ -221,6 +256,8 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
         }
         g.h_dsts[v] = sp;
         g.h_dsts[k + v] = (float2 *)ot;
+        g.h_dsts[2 * k + v] = (float2 *)const_cast<void *>(ft);
+        g.h_dsts[3 * k + v] = (float2 *)const_cast<void *>(sg);
       }
       // pageable sources: each call returns once the host data is staged
       e = cudaMemcpyAsync(g.d_maps, g.h_maps.data(), sizeof(CUtensorMap) * g.h_maps.size(), cudaMemcpyHostToDevice,

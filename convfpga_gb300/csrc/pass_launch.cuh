@@ -54,6 +54,10 @@ constexpr int kModeTma = 0, kModeTable = 1, kModeGather = 2;
 bool encode_cube_map(CUtensorMap *m, const void *base, int n, long long nplanes, int axis, int cols);
 bool encode_rows_map(CUtensorMap *m, const void *base, int n, long long rows, int xc);
 bool encode_rows512_map(CUtensorMap *m, const void *base, long long rows, int xc);
+// Tile order of the two-pass transform: runs of `vals` complex values, `runs` to a tile;
+// dims (vals, tiles, runs), box {vals, box_tiles, 1}, 16-byte chunks swizzled over the box's
+// row size (32 or 64 bytes).
+bool encode_runs_map(CUtensorMap *m, const void *base, int vals, long long tiles, int runs, int box_tiles);
 // As encode_cube_map over planes of N rows of `width` complex values (row pitch = width).
 bool encode_pitched_map(CUtensorMap *m, const void *base, int width, int n, long long nplanes, int axis, int cols);
 

@@ -8,6 +8,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -117,6 +118,20 @@ bool encode_rows512_map(CUtensorMap *m, const void *base, long long rows, int xc
   return r == CUDA_SUCCESS;
 }
 
+bool encode_runs_map(CUtensorMap *m, const void *base, int vals, long long tiles, int runs, int box_tiles) {
+  auto enc = tensor_map_encoder();
+  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15u) != 0 || tiles > 0x7fffffffLL || (vals != 4 && vals != 8))
+    return false;
+  cuuint64_t dims[3] = {(cuuint64_t)vals, (cuuint64_t)tiles, (cuuint64_t)runs};
+  cuuint64_t strides[2] = {(cuuint64_t)vals * runs * 8, (cuuint64_t)vals * 8};
+  cuuint32_t box[3] = {(cuuint32_t)vals, (cuuint32_t)box_tiles, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void *>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, vals == 4 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 // Box shapes of shape variant 0 (the variant table-mode launches use).
 static void v0_shape(int n, int &xc, int &sc) {
   switch (n) {
@@ -172,8 +187,11 @@ cudaError_t set_dependency_wait_limit(int probes) {
 // ------------------------------------------------------------------ plan table
 static bool g_use_tma = true;
 void set_tma_enabled(bool on) { g_use_tma = on; }
+bool tma_enabled() { return g_use_tma; }
 
-static std::atomic<int> g_variant[6][kPassKinds];
+// Every size starts with shape variant 0; x and y of N = 128 and 256 with the two-pass
+// transform, which was faster than the other forms on every working set measured.
+static std::atomic<int> g_variant[6][kPassKinds] = {{}, {}, {}, {0, 0, 0, 0, kXyTwoPass}, {0, 0, 0, 0, kXyTwoPass}, {}};
 
 static int size_index(int n) {
   switch (n) {
@@ -197,7 +215,8 @@ int pass_kind(int axis, int op) {
 void set_pass_variant(int n, int kind, int variant) {
   const int i = size_index(n);
   if (i >= 0 && kind >= 0 && kind < kPassKinds)
-    g_variant[i][kind].store(kind == kKindXy ? (variant < 0 ? 0 : (variant > 2 ? 2 : variant)) : (variant ? 1 : 0));
+    g_variant[i][kind].store(kind == kKindXy ? std::max(0, std::min(variant, tp_size(n) ? kXyTwoPass : 2))
+                                             : (variant ? 1 : 0));
 }
 
 int get_pass_variant(int n, int kind) {
@@ -376,6 +395,7 @@ cudaError_t launch_axis_pass_tc(int n, int axis, int op, const float2 *src, floa
 cudaError_t launch_xy_pass(int n, const float2 *src, float2 *dst, int nplanes, bool inverse, float scale,
                            const float2 *tw512, cudaStream_t s, int variant) {
   if (!g_use_tma) return cudaErrorNotSupported;
+  if (variant == kXyTwoPass) variant = 1;  // a call the two-pass transform does not take
   if (n == 128 || n == 512)
     return variant == 1 ? launch_xy_l2(n, src, dst, nplanes, inverse, scale, tw512, device_status_address(), s)
                         : cudaErrorNotSupported;

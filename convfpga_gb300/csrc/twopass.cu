@@ -1,0 +1,182 @@
+// Launchers of the two-pass 3D transform (twopass.cuh) for N = 128 and 256, and its scratch
+// cubes. One persistent CTA per SM; launches read their operands through plain pointers, and
+// only the runs of tile order go through a tensor map.
+#define CONVGPU_PASS_LAUNCH_IMPL
+#include "engine_internal.h"
+#include "pass_launch.cuh"
+#include "twopass.cuh"
+
+#include <algorithm>
+
+namespace convgpu {
+
+bool tp_size(int n) { return n == 128 || n == 256; }
+
+namespace {
+
+int sm_count() {
+  static int of[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  if (of[dev] == 0 && cudaDeviceGetAttribute(&of[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+  return of[dev];
+}
+
+template <class K, class... M>
+cudaError_t launch(K kern, int &done, int smem, int threads, long long tiles, cudaStream_t s, const M &...args) {
+  if (tiles <= 0 || tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  const cudaError_t e = set_smem_once(kern, smem, done);
+  if (e != cudaSuccess) return e;
+  kern<<<(unsigned)std::min<long long>(tiles, sm_count()), threads, smem, s>>>(args...);
+  return cudaGetLastError();
+}
+
+template <int N>
+bool encode_tiles(CUtensorMap *m, const void *cubes, int nvol) {
+  using S = TpShape<N>;
+  return encode_runs_map(m, cubes, 2 * S::C, (long long)nvol * N * S::J / S::C, (N / S::J) * (N / 2), N);
+}
+
+template <int N>
+cudaError_t fwd(const TpArgs &a, bool real, const CUtensorMap &m, cudaStream_t s) {
+  const long long tiles = (long long)a.nvol * (N / TpShape<N>::J) * (N / 2);
+  static int done[2] = {0, 0};
+  constexpr int smem = tp_outer_smem<N>(), threads = kTpThreads<N> + 32;
+  return real ? launch(k_tp_fwd<N, true>, done[1], smem, threads, tiles, s, m, a)
+              : launch(k_tp_fwd<N, false>, done[0], smem, threads, tiles, s, m, a);
+}
+
+template <int N>
+cudaError_t inv(const TpArgs &a, const CUtensorMap &m, cudaStream_t s) {
+  const long long tiles = (long long)a.nvol * (N / TpShape<N>::J) * (N / 2);
+  static int done = 0;
+  return launch(k_tp_inv<N>, done, tp_outer_smem<N>(), kTpThreads<N>, tiles, s, m, a);
+}
+
+template <int N>
+cudaError_t mid(const TpArgs &a, int mode, cudaStream_t s) {
+  const long long tiles = (long long)a.nvol * N * TpShape<N>::J / TpShape<N>::C;
+  static int done[3] = {0, 0, 0};
+  constexpr int smem = tp_mid_smem<N>(), threads = kTpThreads<N>;
+  switch (mode) {
+    case TP_PAIR: return launch(k_tp_mid<N, TP_PAIR>, done[0], smem, threads, tiles, s, a);
+    case TP_SPECTRUM: return launch(k_tp_mid<N, TP_SPECTRUM>, done[1], smem, threads, tiles, s, a);
+    case TP_FWD: return launch(k_tp_mid<N, TP_FWD>, done[2], smem, threads, tiles, s, a);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+TpArgs args(int n, const void *src, void *dst, int nvol, const float2 *tw512) {
+  TpArgs a{};
+  a.src = static_cast<const float2 *>(src);
+  a.dst = static_cast<float2 *>(dst);
+  a.src_vol = a.dst_vol = (long long)n * n * n;
+  a.nvol = nvol;
+  a.scale = 1.f;
+  a.tw512 = tw512;
+  a.status = device_status_address();
+  return a;
+}
+
+bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+float2 *g_scratch[2] = {nullptr, nullptr};  // N = 128, 256
+
+}  // namespace
+
+int tp_scratch_cubes(int n) { return n == 128 ? kTpScratchCubes128 : kTpScratchCubes256; }
+
+float2 *tp_scratch(int n, bool may_allocate) {
+  float2 *&p = g_scratch[n == 128 ? 0 : 1];
+  if (!p && may_allocate) {
+    void *q = nullptr;
+    if (cudaMalloc(&q, (size_t)tp_scratch_cubes(n) * n * n * n * sizeof(float2)) == cudaSuccess)
+      p = static_cast<float2 *>(q);
+    else
+      cudaGetLastError();
+  }
+  return p;
+}
+
+void release_tp() {
+  for (auto &p : g_scratch) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  }
+}
+
+bool tp_encode_tiles(CUtensorMap *m, const void *cubes, int n, int nvol) {
+  return n == 128 ? encode_tiles<128>(m, cubes, nvol) : (n == 256 && encode_tiles<256>(m, cubes, nvol));
+}
+
+cudaError_t launch_tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, const float2 *tw512,
+                          cudaStream_t s) {
+  const TpArgs a = args(n, src, dst, nvol, tw512);
+  CUtensorMap m;
+  if (!tp_size(n) || !aligned16(src) || !tp_encode_tiles(&m, dst, n, nvol)) return cudaErrorNotSupported;
+  return n == 128 ? fwd<128>(a, real, m, s) : fwd<256>(a, real, m, s);
+}
+
+cudaError_t launch_tp_inv(int n, const float2 *src, float2 *dst, int nvol, float scale, const float2 *tw512,
+                          cudaStream_t s) {
+  TpArgs a = args(n, src, dst, nvol, tw512);
+  a.scale = scale;
+  CUtensorMap m;
+  if (!tp_size(n) || !tp_encode_tiles(&m, src, n, nvol)) return cudaErrorNotSupported;
+  return n == 128 ? inv<128>(a, m, s) : inv<256>(a, m, s);
+}
+
+cudaError_t launch_tp_mid(int n, int mode, const float2 *src, float2 *dst, const float2 *filt, long long filt_vol,
+                          int nvol, const float2 *tw512, cudaStream_t s) {
+  TpArgs a = args(n, src, dst, nvol, tw512);
+  a.filt = filt;
+  a.filt_vol = filt_vol;
+  if (!tp_size(n) || !aligned16(src) || !aligned16(dst) || (mode != TP_FWD && !aligned16(filt)))
+    return cudaErrorNotSupported;
+  return n == 128 ? mid<128>(a, mode, s) : mid<256>(a, mode, s);
+}
+
+cudaError_t launch_tp_fwd_table(int n, const float2 *const *srcs, const CUtensorMap *dst_maps, int nvol,
+                                const float2 *tw512, cudaStream_t s) {
+  TpArgs a = args(n, nullptr, nullptr, nvol, tw512);
+  a.srcs = srcs;
+  a.maps = dst_maps;
+  CUtensorMap m{};
+  return n == 128 ? fwd<128>(a, false, m, s) : (n == 256 ? fwd<256>(a, false, m, s) : cudaErrorInvalidValue);
+}
+
+cudaError_t launch_tp_inv_table(int n, const CUtensorMap *src_maps, float2 *const *dsts, int nvol, float scale,
+                                const float2 *tw512, cudaStream_t s) {
+  TpArgs a = args(n, nullptr, nullptr, nvol, tw512);
+  a.scale = scale;
+  a.maps = src_maps;
+  a.dsts = dsts;
+  CUtensorMap m{};
+  return n == 128 ? inv<128>(a, m, s) : (n == 256 ? inv<256>(a, m, s) : cudaErrorInvalidValue);
+}
+
+cudaError_t launch_tp_mid_table(int n, const float2 *const *srcs, float2 *const *dsts, const float2 *const *filts,
+                                int nvol, const float2 *tw512, cudaStream_t s) {
+  TpArgs a = args(n, nullptr, nullptr, nvol, tw512);
+  a.srcs = srcs;
+  a.dsts = dsts;
+  a.filts = filts;
+  return n == 128 ? mid<128>(a, TP_PAIR, s) : (n == 256 ? mid<256>(a, TP_PAIR, s) : cudaErrorInvalidValue);
+}
+
+template <int N>
+static cudaError_t prepare() {
+  cudaError_t e = cudaSuccess;
+  const int outer = tp_outer_smem<N>(), middle = tp_mid_smem<N>();
+  auto set = [&](auto kern, int smem) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  };
+  set(k_tp_fwd<N, false>, outer);
+  set(k_tp_inv<N>, outer);
+  set(k_tp_mid<N, TP_PAIR>, middle);
+  return e;
+}
+
+cudaError_t prepare_tp(int n) { return n == 128 ? prepare<128>() : (n == 256 ? prepare<256>() : cudaErrorInvalidValue); }
+
+}  // namespace convgpu

@@ -1,0 +1,561 @@
+// A 3D convolution in tiles instead of axes: the whole forward transform is two passes over
+// memory and so is the inverse, with the product between them.
+//
+// A cube of N^3 points is cut so that each pass transforms as many points as a CTA holds.
+// With y = y0 + R j (R = N / J) and planes zz and zz + N/2 together:
+//   k_tp_fwd   the radix-2 step of z across the two planes, all of x, and J points of y: a
+//              tile of J rows x N points x 2 planes (64 KB at N = 256);
+//   k_tp_mid   the remaining R points of y and N/2 points of z: a tile of R rows x N/2 points
+//              x C columns; forward, product with the filter's spectrum, inverse;
+//   k_tp_inv   the mirror of k_tp_fwd.
+// Against one pass per axis (or x and y together through an L2-resident ring, xyl2.cuh) a
+// signal crosses memory three times as in the ring form (16 + 24 + 16 N^3 bytes with its
+// filter operand), but no CTA waits for another, the twelve radix-16 steps of forward and
+// inverse need eight exchanges instead of twelve, and nothing goes through a ring in L2.
+//
+// The two planes' values are the two lanes of a pair (tilefft.cuh). The radix-2 step turns
+// them into the even and odd half of z, which stay independent, so a pair is transformed
+// lane by lane from the first load to the last store:
+//   lane 0: p(zz) + p(zz + N/2), lane 1: (p(zz) - p(zz + N/2)) W_N^zz.
+// The intermediate array ("tile order") holds a cube as tiles of k_tp_mid, contiguous:
+//   tile g N + kx (g = j' / C), in it unit (y0 N/2 + zz) C + j' % C
+// so a thread of k_tp_fwd, which ends with all j' of one kx, stores runs of C 16-byte units,
+// and k_tp_mid reads and writes whole tiles. Scattering runs of 32 bytes costs nothing: a
+// tile scatter of 4 cubes of 256^3 measured 169 us with 32-byte runs and 164 us with 64-byte
+// runs, a plain copy 170 us (neighbouring tiles in flight fill each other's lines in L2).
+// A spectrum in tile order holds, in tile (g, kx), unit (k2 N/2 + kz') C + c: the pairs
+// (kz = 2 kz' and 2 kz' + 1) at ky = g C + c + J k2.
+//
+// Persistent CTAs take tiles in order through a few buffers in shared memory. The reference streams each axis through its
+// own engine with transposes between (kernels/conv3D.cl:71-420).
+#pragma once
+
+#include "tilefft.cuh"
+
+namespace convgpu {
+
+// Per-size shape: J rows of the outer tile, C interleaved columns of the middle tile, G
+// groups of threads per CTA (one CTA per SM), B tile buffers. A group transforms one tile at
+// a time; the other B - G buffers are in flight, so a group finds its next tile landed.
+//   256: 64 KB tiles, 2 groups of 256 threads x 128 registers, 3 buffers.
+//   128: 32 KB tiles, 4 groups of 128 threads, 6 buffers.
+// One CTA of 16 compute warps per SM, since a thread holds a tile's 16 pairs (64 registers).
+// Measured, us: 4 cubes of 256^3: k_tp_fwd 195 and k_tp_inv 194 (1.07 GB each: 5.5 TB/s; two
+// CTAs of one tile each, loaded and stored from registers, took 215 and 276), k_tp_mid with
+// a filter per cube 322 (357 so), so 905 for a batch with its filters, against 1,083 for the
+// L2-staged x+y passes and the fused z pass; 8 cubes of 128^3 under one filter 190 against
+// 226.
+template <int N>
+struct TpShape;
+template <>
+struct TpShape<256> {
+  static constexpr int J = 16, C = 2, PAD = 0, G = 2, B = 3;
+};
+template <>
+struct TpShape<128> {
+  static constexpr int J = 16, C = 4, PAD = 4, G = 4, B = 6;
+};
+
+// The filter operand of k_tp_mid.
+enum TpMode : int {
+  TP_PAIR = 0,      // filter in tile order, not yet transformed along the rest of y and z
+  TP_SPECTRUM = 1,  // filter spectrum in tile order
+  TP_FWD = 2,       // no filter: the forward half alone (makes a spectrum)
+};
+
+struct TpArgs {
+  const float2 *src;   // k_tp_fwd: cubes; k_tp_mid, k_tp_inv: cubes in tile order
+  float2 *dst;
+  const float2 *filt;  // k_tp_mid
+  long long src_vol, dst_vol, filt_vol;  // elements between cubes (0: one for all)
+  int nvol;
+  float scale;  // k_tp_inv
+  const float2 *tw512;
+  unsigned *status;
+  // Cubes at unrelated addresses (device arrays of nvol pointers and tensor maps), else null.
+  const CUtensorMap *maps;  // k_tp_fwd: dst; k_tp_inv: src
+  const float2 *const *srcs;
+  float2 *const *dsts;
+  const float2 *const *filts;
+  __device__ __forceinline__ const float2 *src_of(int v) const { return srcs ? srcs[v] : src + v * src_vol; }
+  __device__ __forceinline__ float2 *dst_of(int v) const { return dsts ? dsts[v] : dst + v * dst_vol; }
+  __device__ __forceinline__ const float2 *filt_of(int v) const { return filts ? filts[v] : filt + v * filt_vol; }
+};
+
+template <int N>
+struct TpFwdTile : Tile<N, TpShape<N>::J, 1, TpShape<N>::PAD> {
+  using Tile<N, TpShape<N>::J, 1, TpShape<N>::PAD>::Tile;
+};
+template <int N>
+struct TpMidTile : Tile<N / 2, N / TpShape<N>::J, TpShape<N>::C> {
+  using Tile<N / 2, N / TpShape<N>::J, TpShape<N>::C>::Tile;
+};
+
+template <int N>
+constexpr int kTpThreads = TpFwdTile<N>::NT *TpShape<N>::G;
+
+// Bytes between the tile buffers: the largest tile (the outer one's rows may be padded), a
+// multiple of 1 KB.
+template <int N>
+constexpr int kTpBuf = (TpFwdTile<N>::BYTES + 1023) / 1024 * 1024;
+
+// Shared memory: barriers and TMEM slot (1 KB, keeps the tiles aligned), tiles, row
+// twiddles, then the outer passes' step twiddles (two sets of J per group) and the linear
+// table W_N^j.
+template <int N>
+constexpr int tp_outer_smem() {
+  return 1024 + TpShape<N>::B * kTpBuf<N> + N * 16 + TpShape<N>::G * 2 * TpShape<N>::J * 16 + N * 8;
+}
+template <int N>
+constexpr int tp_mid_smem() {
+  return 1024 + TpShape<N>::B * kTpBuf<N> + (N / 2) * 16;
+}
+__device__ __forceinline__ void stg_unit(float2 *p, Pair a) {
+  asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a.re), "l"(a.im) : "memory");
+}
+
+// Step twiddles of outer tile (y0, zz): entry j' = {W_N^(y0 j'), W_N^(y0 j' + zz)} as
+// {c0, c1, s0, s1}; written by the group's first J threads into one of its two sets, since
+// slow threads may still read the previous tile's.
+template <int N>
+__device__ __forceinline__ void tp_step_tw(uint32_t utw, uint32_t lin, int tid, int y0, int zz) {
+  if (tid < TpShape<N>::J) {
+    const float2 a = lds_f2(lin + ((y0 * tid) & (N - 1)) * 8), b = lds_f2(lin + ((y0 * tid + zz) & (N - 1)) * 8);
+    sts_pair(utw + tid * 16, Pair{pk(a.x, b.x), pk(-a.y, -b.y)});
+  }
+}
+
+// Buffers and barriers of a CTA's stream of loads. Load n belongs to group n % G and lands
+// in buffer n % B; load n + B takes the buffer once that group is done with it. Its "full"
+// barrier is the group's own, one of 4 in turn: a group waits for its loads in order, so a
+// parity is never read a phase early (a barrier per buffer serves several groups, and one
+// that is ahead would take the phase before its load's for its own), and a barrier is never
+// armed while its earlier copy is outstanding: load n + 4 G is issued once load n + 4 G - B
+// is consumed, by the group that consumed load n + B before, which took load n's buffer.
+template <int B, int G>
+struct TpStream {
+  static_assert(2 * B % G == 0 && 4 * G - B >= B, "barriers per group");
+  uint32_t bar, tiles, pitch;
+  __device__ __forceinline__ uint32_t full(int n) const { return bar + ((n % G) * 4 + (n / G) % 4) * 8; }
+  __device__ __forceinline__ uint32_t staged(int n) const { return bar + 128 + (n % B) * 8; }
+  __device__ __forceinline__ uint32_t buf(int n) const { return tiles + (n % B) * pitch; }
+  // A bounded wait that gave up marks the CTA: it carries on with what its buffers hold
+  // (wrong output, reported through the status word), waits no more and loads no more.
+  __device__ __forceinline__ uint32_t mark() const { return bar + 192; }
+  __device__ __forceinline__ bool marked() const {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(mark()) : "memory");
+    return v != 0;
+  }
+  __device__ __forceinline__ bool wait_on(uint32_t b, uint32_t parity) const {
+    bool ok = mbar_try_wait(b, parity);
+    if (!ok && !marked()) {
+      ok = mbar_wait_bounded(b, parity);
+      if (!ok) asm volatile("st.shared.u32 [%0], %1;" ::"r"(mark()), "r"(1u) : "memory");
+    }
+    __syncwarp();
+    return ok;
+  }
+  // By all lanes of each warp.
+  __device__ __forceinline__ bool wait(int n) const { return wait_on(full(n), (uint32_t)(n / (4 * G)) & 1u); }
+  __device__ __forceinline__ bool wait_staged(int n) const { return wait_on(staged(n), (uint32_t)(n / B) & 1u); }
+  // By thread 0, before the barriers are used.
+  __device__ __forceinline__ void init(uint32_t stagers) const {
+    for (int i = 0; i < 4 * G; ++i) mbar_init(bar + i * 8, 1);
+    for (int b = 0; b < B; ++b) mbar_init(staged(b), stagers);
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(mark()), "r"(0u) : "memory");
+    mbar_fence_init();
+  }
+};
+
+// After a wait that gave up: reports it, and lets copies still in flight land before the
+// CTA leaves. A barrier's current phase is the one whose parity is not complete.
+template <int B, int G>
+__device__ __forceinline__ void tp_gave_up(const TpStream<B, G> &st, unsigned *status) {
+  if (status) atomicOr(status, kStatusTmaTimeout);
+  for (int b = 0; b < 4 * G; ++b) {
+    const uint32_t parity = mbar_try_wait(st.bar + b * 8, 0) ? 1u : 0u;
+    for (int i = 0; i < 1 << 14; ++i)
+      if (mbar_try_wait(st.bar + b * 8, parity)) break;
+  }
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *m, uint32_t src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)),
+               "r"(src), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+
+// Byte offset of unit c of kx's run in the staged (or landed) box of a column group: boxes
+// of N runs of C units, 16-byte chunks swizzled as the tensor map says (32 or 64 bytes), so
+// that neighbouring kx cover all banks.
+template <int C>
+__device__ __forceinline__ uint32_t tp_run_off(int kx, int c) {
+  return (uint32_t)(kx * C + (c ^ ((kx * C / 8) & (C - 1)))) * 16;
+}
+
+// Forward outer pass. REAL: the source holds N^3 floats per cube. mdst: the destination in
+// tile order, dims (2 C values of a run, tiles, runs of a tile), box (2 C, N, 1). The groups
+// stage their outputs in the tile's own buffer; one further warp issues every copy: the
+// store of a staged tile, and once that has read the buffer (about 1.8 us of the TMA unit's
+// time for 2,048 runs of 32 bytes) the load that takes it next. A store from the registers
+// (one run per thread) instead holds the LSU pipe for 1.4 cycles per run, 80% of the pass.
+template <int N, bool REAL>
+__global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
+    k_tp_fwd(const __grid_constant__ CUtensorMap mdst, TpArgs a) {
+  using TT = TpFwdTile<N>;
+  using S = TpShape<N>;
+  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B;
+  extern __shared__ __align__(1024) unsigned char smraw[];
+  const uint32_t sm = smem_u32(smraw);
+  const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
+  const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + N * 16, lin = utw0 + G * 2 * J * 16;
+  const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
+  const int ntiles = a.nvol * R * H;
+  const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // tiles of this CTA
+  if (threadIdx.x == 0) st.init(TT::NT);
+  TT::fill_tw(tw, a.tw512);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    const float2 w = __ldg(a.tw512 + i * (512 / N));
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(lin + i * 8), "f"(w.x), "f"(w.y) : "memory");
+  }
+  __syncthreads();
+  bool ok = true;
+  if (g == S::G) {  // the copy warp
+    constexpr uint32_t kRow = REAL ? N * 4 : N * 8;
+    auto load = [&](int n) {  // 2 J row copies, row (j, plane) at j ROWB + plane N 8
+      const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
+      // src_vol counts values, complex or (REAL) float
+      const char *src = a.srcs ? (const char *)a.srcs[vol] : (const char *)a.src + vol * a.src_vol * (REAL ? 4 : 8);
+      if (tid == 0) mbar_arrive_expect_tx(st.full(n), 2 * J * kRow);
+      __syncwarp();
+      for (int i = tid; i < 2 * J; i += 32) {
+        const int j = i >> 1, z = zz + (i & 1) * H;
+        bulk_load(st.buf(n) + j * TT::ROWB + (i & 1) * (N * 8), src + ((long long)z * N + y0 + R * j) * kRow, kRow,
+                  st.full(n));
+      }
+    };
+    for (int n = 0; n < B && n < mine; ++n) load(n);
+    for (int n = 0; n < mine; ++n) {
+      ok &= st.wait_staged(n);
+      if (tid == 0) {
+        const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H);
+        const CUtensorMap *m = a.maps ? a.maps + vol : &mdst;
+        if (a.maps) tensormap_acquire(m);
+#pragma unroll
+        for (int k = 0; k < J / C; ++k)
+          tma_store_3d(m, st.buf(n) + k * (N * C * 16), 0, ((a.maps ? 0 : vol) * (J / C) + k) * N, r);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      }
+      __syncwarp();
+      if (n + B < mine && !__any_sync(~0u, st.marked())) load(n + B);
+    }
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (!ok) tp_gave_up(st, a.status);
+    return;
+  }
+  TT tt(tid, 1 + g);
+  int set = 0;
+  for (int n = g; n < mine; n += G) {
+    const int r = (blockIdx.x + n * gridDim.x) % (R * H), y0 = r / H, zz = r % H;
+    const uint32_t utw = utw0 + (g * 2 + set) * (J * 16);
+    tp_step_tw<N>(utw, lin, tid, y0, zz);
+    tt.at(st.buf(n));
+    ok &= st.wait(n);
+    Pair v[16];
+#pragma unroll
+    for (int i = 0; i < TT::B1; ++i)
+#pragma unroll
+      for (int e = 0; e < TT::R1; ++e) {
+        const int x = tt.t1(i) + TT::R2 * e;
+        if constexpr (REAL) {
+          const float p = lds_f(tt.rowb + x * 4), q = lds_f(tt.rowb + N * 8 + x * 4);
+          v[i * TT::R1 + e] = {pk(p + q, p - q), 0ull};
+        } else {
+          const float2 p = lds_f2(tt.rowb + x * 8), q = lds_f2(tt.rowb + N * 8 + x * 8);
+          v[i * TT::R1 + e] = {pk(p.x + q.x, p.x - q.x), pk(p.y + q.y, p.y - q.y)};
+        }
+      }
+    __syncwarp();
+    tt.forward(v, tw, [&] { tt.sync(); });  // every column read: the buffer takes the outputs
+#pragma unroll
+    for (int i = 0; i < TT::B3; ++i) {
+      const int kx = tt.colt + i * TT::NTC;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const Pair s = lds_pair(utw + j * 16);
+        sts_pair(tt.base + (j / C) * (N * C * 16) + tp_run_off<C>(kx, j % C), pmul_tw(v[i * J + j], s.re, s.im));
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_arrive(st.staged(n));
+    set ^= 1;
+  }
+  if (!ok) tp_gave_up(st, a.status);
+}
+
+// Inverse outer pass: tile order -> cubes, scaled. src and dst must not overlap. msrc: as
+// k_tp_fwd's mdst.
+template <int N>
+__global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_inv(const __grid_constant__ CUtensorMap msrc, TpArgs a) {
+  using TT = TpFwdTile<N>;
+  using S = TpShape<N>;
+  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B;
+  extern __shared__ __align__(1024) unsigned char smraw[];
+  const uint32_t sm = smem_u32(smraw);
+  const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
+  const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + N * 16, lin = utw0 + G * 2 * J * 16;
+  const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
+  TT tt(tid, 1 + g);
+  const int ntiles = a.nvol * R * H;
+  const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  if (threadIdx.x == 0) st.init(1);
+  TT::fill_tw(tw, a.tw512);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    const float2 w = __ldg(a.tw512 + i * (512 / N));
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(lin + i * 8), "f"(w.x), "f"(w.y) : "memory");
+  }
+  __syncthreads();
+  auto load = [&](int n) {  // by one thread
+    const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H);
+    const CUtensorMap *m = a.maps ? a.maps + vol : &msrc;
+    if (a.maps) tensormap_acquire(m);
+    mbar_arrive_expect_tx(st.full(n), J * N * 16);
+#pragma unroll
+    for (int k = 0; k < J / C; ++k)
+      tma_load_3d(st.buf(n) + k * (N * C * 16), m, 0, ((a.maps ? 0 : vol) * (J / C) + k) * N, r, st.full(n));
+  };
+  if (threadIdx.x == 0)
+    for (int n = 0; n < B && n < mine; ++n) load(n);
+  bool ok = true;
+  int set = 0;
+  for (int n = g; n < mine; n += G) {
+    const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
+    const uint32_t utw = utw0 + (g * 2 + set) * (J * 16);
+    tp_step_tw<N>(utw, lin, tid, y0, zz);
+    tt.at(st.buf(n));
+    ok &= st.wait(n);
+    Pair v[16];
+#pragma unroll
+    for (int i = 0; i < TT::B3; ++i)
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+        v[i * J + j] = lds_pair(tt.base + (j / C) * (N * C * 16) + tp_run_off<C>(tt.colt + i * TT::NTC, j % C));
+    tt.sync();  // every thread has its units; the step twiddles are written
+#pragma unroll
+    for (int i = 0; i < TT::B3; ++i)
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const Pair s = lds_pair(utw + j * 16);
+        v[i * J + j] = pmul_tw(pswap(v[i * J + j]), s.re, s.im);
+      }
+    tt.inverse(v, tw, [&] {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tt.sync();
+      if (tid == 0 && n + B < mine && !st.marked()) load(n + B);
+      __syncwarp();
+    });
+    float2 *o0 = a.dst_of(vol) + ((long long)zz * N + y0 + R * tt.row) * N, *o1 = o0 + (long long)H * N * N;
+#pragma unroll
+    for (int i = 0; i < TT::B1; ++i)
+#pragma unroll
+      for (int e = 0; e < TT::R1; ++e) {
+        const int x = tt.t1(i) + TT::R2 * e;
+        const Pair p = v[i * TT::R1 + e];  // swapped: re holds im
+        float2 s = make_float2(lo_of(p.im) + hi_of(p.im), lo_of(p.re) + hi_of(p.re));
+        float2 d = make_float2(lo_of(p.im) - hi_of(p.im), lo_of(p.re) - hi_of(p.re));
+        if (a.scale != 1.0f) {
+          s = make_float2(s.x * a.scale, s.y * a.scale);
+          d = make_float2(d.x * a.scale, d.y * a.scale);
+        }
+        o0[x] = s;
+        o1[x] = d;
+      }
+    set ^= 1;
+  }
+  if (!ok) tp_gave_up(st, a.status);
+}
+
+// 64 registers of a thread to and from its TMEM lane (TP_PAIR parks the filter's spectrum
+// there while the signal is transformed: shared memory holds one tile only, and the
+// registers hold one tile's values only).
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const Pair *v) {
+  uint32_t r[32];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    r[4 * k] = (uint32_t)v[k].re;
+    r[4 * k + 1] = (uint32_t)(v[k].re >> 32);
+    r[4 * k + 2] = (uint32_t)v[k].im;
+    r[4 * k + 3] = (uint32_t)(v[k].im >> 32);
+  }
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(addr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, Pair *v) {  // 4 units
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(addr)
+      : "memory");
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    v[k].re = (f32x2)r[4 * k] | ((f32x2)r[4 * k + 1] << 32);
+    v[k].im = (f32x2)r[4 * k + 2] | ((f32x2)r[4 * k + 3] << 32);
+  }
+}
+
+// Middle pass over tiles of cubes in tile order. Every group reads its whole tile (and the
+// filter's) before it writes the output tile, so dst may be src or, with one filter per
+// cube, the filter array. With a filter a tile is two loads, the filter's and then the
+// signal's, and the groups' loads alternate (load n belongs to group n % G): the filter's
+// values wait in TMEM, so its buffer is free again before the signal's transform starts
+// (reading a spectrum from global memory at the product took 344 us for 4 cubes of 256^3,
+// this 277).
+template <int N, int MODE>
+__global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
+  using TT = TpMidTile<N>;
+  using S = TpShape<N>;
+  constexpr int R = TT::J, C = TT::C, H = N / 2, G = S::G, B = S::B, TILES = N * (N / R) / C;
+  constexpr int LPT = MODE == TP_FWD ? 1 : 2;             // loads per tile
+  constexpr long long ELEMS = (long long)R * H * C * 2;  // complex values per tile
+  static_assert(TT::NT * G == kTpThreads<N> && TT::BYTES <= kTpBuf<N>, "one CTA shape for all passes");
+  constexpr int kCols = TT::NT * G / 2;  // TMEM columns: 64 per warp that shares a lane group
+  extern __shared__ __align__(1024) unsigned char smraw[];
+  const uint32_t sm = smem_u32(smraw), tslot = sm + 200;
+  const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
+  const uint32_t tw = sm + 1024 + B * kTpBuf<N>;
+  const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
+  TT tt(tid, 1 + g);
+  const int ntiles = a.nvol * TILES;
+  const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  // Loads come in rounds of G (one per group, missing ones included so that n % G is the
+  // group); tile of load n: its round's number / LPT.
+  const int loads = (mine + G - 1) / G * G * LPT;
+  if (threadIdx.x == 0) st.init(1);
+  if constexpr (MODE != TP_FWD) {
+    if (threadIdx.x < 32) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tslot), "n"(kCols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+  }
+  TT::fill_tw(tw, a.tw512);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  uint32_t tmem = 0, park = 0;
+  if constexpr (MODE != TP_FWD) {
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot) : "memory");
+    const int w = threadIdx.x >> 5;
+    park = tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(64 * (w >> 2));
+  }
+  // Tile w: cube w % nvol, tile w / nvol: the cubes' tiles against one filter run together.
+  auto load = [&](int n) {  // by one thread; a missing tile's load completes at once
+    const int k = (n / G / LPT) * G + n % G;  // this CTA's tile number
+    if (k >= mine) {
+      mbar_arrive_expect_tx(st.full(n), 0);
+      return;
+    }
+    const int w = blockIdx.x + k * gridDim.x, vol = w % a.nvol;
+    const float2 *cube = (LPT == 2 && (n / G) % 2 == 0) ? a.filt_of(vol) : a.src_of(vol);
+    mbar_arrive_expect_tx(st.full(n), (uint32_t)(ELEMS * 8));
+    bulk_load(st.buf(n), cube + (long long)(w / a.nvol) * ELEMS, (uint32_t)(ELEMS * 8), st.full(n));
+  };
+  if (threadIdx.x == 0)
+    for (int n = 0; n < B && n < loads; ++n) load(n);
+  bool ok = true;
+  int n = g;  // this group's next load
+  Pair v[16];
+  auto read_rows = [&] {
+    tt.at(st.buf(n));
+    ok &= st.wait(n);
+#pragma unroll
+    for (int i = 0; i < TT::B1; ++i)
+#pragma unroll
+      for (int e = 0; e < TT::R1; ++e) v[i * TT::R1 + e] = lds_pair(tt.nat(tt.t1(i) + TT::R2 * e));
+    __syncwarp();
+  };
+  auto release = [&] {  // this group is done with load n's buffer
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tt.sync();
+    if (tid == 0 && n + B < loads && !st.marked()) load(n + B);
+    __syncwarp();  // the TMEM instructions want the whole warp
+    n += G;
+  };
+  // unit of output (i, j) of this thread in a spectrum's tile
+  auto spec = [&](int i, int j) { return ((j * H + tt.colt + i * TT::NTC) * C + tt.c) * 2; };
+  for (int k = g; k < mine; k += G) {
+    const int w = blockIdx.x + k * gridDim.x, vol = w % a.nvol;
+    const long long off = (long long)(w / a.nvol) * ELEMS;
+    if constexpr (MODE != TP_FWD) {
+      if constexpr (MODE == TP_PAIR) {
+        read_rows();
+        tt.forward(v, tw, release);
+      } else {
+        ok &= st.wait(n);
+#pragma unroll
+        for (int i = 0; i < TT::B3; ++i)
+#pragma unroll
+          for (int j = 0; j < R; ++j) v[i * R + j] = lds_pair(st.buf(n) + spec(i, j) * 8);
+        release();
+      }
+      tmem_st16(park, v);
+      tmem_st16(park + 32, v + 8);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    read_rows();
+    if constexpr (MODE == TP_FWD) {
+      tt.forward(v, tw, release);
+      float2 *o = a.dst_of(vol) + off;
+#pragma unroll
+      for (int i = 0; i < TT::B3; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) stg_unit(o + spec(i, j), v[i * R + j]);
+    } else {
+      tt.forward(v, tw, [] {});
+#pragma unroll
+      for (int q = 0; q < 16; q += 4) {
+        Pair f[4];
+        tmem_ld4(park + 4 * q, f);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) v[q + m] = pswap(pmul(v[q + m], f[m]));
+      }
+      tt.inverse(v, tw, release);
+      float2 *o = a.dst_of(vol) + off;
+#pragma unroll
+      for (int i = 0; i < TT::B1; ++i)
+#pragma unroll
+        for (int e = 0; e < TT::R1; ++e)
+          stg_unit(o + ((tt.row * H + tt.t1(i) + TT::R2 * e) * C + tt.c) * 2, pswap(v[i * TT::R1 + e]));
+    }
+  }
+  // A group without a tile in the last round hands its buffers on all the same.
+  for (; n < loads; n += G) {
+    ok &= st.wait(n);
+    if (tid == 0 && n + B < loads && !st.marked()) load(n + B);
+  }
+  if (!ok) tp_gave_up(st, a.status);
+  if constexpr (MODE != TP_FWD) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kCols));
+  }
+}
+
+}  // namespace convgpu

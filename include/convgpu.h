@@ -55,6 +55,10 @@ extern "C" {
  * filter, and the result equals that of the same filter given as complex values with
  * zero imaginary parts. Not with CONVGPU_FILTER_IS_SPECTRUM. The reference takes complex
  * filters only; its real Gaussian filters are stored with zero imaginary parts.
+ * Calls of N = 128 and 256 on the FP32 path also hold 512 MiB of scratch cubes per size,
+ * allocated by the first such call and kept until fpga_final; without them (no memory) the
+ * calls run the passes of the other plan variants. A call captured into a graph allocates
+ * none, so make one call of its size before the capture.
  * d_sig may equal d_out (in place). The library's per-device workspace is shared by
  * all calls: calls on different streams must not overlap. */
 int convgpu_conv3d_device(unsigned N, const float2 *d_sig, const float2 *d_filter, float2 *d_out,
@@ -143,7 +147,9 @@ unsigned long long convgpu_launch_count(void);
  *           bytes (one read + one write of every cube, plus the filter operand read of
  *           the fused z pass); slot = axis * 4 + op, axis 0/1/2 = x/y/z,
  *           op 0 forward, 1 inverse, 2 z fwd->multiply->inv, 3 same with the filter's
- *           z transform fused in; slots 12 / 13: fused x+y pass forward / inverse. */
+ *           z transform fused in; slots 12 / 13: fused x+y pass forward / inverse. The
+ *           two-pass 3D transform's outer passes count as fused x+y passes and its middle
+ *           pass as the z pass, with the bytes of the passes they replace. */
 #define CONVGPU_PASS_SLOTS 14
 int convgpu_pass_timing(int mode, double *ms, unsigned long long *launches, double *bytes);
 
@@ -161,13 +167,15 @@ int convgpu_autotune(const unsigned *sizes, unsigned count, int write_cache);
 /* Plan-table entry of cube size N for pass kind (0 x pass, 1 y/z passes, 2 fused z pass,
  * 3 fused z pass with the filter's z transform, 4 x and y: 0 separate passes; N = 256:
  * 1 one pass staged through an L2-resident scratch ring, 2 one pass on 8-CTA clusters;
- * N = 128 and 512: 1 one pass staged through an L2-resident scratch ring;
+ * N = 128 and 512: 1 one pass staged through an L2-resident scratch ring; N = 128 and 256,
+ * the default there: 3 the two-pass 3D transform, for calls whose cubes are 16-byte aligned
+ * and whose outputs are the signals or do not overlap them (other calls run 1);
  * 5 tensor-core kernels of CONVGPU_TENSOR_SPLIT, N = 256: 0 tcgen05 (TMEM accumulators),
  * 1 mma.sync; 6 x and y passes of the tcgen05 split path, N = 256: 0 separate passes, 1 one
  * pass staged through the L2-resident scratch ring; 7 spectra of real filters
  * (CONVGPU_FILTER_REAL, FP32 path, N >= 64): 0 full spectra, 1 Hermitian half spectra, kx up
  * to N/2 only, with a fused z pass that serves a column tile and its mirror from one read):
- * sets it to set_to (0 or 1; 0..2 for kind 4) when set_to >= 0, and returns the current
+ * sets it to set_to (0 or 1; 0..2 for kind 4, 0..3 with N = 128 or 256) when set_to >= 0, and returns the current
  * variant (or a negative CONVGPU_E* code). */
 int convgpu_plan_variant(unsigned N, int kind, int set_to);
 
