@@ -40,11 +40,10 @@ namespace convgpu {
 //   256: 64 KB tiles, 2 groups of 256 threads x 128 registers, 3 buffers.
 //   128: 32 KB tiles, 4 groups of 128 threads, 6 buffers.
 // One CTA of 16 compute warps per SM, since a thread holds a tile's 16 pairs (64 registers).
-// Measured, us: 4 cubes of 256^3: k_tp_fwd 195 and k_tp_inv 194 (1.07 GB each: 5.5 TB/s; two
+// Measured, us: 4 cubes of 256^3: k_tp_fwd 187 and k_tp_inv 191 (1.07 GB each: 5.7 TB/s; two
 // CTAs of one tile each, loaded and stored from registers, took 215 and 276), k_tp_mid with
-// a filter per cube 322 (357 so), so 905 for a batch with its filters, against 1,083 for the
-// L2-staged x+y passes and the fused z pass; 8 cubes of 128^3 under one filter 190 against
-// 226.
+// a filter per cube 287 (1.6 GB: 5.6 TB/s), so 850 for a batch with its filters, against
+// 1,083 for the L2-staged x+y passes and the fused z pass.
 template <int N>
 struct TpShape;
 template <>
@@ -83,32 +82,28 @@ struct TpArgs {
 };
 
 template <int N>
-struct TpFwdTile : Tile<N, TpShape<N>::J, 1, TpShape<N>::PAD> {
-  using Tile<N, TpShape<N>::J, 1, TpShape<N>::PAD>::Tile;
-};
+using TpOuterTile = OuterTile<N, TpShape<N>::J, TpShape<N>::PAD>;
 template <int N>
-struct TpMidTile : Tile<N / 2, N / TpShape<N>::J, TpShape<N>::C> {
-  using Tile<N / 2, N / TpShape<N>::J, TpShape<N>::C>::Tile;
-};
+using TpMidTile = MidTile<N / 2, N / TpShape<N>::J, TpShape<N>::C>;
 
 template <int N>
-constexpr int kTpThreads = TpFwdTile<N>::NT *TpShape<N>::G;
+constexpr int kTpThreads = TpOuterTile<N>::NT *TpShape<N>::G;
 
 // Bytes between the tile buffers: the largest tile (the outer one's rows may be padded), a
 // multiple of 1 KB.
 template <int N>
-constexpr int kTpBuf = (TpFwdTile<N>::BYTES + 1023) / 1024 * 1024;
+constexpr int kTpBuf = (TpOuterTile<N>::BYTES + 1023) / 1024 * 1024;
 
 // Shared memory: barriers and TMEM slot (1 KB, keeps the tiles aligned), tiles, row
 // twiddles, then the outer passes' step twiddles (two sets of J per group) and the linear
 // table W_N^j.
 template <int N>
 constexpr int tp_outer_smem() {
-  return 1024 + TpShape<N>::B * kTpBuf<N> + N * 16 + TpShape<N>::G * 2 * TpShape<N>::J * 16 + N * 8;
+  return 1024 + TpShape<N>::B * kTpBuf<N> + TpOuterTile<N>::kTwBytes + TpShape<N>::G * 2 * TpShape<N>::J * 16 + N * 8;
 }
 template <int N>
 constexpr int tp_mid_smem() {
-  return 1024 + TpShape<N>::B * kTpBuf<N> + (N / 2) * 16;
+  return 1024 + TpShape<N>::B * kTpBuf<N> + TpMidTile<N>::kTwBytes;
 }
 __device__ __forceinline__ void stg_unit(float2 *p, Pair a) {
   asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a.re), "l"(a.im) : "memory");
@@ -137,7 +132,6 @@ struct TpStream {
   static_assert(2 * B % G == 0 && 4 * G - B >= B, "barriers per group");
   uint32_t bar, tiles, pitch;
   __device__ __forceinline__ uint32_t full(int n) const { return bar + ((n % G) * 4 + (n / G) % 4) * 8; }
-  __device__ __forceinline__ uint32_t staged(int n) const { return bar + 128 + (n % B) * 8; }
   __device__ __forceinline__ uint32_t buf(int n) const { return tiles + (n % B) * pitch; }
   // A bounded wait that gave up marks the CTA: it carries on with what its buffers hold
   // (wrong output, reported through the status word), waits no more and loads no more.
@@ -158,15 +152,41 @@ struct TpStream {
   }
   // By all lanes of each warp.
   __device__ __forceinline__ bool wait(int n) const { return wait_on(full(n), (uint32_t)(n / (4 * G)) & 1u); }
-  __device__ __forceinline__ bool wait_staged(int n) const { return wait_on(staged(n), (uint32_t)(n / B) & 1u); }
   // By thread 0, before the barriers are used.
-  __device__ __forceinline__ void init(uint32_t stagers) const {
+  __device__ __forceinline__ void init() const {
     for (int i = 0; i < 4 * G; ++i) mbar_init(bar + i * 8, 1);
-    for (int b = 0; b < B; ++b) mbar_init(staged(b), stagers);
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(mark()), "r"(0u) : "memory");
     mbar_fence_init();
   }
 };
+
+// TMEM of a CTA (warp 0 allocates and frees): 64 columns per warp that shares a lane group,
+// for the row exchange, and in the middle pass as many again for the filter's values.
+template <int COLS>
+__device__ __forceinline__ uint32_t tp_tmem_alloc(uint32_t slot) {
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "n"(COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  uint32_t tmem;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(slot) : "memory");
+  return tmem;
+}
+template <int COLS>
+__device__ __forceinline__ void tp_tmem_free(uint32_t tmem) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(COLS));
+}
+// This warp's 64 columns of block b.
+__device__ __forceinline__ uint32_t tp_tmem_warp(uint32_t tmem, int b) {
+  const int w = threadIdx.x >> 5;
+  return tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(256 * b + 64 * (w >> 2));
+}
 
 // After a wait that gave up: reports it, and lets copies still in flight land before the
 // CTA leaves. A barrier's current phase is the one whose parity is not complete.
@@ -200,25 +220,35 @@ __device__ __forceinline__ uint32_t tp_run_off(int kx, int c) {
 }
 
 // Forward outer pass. REAL: the source holds N^3 floats per cube. mdst: the destination in
-// tile order, dims (2 C values of a run, tiles, runs of a tile), box (2 C, N, 1). The groups
-// stage their outputs in the tile's own buffer; one further warp issues every copy: the
-// store of a staged tile, and once that has read the buffer (about 1.8 us of the TMA unit's
-// time for 2,048 runs of 32 bytes) the load that takes it next. A store from the registers
-// (one run per thread) instead holds the LSU pipe for 1.4 cycles per run, 80% of the pass.
+// tile order, dims (2 C values of a run, tiles, runs of a tile), box (2 C, N, 1). Every group
+// has a buffer of its own, where its loads land and its exchanges happen; the next load is
+// issued when the columns are in registers. Outputs are staged in the other S = B - G
+// buffers, which the groups take in turn, and a further warp stores them: 2,048 runs of 32
+// bytes keep the TMA unit for about 1.8 us, which the tile's own buffer does not wait for.
+// (Stores from registers, one run per thread, hold the LSU pipe for 1.4 cycles a run, 80% of
+// the pass: 215 us for 4 cubes of 256^3. Staged in the tile's own buffer 195, this 187.)
 template <int N, bool REAL>
 __global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
     k_tp_fwd(const __grid_constant__ CUtensorMap mdst, TpArgs a) {
-  using TT = TpFwdTile<N>;
+  using TT = TpOuterTile<N>;
   using S = TpShape<N>;
-  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B;
+  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B, SB = B - G;
+  static_assert(G % SB == 0, "the groups take the staging buffers in turn");
   extern __shared__ __align__(1024) unsigned char smraw[];
   const uint32_t sm = smem_u32(smraw);
   const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
-  const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + N * 16, lin = utw0 + G * 2 * J * 16;
+  const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + TT::kTwBytes, lin = utw0 + G * 2 * J * 16;
   const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
   const int ntiles = a.nvol * R * H;
   const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // tiles of this CTA
-  if (threadIdx.x == 0) st.init(TT::NT);
+  // staged[s]: the group whose turn it is has staged its tile in buffer G + s; grant[g]: the
+  // buffer of group g's next tile has been stored (a group's own, so its waits are in order).
+  const uint32_t staged = sm + 128, grant = sm + 144;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < SB; ++s) mbar_init(staged + s * 8, TT::NT);
+    for (int i = 0; i < G; ++i) mbar_init(grant + i * 8, 1);
+    st.init();
+  }
   TT::fill_tw(tw, a.tw512);
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const float2 w = __ldg(a.tw512 + i * (512 / N));
@@ -226,75 +256,80 @@ __global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
   }
   __syncthreads();
   bool ok = true;
-  if (g == S::G) {  // the copy warp
-    constexpr uint32_t kRow = REAL ? N * 4 : N * 8;
-    auto load = [&](int n) {  // 2 J row copies, row (j, plane) at j ROWB + plane N 8
-      const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
-      // src_vol counts values, complex or (REAL) float
-      const char *src = a.srcs ? (const char *)a.srcs[vol] : (const char *)a.src + vol * a.src_vol * (REAL ? 4 : 8);
-      if (tid == 0) mbar_arrive_expect_tx(st.full(n), 2 * J * kRow);
-      __syncwarp();
-      for (int i = tid; i < 2 * J; i += 32) {
-        const int j = i >> 1, z = zz + (i & 1) * H;
-        bulk_load(st.buf(n) + j * TT::ROWB + (i & 1) * (N * 8), src + ((long long)z * N + y0 + R * j) * kRow, kRow,
-                  st.full(n));
-      }
-    };
-    for (int n = 0; n < B && n < mine; ++n) load(n);
+  if (g == G) {  // the storing warp
     for (int n = 0; n < mine; ++n) {
-      ok &= st.wait_staged(n);
+      const int s = n % SB;
+      ok &= st.wait_on(staged + s * 8, (uint32_t)(n / SB) & 1u);
       if (tid == 0) {
         const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H);
         const CUtensorMap *m = a.maps ? a.maps + vol : &mdst;
         if (a.maps) tensormap_acquire(m);
 #pragma unroll
         for (int k = 0; k < J / C; ++k)
-          tma_store_3d(m, st.buf(n) + k * (N * C * 16), 0, ((a.maps ? 0 : vol) * (J / C) + k) * N, r);
+          tma_store_3d(m, st.buf(G + s) + k * (N * C * 16), 0, ((a.maps ? 0 : vol) * (J / C) + k) * N, r);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if (n + SB < mine) mbar_arrive(grant + (n + SB) % G * 8);
       }
       __syncwarp();
-      if (n + B < mine && !__any_sync(~0u, st.marked())) load(n + B);
     }
     if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (!ok) tp_gave_up(st, a.status);
     return;
   }
-  TT tt(tid, 1 + g);
+  constexpr uint32_t kRow = REAL ? N * 4 : N * 8;
+  auto load = [&](int n) {  // by the group's first warp: 2 J row copies, row (j, plane) at j ROWB + plane N 8
+    const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
+    // src_vol counts values, complex or (REAL) float
+    const char *src = a.srcs ? (const char *)a.srcs[vol] : (const char *)a.src + vol * a.src_vol * (REAL ? 4 : 8);
+    if (tid == 0) mbar_arrive_expect_tx(st.full(n), 2 * J * kRow);
+    __syncwarp();
+    for (int i = tid; i < 2 * J; i += 32) {
+      const int j = i >> 1, z = zz + (i & 1) * H;
+      bulk_load(st.buf(g) + j * TT::ROWB + (i & 1) * (N * 8), src + ((long long)z * N + y0 + R * j) * kRow, kRow,
+                st.full(n));
+    }
+  };
+  if (tid < 32 && g < mine) load(g);
+  TT tt(tid, 1 + g, tw);
+  tt.at(st.buf(g));
   int set = 0;
   for (int n = g; n < mine; n += G) {
     const int r = (blockIdx.x + n * gridDim.x) % (R * H), y0 = r / H, zz = r % H;
     const uint32_t utw = utw0 + (g * 2 + set) * (J * 16);
     tp_step_tw<N>(utw, lin, tid, y0, zz);
-    tt.at(st.buf(n));
     ok &= st.wait(n);
     Pair v[16];
 #pragma unroll
-    for (int i = 0; i < TT::B1; ++i)
-#pragma unroll
-      for (int e = 0; e < TT::R1; ++e) {
-        const int x = tt.t1(i) + TT::R2 * e;
-        if constexpr (REAL) {
-          const float p = lds_f(tt.rowb + x * 4), q = lds_f(tt.rowb + N * 8 + x * 4);
-          v[i * TT::R1 + e] = {pk(p + q, p - q), 0ull};
-        } else {
-          const float2 p = lds_f2(tt.rowb + x * 8), q = lds_f2(tt.rowb + N * 8 + x * 8);
-          v[i * TT::R1 + e] = {pk(p.x + q.x, p.x - q.x), pk(p.y + q.y, p.y - q.y)};
-        }
+    for (int e = 0; e < 16; ++e) {
+      const int x = tt.t + TT::R2 * e;
+      if constexpr (REAL) {
+        const float p = lds_f(tt.rowb + x * 4), q = lds_f(tt.rowb + N * 8 + x * 4);
+        v[e] = {pk(p + q, p - q), 0ull};
+      } else {
+        const float2 p = lds_f2(tt.rowb + x * 8), q = lds_f2(tt.rowb + N * 8 + x * 8);
+        v[e] = {pk(p.x + q.x, p.x - q.x), pk(p.y + q.y, p.y - q.y)};
       }
+    }
     __syncwarp();
-    tt.forward(v, tw, [&] { tt.sync(); });  // every column read: the buffer takes the outputs
+    tt.forward(v, [&] {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tt.sync();
+      if (tid < 32 && n + G < mine && !__any_sync(~0u, st.marked())) load(n + G);
+    });
+    if (n >= SB) ok &= st.wait_on(grant + g * 8, (uint32_t)(n / G - (g < SB ? 1 : 0)) & 1u);
+    const uint32_t out = st.buf(G + n % SB);
 #pragma unroll
     for (int i = 0; i < TT::B3; ++i) {
-      const int kx = tt.colt + i * TT::NTC;
+      const int kx = tt.q + i * TT::NT;
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const Pair s = lds_pair(utw + j * 16);
-        sts_pair(tt.base + (j / C) * (N * C * 16) + tp_run_off<C>(kx, j % C), pmul_tw(v[i * J + j], s.re, s.im));
+        sts_pair(out + (j / C) * (N * C * 16) + tp_run_off<C>(kx, j % C), pmul_tw(v[i * J + j], s.re, s.im));
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_arrive(st.staged(n));
+    mbar_arrive(staged + n % SB * 8);
     set ^= 1;
   }
   if (!ok) tp_gave_up(st, a.status);
@@ -304,24 +339,24 @@ __global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
 // k_tp_fwd's mdst.
 template <int N>
 __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_inv(const __grid_constant__ CUtensorMap msrc, TpArgs a) {
-  using TT = TpFwdTile<N>;
+  using TT = TpOuterTile<N>;
   using S = TpShape<N>;
   constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B;
   extern __shared__ __align__(1024) unsigned char smraw[];
   const uint32_t sm = smem_u32(smraw);
   const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
-  const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + N * 16, lin = utw0 + G * 2 * J * 16;
+  const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + TT::kTwBytes, lin = utw0 + G * 2 * J * 16;
   const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
-  TT tt(tid, 1 + g);
   const int ntiles = a.nvol * R * H;
   const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  if (threadIdx.x == 0) st.init(1);
+  if (threadIdx.x == 0) st.init();
   TT::fill_tw(tw, a.tw512);
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const float2 w = __ldg(a.tw512 + i * (512 / N));
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(lin + i * 8), "f"(w.x), "f"(w.y) : "memory");
   }
   __syncthreads();
+  TT tt(tid, 1 + g, tw);
   auto load = [&](int n) {  // by one thread
     const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H);
     const CUtensorMap *m = a.maps ? a.maps + vol : &msrc;
@@ -346,7 +381,7 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_inv(const __grid_consta
     for (int i = 0; i < TT::B3; ++i)
 #pragma unroll
       for (int j = 0; j < J; ++j)
-        v[i * J + j] = lds_pair(tt.base + (j / C) * (N * C * 16) + tp_run_off<C>(tt.colt + i * TT::NTC, j % C));
+        v[i * J + j] = lds_pair(tt.base + (j / C) * (N * C * 16) + tp_run_off<C>(tt.q + i * TT::NT, j % C));
     tt.sync();  // every thread has its units; the step twiddles are written
 #pragma unroll
     for (int i = 0; i < TT::B3; ++i)
@@ -355,7 +390,7 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_inv(const __grid_consta
         const Pair s = lds_pair(utw + j * 16);
         v[i * J + j] = pmul_tw(pswap(v[i * J + j]), s.re, s.im);
       }
-    tt.inverse(v, tw, [&] {
+    tt.inverse(v, [&] {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tt.sync();
       if (tid == 0 && n + B < mine && !st.marked()) load(n + B);
@@ -363,20 +398,18 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_inv(const __grid_consta
     });
     float2 *o0 = a.dst_of(vol) + ((long long)zz * N + y0 + R * tt.row) * N, *o1 = o0 + (long long)H * N * N;
 #pragma unroll
-    for (int i = 0; i < TT::B1; ++i)
-#pragma unroll
-      for (int e = 0; e < TT::R1; ++e) {
-        const int x = tt.t1(i) + TT::R2 * e;
-        const Pair p = v[i * TT::R1 + e];  // swapped: re holds im
-        float2 s = make_float2(lo_of(p.im) + hi_of(p.im), lo_of(p.re) + hi_of(p.re));
-        float2 d = make_float2(lo_of(p.im) - hi_of(p.im), lo_of(p.re) - hi_of(p.re));
-        if (a.scale != 1.0f) {
-          s = make_float2(s.x * a.scale, s.y * a.scale);
-          d = make_float2(d.x * a.scale, d.y * a.scale);
-        }
-        o0[x] = s;
-        o1[x] = d;
+    for (int e = 0; e < 16; ++e) {
+      const int x = tt.t + TT::R2 * e;
+      const Pair p = v[e];  // swapped: re holds im
+      float2 s = make_float2(lo_of(p.im) + hi_of(p.im), lo_of(p.re) + hi_of(p.re));
+      float2 d = make_float2(lo_of(p.im) - hi_of(p.im), lo_of(p.re) - hi_of(p.re));
+      if (a.scale != 1.0f) {
+        s = make_float2(s.x * a.scale, s.y * a.scale);
+        d = make_float2(d.x * a.scale, d.y * a.scale);
       }
+      o0[x] = s;
+      o1[x] = d;
+    }
     set ^= 1;
   }
   if (!ok) tp_gave_up(st, a.status);
@@ -425,7 +458,7 @@ __device__ __forceinline__ void tmem_ld4(uint32_t addr, Pair *v) {  // 4 units
 // signal's, and the groups' loads alternate (load n belongs to group n % G): the filter's
 // values wait in TMEM, so its buffer is free again before the signal's transform starts
 // (reading a spectrum from global memory at the product took 344 us for 4 cubes of 256^3,
-// this 277).
+// this 277 otherwise alike).
 template <int N, int MODE>
 __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
   using TT = TpMidTile<N>;
@@ -434,36 +467,21 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
   constexpr int LPT = MODE == TP_FWD ? 1 : 2;             // loads per tile
   constexpr long long ELEMS = (long long)R * H * C * 2;  // complex values per tile
   static_assert(TT::NT * G == kTpThreads<N> && TT::BYTES <= kTpBuf<N>, "one CTA shape for all passes");
-  constexpr int kCols = TT::NT * G / 2;  // TMEM columns: 64 per warp that shares a lane group
+  constexpr int kCols = MODE == TP_FWD ? 256 : 512;  // TMEM columns
   extern __shared__ __align__(1024) unsigned char smraw[];
   const uint32_t sm = smem_u32(smraw), tslot = sm + 200;
   const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
   const uint32_t tw = sm + 1024 + B * kTpBuf<N>;
   const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
-  TT tt(tid, 1 + g);
   const int ntiles = a.nvol * TILES;
   const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   // Loads come in rounds of G (one per group, missing ones included so that n % G is the
   // group); tile of load n: its round's number / LPT.
   const int loads = (mine + G - 1) / G * G * LPT;
-  if (threadIdx.x == 0) st.init(1);
-  if constexpr (MODE != TP_FWD) {
-    if (threadIdx.x < 32) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tslot), "n"(kCols)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-  }
+  if (threadIdx.x == 0) st.init();
   TT::fill_tw(tw, a.tw512);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  uint32_t tmem = 0, park = 0;
-  if constexpr (MODE != TP_FWD) {
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tslot) : "memory");
-    const int w = threadIdx.x >> 5;
-    park = tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(64 * (w >> 2));
-  }
+  const uint32_t tmem = tp_tmem_alloc<kCols>(tslot), park = tp_tmem_warp(tmem, 1);
+  TT tt(tid, 1 + g, tp_tmem_warp(tmem, 0), tw);
   // Tile w: cube w % nvol, tile w / nvol: the cubes' tiles against one filter run together.
   auto load = [&](int n) {  // by one thread; a missing tile's load completes at once
     const int k = (n / G / LPT) * G + n % G;  // this CTA's tile number
@@ -485,9 +503,7 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
     tt.at(st.buf(n));
     ok &= st.wait(n);
 #pragma unroll
-    for (int i = 0; i < TT::B1; ++i)
-#pragma unroll
-      for (int e = 0; e < TT::R1; ++e) v[i * TT::R1 + e] = lds_pair(tt.nat(tt.t1(i) + TT::R2 * e));
+    for (int e = 0; e < 16; ++e) v[e] = lds_pair(tt.nat(tt.t + TT::R2 * e));
     __syncwarp();
   };
   auto release = [&] {  // this group is done with load n's buffer
@@ -505,7 +521,7 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
     if constexpr (MODE != TP_FWD) {
       if constexpr (MODE == TP_PAIR) {
         read_rows();
-        tt.forward(v, tw, release);
+        tt.forward(v, release);
       } else {
         ok &= st.wait(n);
 #pragma unroll
@@ -520,14 +536,14 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
     }
     read_rows();
     if constexpr (MODE == TP_FWD) {
-      tt.forward(v, tw, release);
+      tt.forward(v, release);
       float2 *o = a.dst_of(vol) + off;
 #pragma unroll
       for (int i = 0; i < TT::B3; ++i)
 #pragma unroll
         for (int j = 0; j < R; ++j) stg_unit(o + spec(i, j), v[i * R + j]);
     } else {
-      tt.forward(v, tw, [] {});
+      tt.forward(v, [] {});
 #pragma unroll
       for (int q = 0; q < 16; q += 4) {
         Pair f[4];
@@ -535,13 +551,11 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
 #pragma unroll
         for (int m = 0; m < 4; ++m) v[q + m] = pswap(pmul(v[q + m], f[m]));
       }
-      tt.inverse(v, tw, release);
+      tt.inverse(v, release);
       float2 *o = a.dst_of(vol) + off;
 #pragma unroll
-      for (int i = 0; i < TT::B1; ++i)
-#pragma unroll
-        for (int e = 0; e < TT::R1; ++e)
-          stg_unit(o + ((tt.row * H + tt.t1(i) + TT::R2 * e) * C + tt.c) * 2, pswap(v[i * TT::R1 + e]));
+      for (int e = 0; e < 16; ++e)
+        stg_unit(o + ((tt.row * H + tt.t + TT::R2 * e) * C + tt.c) * 2, pswap(v[e]));
     }
   }
   // A group without a tile in the last round hands its buffers on all the same.
@@ -550,12 +564,7 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
     if (tid == 0 && n + B < loads && !st.marked()) load(n + B);
   }
   if (!ok) tp_gave_up(st, a.status);
-  if constexpr (MODE != TP_FWD) {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kCols));
-  }
+  tp_tmem_free<kCols>(tmem);
 }
 
 }  // namespace convgpu

@@ -12,7 +12,6 @@ import pytest
 
 # N: (J rows of the outer tile, C interleaved columns of the middle tile)
 SHAPES = {32: (8, 2), 64: (8, 4), 128: (16, 4), 256: (16, 2)}
-SPLIT = {256: (16, 16), 128: (16, 8), 64: (8, 8), 32: (8, 4), 16: (4, 4)}
 
 
 def _fwd(cube, j_rows, c_cols):
@@ -78,47 +77,95 @@ def test_two_pass_convolution_restated(n):
     assert np.linalg.norm(got - ref) < 1e-12 * np.linalg.norm(ref)
 
 
-def _tiles():
-    for n, (j_rows, c_cols) in SHAPES.items():
-        if n >= 128:
-            yield n, j_rows, 1
-            yield n // 2, n // j_rows, c_cols
+def _banks(units):
+    for at in range(0, len(units), 8):
+        assert len(set(units[at:at + 8] % 8)) == 8
 
 
-@pytest.mark.parametrize("n,j_rows,c_cols", list(_tiles()))
-def test_tile_slots(n, j_rows, c_cols):
-    """The row exchange's slots (tilefft.cuh: ex_w by its writers, ex_r by its readers) and the
-    column slots are permutations of the tile, both sides agree, and 8 consecutive lanes of
-    each access hit 8 different 16-byte bank groups."""
-    r1, r2 = SPLIT[n]
-    t_row = n // 16
-    nt = n * j_rows * c_cols // 16
-    sw = min(r2, 8) - 1
+@pytest.mark.parametrize("n", [128, 256])
+def test_outer_tile_slots(n):
+    """The outer tile's row exchange (written by ex_w, read by ex_r) and its column slots are
+    permutations of the tile, both sides agree, and 8 consecutive lanes of each access hit 8
+    different 16-byte bank groups."""
+    j_rows, r2 = SHAPES[n][0], n // 16
+    nt, sw = n * j_rows // 16, min(r2, 8) - 1
     tid = np.arange(nt)
-    c, t, row, colt = tid % c_cols, tid // c_cols % t_row, tid // (c_cols * t_row), tid // c_cols
-
-    def unit(row, i, c):
-        return (row * n + i) * c_cols + c
-
-    def banks(u):
-        for at in range(0, nt, 8):
-            assert len(set(u[at:at + 8] % 8)) == 8
+    t, row = tid % r2, tid // r2
     written, read, cols = {}, {}, set()
-    for i in range(16 // r1):
-        for k1 in range(r1):
-            u = unit(row, k1 * r2 + ((t + i * t_row) ^ (k1 & sw)), c)
-            banks(u)
-            written.update({int(a): (int(b), k1, int(d), int(e)) for a, b, d, e in zip(u, row, t + i * t_row, c)})
+    for k1 in range(16):
+        u = row * n + k1 * r2 + (t ^ (k1 & sw))
+        _banks(u)
+        written.update({int(a): (int(b), k1, int(c)) for a, b, c in zip(u, row, t)})
     for i in range(16 // r2):
         for tt in range(r2):
-            k1 = t + i * t_row
-            u = unit(row, k1 * r2 + (tt ^ (k1 & sw)), c)
-            banks(u)
-            read.update({int(a): (int(b), int(d), tt, int(e)) for a, b, d, e in zip(u, row, k1, c)})
-    assert written == read and sorted(written) == list(range(n * j_rows * c_cols))
+            k1 = t + i * r2
+            u = row * n + k1 * r2 + (tt ^ (k1 & sw))
+            _banks(u)
+            read.update({int(a): (int(b), int(c), tt) for a, b, c in zip(u, row, k1)})
+    assert written == read and sorted(written) == list(range(n * j_rows))
     for i in range(16 // j_rows):
         for j in range(j_rows):
-            u = unit(j, colt + i * (nt // c_cols), c)
-            banks(u)
+            u = j * n + tid + i * nt
+            _banks(u)
             cols.update(u.tolist())
-    assert cols == set(range(n * j_rows * c_cols))
+    assert cols == set(range(n * j_rows))
+
+
+def _trip(regs, col_of, reg_of):
+    """rows-shape store, fragment-shape load of one warp's 32 lanes x 64 columns. regs: {(lane,
+    label): value}; col_of(label): its column; returns {(lane, register): value}."""
+    cell = {(lane, col_of(label)): v for (lane, label), v in regs.items()}
+    out = {}
+    for lane in range(32):
+        for half in range(2):
+            for rep in range(8):
+                for q in range(4):
+                    row, col = 16 * half + lane // 4 + 8 * (q >> 1), 8 * rep + 2 * (lane % 4) + (q & 1)
+                    out[(lane, half * 32 + rep * 4 + q)] = cell[(row, col)]
+    return out
+
+
+@pytest.mark.parametrize("n", [128, 256])
+def test_middle_tile_exchange(n):
+    """Two trips through TMEM take unit (k1) of lane (l4..l0) to lane (l0, k1), register
+    s = (l4 l3 l2 l1); the twiddles between them are those of (t, k1); the shared-memory slots
+    that follow are a permutation of the warp's rows and free of bank conflicts."""
+    c_cols, r2 = SHAPES[n][1], n // 32
+    col1 = lambda k, w: (k >> 2) << 1 | (k >> 1 & 1) << 3 | w << 4 | (k & 1) << 5
+    frag1 = lambda m, w: (m >> 3) << 5 | (m & 1) << 4 | w << 3 | (m >> 1 & 1) << 2 | (m >> 2 & 1) << 1
+    col2 = lambda m, w: (m >> 3) << 5 | (m >> 2 & 1) << 4 | w << 3 | (m & 3) << 1
+    frag2 = lambda s, w: (s >> 1 & 1) << 5 | (s >> 2) << 3 | w << 2 | (s & 1) << 1
+    first = {(lane, (k, w, h)): (lane, k, w, h) for lane in range(32) for k in range(16) for w in range(2) for h in range(2)}
+    a = _trip(first, lambda x: col1(x[0], x[1]) + x[2], None)
+    between = {}
+    for lane in range(32):
+        for m in range(16):
+            for w in range(2):
+                for h in range(2):
+                    from_lane, k, w2, h2 = a[(lane, frag1(m, w) + h)]
+                    q = (lane >> 3) * 4 + (lane & 3)  # the table's entry m 16 + q is for this t and k1
+                    s = (m >> 2) << 2 | q >> 2
+                    assert (from_lane >> 1, k, w2, h2) == (s, (q & 3) << 2 | (m & 3), w, h)
+                    between[(lane, (m, w, h))] = (from_lane, k, w, h)
+    b = _trip(between, lambda x: col2(x[0], x[1]) + x[2], None)
+    for lane in range(32):
+        for s in range(16):
+            for w in range(2):
+                for h in range(2):
+                    assert b[(lane, frag2(s, w) + h)] == (s << 1 | lane >> 4, lane & 15, w, h)
+    # lane before = (row, t, c) = 16 row + C t + c; butterfly i's input t is unit_of(i, t)
+    unit_of = lambda i, t: i * 8 + t if c_cols == 2 else (i >> 1) * 8 + t * 2 + (i & 1)
+    slots = set()
+    for i in range(16 // r2):
+        for k2 in range(r2):
+            u = []
+            for lane in range(32):
+                l0 = lane >> 4
+                row, c = (i, l0) if c_cols == 2 else (i >> 1, (i & 1) * 2 + l0)
+                for t in range(r2):
+                    assert unit_of(i, t) << 1 | l0 == 16 * row + c_cols * t + c
+                kx = (lane & 15) + 16 * k2
+                u.append(row * (n // 2) * c_cols + kx * c_cols + (c ^ ((kx * c_cols // 8) & (c_cols - 1))))
+            _banks(np.array(u))
+            slots.update(u)
+    assert slots == set(range(n * c_cols))
