@@ -594,12 +594,35 @@ static size_t workspace_bytes_for(unsigned n, unsigned how_many, unsigned flags)
 // pass instead of as a pass of its own.
 constexpr unsigned kSharedFilterFusedMax = 2;
 
+static bool apart(const void *a, size_t an, const void *b, size_t bn) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x + an <= y || y + bn <= x;
+}
+
+// The one-launch path of 16^3 cubes reads a cube's operands before it writes its output, but
+// the cubes in any order: outputs must be the signals or apart from them, and apart from
+// the filters unless each is its own cube's.
+static bool cube16_takes(const float2 *sig, const float2 *filt, const float2 *out, unsigned how_many, unsigned flags) {
+  const size_t cube = 4096 * sizeof(float2), all = cube * how_many;
+  const size_t fbytes = ((flags & kFlagPerSignalFilter) ? all : cube) / ((flags & kFlagFilterReal) ? 2 : 1);
+  const bool own = filt == out && (flags & kFlagPerSignalFilter) && !(flags & kFlagFilterReal);
+  return (sig == out || apart(sig, all, out, all)) && (own || apart(filt, fbytes, out, all)) &&
+         how_many <= 0x7fffffffu;
+}
+
 // Whole convolution on device pointers, enqueued on stream s using workspace ws.
 static cudaError_t enqueue_conv_device(unsigned n, const float2 *sig, const float2 *filt, float2 *out,
                                        unsigned how_many, unsigned flags, float2 *ws, cudaStream_t s) {
   const float scale = (flags & kFlagNormalize) ? (float)(1.0 / ((double)n * n * n)) : 1.0f;
   const long long V = (long long)n * n * n;
   const int tc = tc_of(flags);
+  if (n == 16 && cube16_takes(sig, filt, out, how_many, flags)) {
+    const cudaError_t e =
+        launch_cube16(sig, filt, out, (int)how_many, (flags & kFlagPerSignalFilter) != 0,
+                      (flags & kFlagFilterReal) != 0, (flags & kFlagFilterIsSpectrum) != 0, scale, s);
+    if (e == cudaSuccess) count_launches(1);
+    return e;
+  }
   if (flags & kFlagFilterIsSpectrum) {
     const long long sv = (flags & kFlagPerSignalFilter) ? V : 0;
     return enqueue_signals(n, sig, out, filt, sv, OP_CONV, how_many, scale, s, nullptr, tc);

@@ -106,6 +106,15 @@ constexpr int kTpScratchCubes128 = 32, kTpScratchCubes256 = 4;
 int tp_scratch_cubes(int n);
 float2 *tp_scratch(int n, bool may_allocate);
 void release_tp();
+// Convolutions of 16^3 cubes in one launch, one CTA per cube (cube16.cu): filt holds one filter
+// (N^3 floats with `real`) for all or, with per_signal, one per cube, or spectra. A cube's
+// signal and filter are read before its output is written; no other filter may lie in it.
+// The table form takes device arrays of pointers (prepare_cube16 before a capture).
+cudaError_t launch_cube16(const float2 *sig, const void *filt, float2 *out, int cubes, bool per_signal, bool real,
+                          bool spectrum, float scale, cudaStream_t s);
+cudaError_t launch_cube16_table(const float2 *const *sigs, const float2 *const *filts, float2 *const *outs, int cubes,
+                                float scale, cudaStream_t s);
+cudaError_t prepare_cube16();
 // Fused x + y pass over `nplanes` planes (N = 128, 256, 512; cudaErrorNotSupported otherwise
 // or when tensor maps cannot describe the operands). Plan kind kKindXy, N = 256: variant 1
 // stages the x-transformed planes through an L2-resident scratch ring (one persistent

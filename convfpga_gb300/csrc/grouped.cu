@@ -33,7 +33,7 @@ namespace {
 // pass's rows maps (N = 256 and 128): filter, signal, out; then the two-pass transform's
 // maps of cubes in tile order: spectrum, out
 constexpr int kKinds = 12;
-enum XyForm { kXySeparate = 0, kXyStaged = 1, kXyTiles = 2 };
+enum XyForm { kXySeparate = 0, kXyStaged = 1, kXyTiles = 2, kWhole = 3 };  // kWhole: N = 16, one launch
 
 struct SizeGroup {
   int n = 0;
@@ -70,7 +70,7 @@ struct GPlan {
 };
 
 std::mutex g_mu;
-// key: job sizes, normalize + 2 * (form of N = 256 + 3 * form of N = 128)
+// key: job sizes, normalize + 2 * (form of N = 256, 128 and 16, base 4)
 std::map<std::pair<std::vector<int>, int>, std::unique_ptr<GPlan>> g_plans;
 
 cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, cudaStream_t s) {
@@ -79,6 +79,7 @@ cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, 
   float2 *const *spec = g.d_dsts;
   float2 *const *out = g.d_dsts + k;
   cudaError_t e;
+  if (g.xy == kWhole) return launch_cube16_table(g.d_dsts + 3 * k, g.d_dsts + 2 * k, out, k, scale, s);
   if (g.xy == kXyTiles) {
     if ((e = launch_tp_fwd_table(g.n, g.d_dsts + 2 * k, m + 10 * k, k, tw512, s)) != cudaSuccess) return e;
     if ((e = launch_tp_fwd_table(g.n, g.d_dsts + 3 * k, m + 11 * k, k, tw512, s)) != cudaSuccess) return e;
@@ -105,8 +106,8 @@ cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, 
   return launch_axis_pass_table(g.n, 0, OP_INV, m + 2 * k, nullptr, out, k, scale, tw512, s);
 }
 
-// f256, f128: form of the x and y passes for N = 256 and 128.
-cudaError_t build(GPlan &p, bool normalize, XyForm f256, XyForm f128, const float2 *tw512) {
+// f256, f128, f16: form of the classes N = 256, 128 and 16.
+cudaError_t build(GPlan &p, bool normalize, XyForm f256, XyForm f128, XyForm f16, const float2 *tw512) {
   std::map<int, int> idx;
   for (int j = 0; j < (int)p.sizes.size(); ++j) {
     const int n = p.sizes[j];
@@ -133,7 +134,8 @@ cudaError_t build(GPlan &p, bool normalize, XyForm f256, XyForm f128, const floa
     g.h_dsts.resize(4 * k);
     if ((e = cudaMalloc(&g.d_maps, sizeof(CUtensorMap) * kKinds * k)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&g.d_dsts, sizeof(float2 *) * 4 * k)) != cudaSuccess) return e;
-    g.xy = g.n == 256 ? f256 : (g.n == 128 ? f128 : kXySeparate);
+    g.xy = g.n == 256 ? f256 : (g.n == 128 ? f128 : (g.n == 16 ? f16 : kXySeparate));
+    if (g.xy == kWhole && (e = prepare_cube16()) != cudaSuccess) return e;
     if (g.xy == kXyTiles && (e = prepare_tp(g.n)) != cudaSuccess) return e;
     if (g.xy == kXyStaged) {
       if ((e = prepare_xy_l2(g.n)) != cudaSuccess) return e;
@@ -217,12 +219,22 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
     return v == 1 || v == kXyTwoPass ? kXyStaged : kXySeparate;
   };
   const XyForm f256 = form(256), f128 = form(128);
-  auto key = std::make_pair(sizes, (normalize ? 1 : 0) + 2 * (f256 + 3 * f128));
+  // 16^3 jobs run whole, in any order: no filter of theirs may lie among their outputs.
+  uintptr_t flo = ~(uintptr_t)0, fhi = 0, olo = ~(uintptr_t)0, ohi = 0;
+  for (unsigned j = 0; j < njobs; ++j) {
+    if (sizes[j] != 16) continue;
+    const uintptr_t bytes = 4096 * sizeof(float2), f = reinterpret_cast<uintptr_t>(ptrs[3 * j + 1]),
+                    o = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
+    flo = std::min(flo, f), fhi = std::max(fhi, f + bytes);
+    olo = std::min(olo, o), ohi = std::max(ohi, o + bytes);
+  }
+  const XyForm f16 = (fhi <= olo || ohi <= flo) ? kWhole : kXySeparate;
+  auto key = std::make_pair(sizes, (normalize ? 1 : 0) + 2 * (f256 + 4 * f128 + 16 * f16));
   auto it = g_plans.find(key);
   if (it == g_plans.end()) {
     auto p = std::make_unique<GPlan>();
     p->sizes = sizes;
-    cudaError_t e = build(*p, normalize, f256, f128, tw512);
+    cudaError_t e = build(*p, normalize, f256, f128, f16, tw512);
     if (e != cudaSuccess) {
       err = std::string("uneven grouped plan: ") + cudaGetErrorString(e);
       cudaGetLastError();
