@@ -507,9 +507,10 @@ static cudaError_t pass_tp(int slot, double bytes, cudaStream_t s, F &&launch) {
   }
   return e;
 }
-static cudaError_t tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, cudaStream_t s) {
-  return pass_tp(12, (real ? 28.0 : 32.0) * n * n * n * nvol, s,
-                 [&] { return launch_tp_fwd(n, src, dst, nvol, real, g.tw512, s); });
+static cudaError_t tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, cudaStream_t s,
+                          const float2 *src2 = nullptr, float2 *dst2 = nullptr, int nvol2 = 0) {
+  return pass_tp(12, (real ? 28.0 : 32.0) * n * n * n * (nvol + nvol2), s,
+                 [&] { return launch_tp_fwd(n, src, dst, nvol, real, g.tw512, s, src2, dst2, nvol2); });
 }
 static cudaError_t tp_mid(int n, int mode, const float2 *src, float2 *dst, const float2 *filt, long long filt_vol,
                           int nvol, cudaStream_t s) {
@@ -521,10 +522,13 @@ static cudaError_t tp_inv(int n, const float2 *src, float2 *dst, int nvol, float
   return pass_tp(13, 32.0 * n * n * n * nvol, s, [&] { return launch_tp_inv(n, src, dst, nvol, scale, g.tw512, s); });
 }
 
-// Largest batch for which a shared filter's second pass runs inside every signal's middle
-// pass (TP_PAIR) instead of once before them (TP_FWD, then TP_SPECTRUM). Measured, us a
-// cube: 256^3 80 with it, 69 without and 46 once for the filter; 128^3 10, 8.1 and 6.
-constexpr unsigned kTpSharedPairMax = 3;
+// A shared filter's second pass runs inside every signal's middle pass (TP_PAIR) for small
+// batches, and otherwise once before them (TP_FWD, then TP_SPECTRUM): a quarter of the middle
+// pass's work for every cube against one more launch and the filter's own tiles. Measured, us,
+// inside / once: 32^3 x17 22.0 / 24.6, x100 63.4 / 64.5, x300 128.3 / 125.1; 64^3 x8 38.8 /
+// 41.1, x17 64.8 / 64.7, x100 253.7 / 239.2; 128^3 x4 106.1 / 104.3; 256^3 x3 582.5 / 584.0.
+constexpr unsigned kTpSharedPairCubes = 3;
+constexpr long long kTpSharedPairPoints = 1ll << 22;
 
 // Convolutions by the two-pass transform. With a filter per signal and outputs of their own,
 // signals go through the outputs and back through the filters' workspace, all at once;
@@ -544,31 +548,34 @@ static cudaError_t enqueue_tp(int n, const float2 *sig, const float2 *filt, floa
   const bool direct = pairs && !overlap;
   float2 *scratch = tp_scratch(n, !capturing(s));
   if (!direct && !scratch) return cudaErrorNotSupported;
+  // Filters are read before any output is written: a caller may convolve into them.
+  const uintptr_t fbytes = (uintptr_t)V * (per_signal ? how_many : 1) * (real ? 4 : 8);
+  const bool filters_apart = fu + fbytes <= ou || ou + bytes <= fu;
   if (direct) {
-    CG_TRY(tp_fwd(n, filt, ws, how_many, real, s));
-    CG_TRY(tp_fwd(n, sig, out, how_many, false, s));
+    if (!real && filters_apart) {
+      CG_TRY(tp_fwd(n, filt, ws, how_many, false, s, sig, out, how_many));
+    } else {
+      CG_TRY(tp_fwd(n, filt, ws, how_many, real, s));
+      CG_TRY(tp_fwd(n, sig, out, how_many, false, s));
+    }
     CG_TRY(tp_mid(n, kTpPair, out, ws, ws, V, how_many, s));
     CG_TRY(tp_inv(n, ws, out, how_many, scale, s));
     return cudaSuccess;
   }
   const unsigned chunk = std::min<unsigned>(how_many, tp_scratch_cubes(n));
-  // Filters are read before any output is written: a caller may convolve into them.
-  const uintptr_t fbytes = (uintptr_t)V * (per_signal ? how_many : 1) * (real ? 4 : 8);
-  const bool filters_first = !per_signal || (fu < ou + bytes && ou < fu + fbytes);
-  const bool spectrum = !per_signal && how_many > kTpSharedPairMax;
-  if (filters_first) CG_TRY(tp_fwd(n, filt, ws, per_signal ? how_many : 1, real, s));
+  const bool spectrum = !per_signal && how_many > kTpSharedPairCubes && V * how_many > kTpSharedPairPoints;
+  // All filters go with the first chunk of signals (into the scratch), in one launch unless
+  // they are real.
+  const int nf = per_signal ? (int)how_many : 1;
+  if (real)
+    CG_TRY(tp_fwd(n, filt, ws, nf, true, s));
+  else
+    CG_TRY(tp_fwd(n, filt, ws, nf, false, s, sig, scratch, (int)chunk));
   if (spectrum) CG_TRY(tp_mid(n, kTpFwd, ws, ws, nullptr, 0, 1, s));
   for (unsigned i = 0; i < how_many; i += chunk) {
     const int k = (int)std::min(chunk, how_many - i);
-    const float2 *f = ws;
-    if (per_signal) {
-      if (filters_first)
-        f = ws + i * V;
-      else
-        CG_TRY(tp_fwd(n, real ? (const void *)((const float *)(const void *)filt + i * V) : (const void *)(filt + i * V),
-                      ws, k, real, s));
-    }
-    CG_TRY(tp_fwd(n, sig + i * V, scratch, k, false, s));
+    const float2 *f = per_signal ? ws + i * V : ws;
+    if (real || i > 0) CG_TRY(tp_fwd(n, sig + i * V, scratch, k, false, s));
     CG_TRY(tp_mid(n, spectrum ? kTpSpectrum : kTpPair, scratch, scratch, f, per_signal ? V : 0, k, s));
     CG_TRY(tp_inv(n, scratch, out + i * V, k, scale, s));
   }

@@ -71,7 +71,7 @@ cudaError_t launch_xy_l2_tc_pass(int n, const float2 *src, float2 *dst, int npla
 int pass_kind(int axis, int op);
 void set_pass_variant(int n, int kind, int variant);
 int get_pass_variant(int n, int kind);
-// Plan kind kKindXy, variant 3 (N = 128 and 256): the two-pass 3D transform (twopass.cuh) in
+// Plan kind kKindXy, variant 3 (N = 32 to 256): the two-pass 3D transform (twopass.cuh) in
 // place of the x, y and z passes, for the calls it takes; the others run variant 1.
 constexpr int kXyTwoPass = 3;
 bool tp_size(int n);
@@ -79,10 +79,11 @@ bool tp_size(int n);
 constexpr int kTpPair = 0, kTpSpectrum = 1, kTpFwd = 2;
 // Forward outer pass (cubes, or N^3 floats each with `real`, to tile order), middle pass, and
 // inverse outer pass (tile order to cubes). src and dst of the outer passes must not
-// overlap; the middle pass may write over its source or its filters. cudaErrorNotSupported
+// overlap; the middle pass may write over its source or its filters. The forward pass can
+// take a second set of (complex) cubes along. cudaErrorNotSupported
 // when an operand is not 16-byte aligned.
 cudaError_t launch_tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, const float2 *tw512,
-                          cudaStream_t s);
+                          cudaStream_t s, const float2 *src2 = nullptr, float2 *dst2 = nullptr, int nvol2 = 0);
 cudaError_t launch_tp_mid(int n, int mode, const float2 *src, float2 *dst, const float2 *filt, long long filt_vol,
                           int nvol, const float2 *tw512, cudaStream_t s);
 cudaError_t launch_tp_inv(int n, const float2 *src, float2 *dst, int nvol, float scale, const float2 *tw512,
@@ -98,11 +99,11 @@ cudaError_t launch_tp_mid_table(int n, const float2 *const *srcs, float2 *const 
                                 int nvol, const float2 *tw512, cudaStream_t s);
 cudaError_t launch_tp_inv_table(int n, const CUtensorMap *src_maps, float2 *const *dsts, int nvol, float scale,
                                 const float2 *tw512, cudaStream_t s);
-// The process's scratch cubes in tile order, tp_scratch_cubes(n) of them (512 MiB): the
-// signals a call transforms at a time. Fewer cost more in launches than L2 gives back: a
+// The process's scratch cubes in tile order, tp_scratch_cubes(n) of them (512 MiB, 256 at
+// N = 64, 128 at N = 32): the signals a call transforms at a time. Fewer cost more in launches than L2 gives back: a
 // call of 16 cubes of 128^3 took 403 us by 4, 357 by 8 and 339 at once. Null when not
 // allocated and not (or not to be) allocatable.
-constexpr int kTpScratchCubes128 = 32, kTpScratchCubes256 = 4;
+constexpr int kTpScratchCubes32 = 512, kTpScratchCubes64 = 128, kTpScratchCubes128 = 32, kTpScratchCubes256 = 4;
 int tp_scratch_cubes(int n);
 float2 *tp_scratch(int n, bool may_allocate);
 void release_tp();

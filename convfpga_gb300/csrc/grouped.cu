@@ -33,7 +33,10 @@ namespace {
 // pass's rows maps (N = 256 and 128): filter, signal, out; then the two-pass transform's
 // maps of cubes in tile order: spectrum, out
 constexpr int kKinds = 12;
-enum XyForm { kXySeparate = 0, kXyStaged = 1, kXyTiles = 2, kWhole = 3 };  // kWhole: N = 16, one launch
+// kXyTiles: filters and signals forward in one launch; kXyTilesOrdered: one after the other,
+// where a filter lies among the outputs. kWhole: N = 16, one launch.
+enum XyForm { kXySeparate = 0, kXyStaged = 1, kXyTiles = 2, kXyTilesOrdered = 3, kWhole = 4 };
+static bool tiles(XyForm f) { return f == kXyTiles || f == kXyTilesOrdered; }
 
 struct SizeGroup {
   int n = 0;
@@ -70,7 +73,7 @@ struct GPlan {
 };
 
 std::mutex g_mu;
-// key: job sizes, normalize + 2 * (form of N = 256, 128 and 16, base 4)
+// key: job sizes, normalize + 2 * (form of each size, base 5)
 std::map<std::pair<std::vector<int>, int>, std::unique_ptr<GPlan>> g_plans;
 
 cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, cudaStream_t s) {
@@ -80,9 +83,10 @@ cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, 
   float2 *const *out = g.d_dsts + k;
   cudaError_t e;
   if (g.xy == kWhole) return launch_cube16_table(g.d_dsts + 3 * k, g.d_dsts + 2 * k, out, k, scale, s);
-  if (g.xy == kXyTiles) {
-    if ((e = launch_tp_fwd_table(g.n, g.d_dsts + 2 * k, m + 10 * k, k, tw512, s)) != cudaSuccess) return e;
-    if ((e = launch_tp_fwd_table(g.n, g.d_dsts + 3 * k, m + 11 * k, k, tw512, s)) != cudaSuccess) return e;
+  if (tiles(g.xy)) {
+    const int both = g.xy == kXyTiles ? 2 * k : k;  // filters, then signals
+    if ((e = launch_tp_fwd_table(g.n, g.d_dsts + 2 * k, m + 10 * k, both, tw512, s)) != cudaSuccess) return e;
+    if (both == k && (e = launch_tp_fwd_table(g.n, g.d_dsts + 3 * k, m + 11 * k, k, tw512, s)) != cudaSuccess) return e;
     if ((e = launch_tp_mid_table(g.n, out, spec, spec, k, tw512, s)) != cudaSuccess) return e;
     return launch_tp_inv_table(g.n, m + 10 * k, out, k, scale, tw512, s);
   }
@@ -106,8 +110,13 @@ cudaError_t enqueue_group(const SizeGroup &g, float scale, const float2 *tw512, 
   return launch_axis_pass_table(g.n, 0, OP_INV, m + 2 * k, nullptr, out, k, scale, tw512, s);
 }
 
-// f256, f128, f16: form of the classes N = 256, 128 and 16.
-cudaError_t build(GPlan &p, bool normalize, XyForm f256, XyForm f128, XyForm f16, const float2 *tw512) {
+// Form of each size class, and where they stand.
+struct Forms {
+  XyForm of[6] = {};
+  static int index(int n) { return n == 16 ? 0 : (n == 32 ? 1 : (n == 64 ? 2 : (n == 128 ? 3 : (n == 256 ? 4 : 5)))); }
+};
+
+cudaError_t build(GPlan &p, bool normalize, const Forms &forms, const float2 *tw512) {
   std::map<int, int> idx;
   for (int j = 0; j < (int)p.sizes.size(); ++j) {
     const int n = p.sizes[j];
@@ -134,9 +143,9 @@ cudaError_t build(GPlan &p, bool normalize, XyForm f256, XyForm f128, XyForm f16
     g.h_dsts.resize(4 * k);
     if ((e = cudaMalloc(&g.d_maps, sizeof(CUtensorMap) * kKinds * k)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&g.d_dsts, sizeof(float2 *) * 4 * k)) != cudaSuccess) return e;
-    g.xy = g.n == 256 ? f256 : (g.n == 128 ? f128 : (g.n == 16 ? f16 : kXySeparate));
+    g.xy = forms.of[Forms::index(g.n)];
     if (g.xy == kWhole && (e = prepare_cube16()) != cudaSuccess) return e;
-    if (g.xy == kXyTiles && (e = prepare_tp(g.n)) != cudaSuccess) return e;
+    if (tiles(g.xy) && (e = prepare_tp(g.n)) != cudaSuccess) return e;
     if (g.xy == kXyStaged) {
       if ((e = prepare_xy_l2(g.n)) != cudaSuccess) return e;
       if ((e = cudaMalloc(&g.d_ctr, xy_l2_counter_bytes(g.n, (int)k))) != cudaSuccess) return e;
@@ -156,15 +165,16 @@ cudaError_t build(GPlan &p, bool normalize, XyForm f256, XyForm f128, XyForm f16
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    // Classes of the two-pass transform run one after another, before the others: a CTA of
-    // theirs holds an SM and a fixed share of the tiles, so kernels beside it would leave
-    // some CTAs waiting for an SM.
+    // Large classes of the two-pass transform run one after another, before the others: a CTA
+    // of theirs holds an SM and a fixed share of the tiles, so kernels beside it would leave
+    // some CTAs waiting for an SM. Classes below 128 (a few percent of the points of a
+    // mixed batch) run side by side after them.
     auto scale_of = [&](int n) { return normalize ? (float)(1.0 / ((double)n * n * n)) : 1.0f; };
     for (auto &g : p.groups)
-      if (g.xy == kXyTiles && e == cudaSuccess) e = enqueue_group(g, scale_of(g.n), tw512, cap);
+      if (tiles(g.xy) && g.n >= 128 && e == cudaSuccess) e = enqueue_group(g, scale_of(g.n), tw512, cap);
     cudaEventRecord(ev.back(), cap);
     for (size_t gi = 0; gi < p.groups.size() && e == cudaSuccess; ++gi) {
-      if (p.groups[gi].xy == kXyTiles) continue;
+      if (tiles(p.groups[gi].xy) && p.groups[gi].n >= 128) continue;
       const float scale = scale_of(p.groups[gi].n);
       cudaStreamWaitEvent(br[gi], ev.back(), 0);
       e = enqueue_group(p.groups[gi], scale, tw512, br[gi]);
@@ -205,6 +215,18 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
   // The L2-staged variant (1) and the two-pass transform (3) have table modes. The latter
   // takes signals through their outputs, so a class with a job in place (or partly so) runs
   // the former, as does every class when tensor maps are switched off.
+  // No filter of a class lies among its outputs (by the ranges they span).
+  auto filters_apart = [&](int n) {
+    uintptr_t flo = ~(uintptr_t)0, fhi = 0, olo = ~(uintptr_t)0, ohi = 0;
+    for (unsigned j = 0; j < njobs; ++j) {
+      if (sizes[j] != n) continue;
+      const uintptr_t bytes = (uintptr_t)n * n * n * sizeof(float2), f = reinterpret_cast<uintptr_t>(ptrs[3 * j + 1]),
+                      o = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
+      flo = std::min(flo, f), fhi = std::max(fhi, f + bytes);
+      olo = std::min(olo, o), ohi = std::max(ohi, o + bytes);
+    }
+    return fhi <= olo || ohi <= flo;
+  };
   auto form = [&](int n) {
     const int v = get_pass_variant(n, kKindXy);
     if (v == kXyTwoPass && tma_enabled()) {
@@ -214,27 +236,22 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
         const uintptr_t su = reinterpret_cast<uintptr_t>(ptrs[3 * j]), ou = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
         if (sizes[j] == n && su < ou + bytes && ou < su + bytes) apart = false;
       }
-      if (apart) return kXyTiles;
+      if (apart) return filters_apart(n) ? kXyTiles : kXyTilesOrdered;
     }
-    return v == 1 || v == kXyTwoPass ? kXyStaged : kXySeparate;
+    return n >= 128 && (v == 1 || v == kXyTwoPass) ? kXyStaged : kXySeparate;
   };
-  const XyForm f256 = form(256), f128 = form(128);
-  // 16^3 jobs run whole, in any order: no filter of theirs may lie among their outputs.
-  uintptr_t flo = ~(uintptr_t)0, fhi = 0, olo = ~(uintptr_t)0, ohi = 0;
-  for (unsigned j = 0; j < njobs; ++j) {
-    if (sizes[j] != 16) continue;
-    const uintptr_t bytes = 4096 * sizeof(float2), f = reinterpret_cast<uintptr_t>(ptrs[3 * j + 1]),
-                    o = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
-    flo = std::min(flo, f), fhi = std::max(fhi, f + bytes);
-    olo = std::min(olo, o), ohi = std::max(ohi, o + bytes);
-  }
-  const XyForm f16 = (fhi <= olo || ohi <= flo) ? kWhole : kXySeparate;
-  auto key = std::make_pair(sizes, (normalize ? 1 : 0) + 2 * (f256 + 4 * f128 + 16 * f16));
+  Forms forms;
+  for (int n : {32, 64, 128, 256}) forms.of[Forms::index(n)] = form(n);
+  // 16^3 jobs run whole, in any order
+  forms.of[0] = filters_apart(16) ? kWhole : kXySeparate;
+  int form_key = 0;
+  for (XyForm f : forms.of) form_key = 5 * form_key + f;
+  auto key = std::make_pair(sizes, (normalize ? 1 : 0) + 2 * form_key);
   auto it = g_plans.find(key);
   if (it == g_plans.end()) {
     auto p = std::make_unique<GPlan>();
     p->sizes = sizes;
-    cudaError_t e = build(*p, normalize, f256, f128, f16, tw512);
+    cudaError_t e = build(*p, normalize, forms, tw512);
     if (e != cudaSuccess) {
       err = std::string("uneven grouped plan: ") + cudaGetErrorString(e);
       cudaGetLastError();
@@ -257,7 +274,7 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
                   encode_table_map(&g.h_maps[2 * k + v], ot, g.n, 0) && encode_table_map(&g.h_maps[3 * k + v], sp, g.n, 1) &&
                   encode_table_map(&g.h_maps[4 * k + v], ot, g.n, 1) && encode_table_map(&g.h_maps[5 * k + v], ot, g.n, 2) &&
                   encode_table_map(&g.h_maps[6 * k + v], sp, g.n, 2);
-        if (ok && g.xy == kXyTiles)
+        if (ok && tiles(g.xy))
           ok = tp_encode_tiles(&g.h_maps[10 * k + v], sp, g.n, 1) && tp_encode_tiles(&g.h_maps[11 * k + v], ot, g.n, 1);
         if (ok && g.xy == kXyStaged)
           ok = encode_xy_table_map(&g.h_maps[7 * k + v], ft, g.n) &&

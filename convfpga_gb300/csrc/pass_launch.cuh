@@ -56,7 +56,7 @@ bool encode_rows_map(CUtensorMap *m, const void *base, int n, long long rows, in
 bool encode_rows512_map(CUtensorMap *m, const void *base, long long rows, int xc);
 // Tile order of the two-pass transform: runs of `vals` complex values, `runs` to a tile;
 // dims (vals, tiles, runs), box {vals, box_tiles, 1}, 16-byte chunks swizzled over the box's
-// row size (32 or 64 bytes).
+// row size (32, 64 or 128 bytes).
 bool encode_runs_map(CUtensorMap *m, const void *base, int vals, long long tiles, int runs, int box_tiles);
 // As encode_cube_map over planes of N rows of `width` complex values (row pitch = width).
 bool encode_pitched_map(CUtensorMap *m, const void *base, int width, int n, long long nplanes, int axis, int cols);

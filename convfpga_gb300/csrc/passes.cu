@@ -120,14 +120,16 @@ bool encode_rows512_map(CUtensorMap *m, const void *base, long long rows, int xc
 
 bool encode_runs_map(CUtensorMap *m, const void *base, int vals, long long tiles, int runs, int box_tiles) {
   auto enc = tensor_map_encoder();
-  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15u) != 0 || tiles > 0x7fffffffLL || (vals != 4 && vals != 8))
+  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15u) != 0 || tiles > 0x7fffffffLL || (vals != 4 && vals != 8 && vals != 16))
     return false;
   cuuint64_t dims[3] = {(cuuint64_t)vals, (cuuint64_t)tiles, (cuuint64_t)runs};
   cuuint64_t strides[2] = {(cuuint64_t)vals * runs * 8, (cuuint64_t)vals * 8};
   cuuint32_t box[3] = {(cuuint32_t)vals, (cuuint32_t)box_tiles, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void *>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, vals == 4 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   vals == 4 ? CU_TENSOR_MAP_SWIZZLE_32B
+                             : (vals == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B),
                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -189,9 +191,11 @@ static bool g_use_tma = true;
 void set_tma_enabled(bool on) { g_use_tma = on; }
 bool tma_enabled() { return g_use_tma; }
 
-// Every size starts with shape variant 0; x and y of N = 128 and 256 with the two-pass
+// Every size starts with shape variant 0; x and y of N = 32 to 256 with the two-pass
 // transform, which was faster than the other forms on every working set measured.
-static std::atomic<int> g_variant[6][kPassKinds] = {{}, {}, {}, {0, 0, 0, 0, kXyTwoPass}, {0, 0, 0, 0, kXyTwoPass}, {}};
+#define CG_TWO_PASS {0, 0, 0, 0, kXyTwoPass}
+static std::atomic<int> g_variant[6][kPassKinds] = {{}, CG_TWO_PASS, CG_TWO_PASS, CG_TWO_PASS, CG_TWO_PASS, {}};
+#undef CG_TWO_PASS
 
 static int size_index(int n) {
   switch (n) {

@@ -84,6 +84,15 @@ template <int R>
 struct PDft;
 
 template <>
+struct PDft<2> {
+  static __device__ __forceinline__ void run(Pair *x) {
+    const Pair a = x[0], b = x[1];
+    x[0] = padd(a, b);
+    x[1] = psub(a, b);
+  }
+};
+
+template <>
 struct PDft<4> {
   static __device__ __forceinline__ void run(Pair *x) { pdft4(x[0], x[1], x[2], x[3]); }
 };
@@ -186,6 +195,31 @@ __device__ __forceinline__ float lds_f(uint32_t a) {
   return v;
 }
 
+// Barrier of a group of NT threads: named, or its warp's.
+template <int NT>
+__device__ __forceinline__ void group_sync(int id) {
+  if constexpr (NT == 32)
+    __syncwarp();
+  else
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(NT) : "memory");
+}
+
+// Whether any of the group's threads says so, at a barrier of the group.
+template <int NT>
+__device__ __forceinline__ bool group_any(int id, bool v) {
+  if constexpr (NT == 32) return __any_sync(~0u, v);
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %3, 0;\n\t"
+      "bar.red.or.pred p, %1, %2, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(any)
+      : "r"(id), "n"(NT), "r"((uint32_t)v)
+      : "memory");
+  return any != 0;
+}
+
 // Transform of J rows of N = 16 R2 units along the rows and across them, by a group of
 // N J / 16 threads with a named barrier of its own, both exchanges in the shared-memory tile.
 // A thread holds 16 units; the T = R2 threads of a row are neighbours in one warp, so the
@@ -226,9 +260,7 @@ struct OuterTile {
     base = tile_addr;
     rowb = tile_addr + row * ROWB;
   }
-  __device__ __forceinline__ void sync() const {
-    asm volatile("bar.sync %0, %1;" ::"r"(barrier), "n"(NT) : "memory");
-  }
+  __device__ __forceinline__ void sync() const { group_sync<NT>(barrier); }
   // slots: kx of this thread's row; (k1, t) by its writers and its readers; column
   __device__ __forceinline__ uint32_t nat(int x) const { return rowb + x * 16; }
   __device__ __forceinline__ uint32_t ex_w(int k1) const { return rowb + (t ^ (k1 & SW)) * 16 + k1 * (R2 * 16); }
@@ -483,7 +515,8 @@ struct MidTile {
   static constexpr int B2 = U / R2, B3 = U / J;   // butterflies per thread
   static constexpr int ROWB = N * C * 16;         // bytes per row
   static constexpr int BYTES = J * ROWB;
-  static_assert(T * C == 16 && (C == 2 || C == 4), "two rows to a warp");
+  static constexpr int HC = C / 2;                // interleaves that l4..l1 hold: lane = (row, t, c)
+  static_assert(T * C == 16 && C >= 2, "two rows to a warp");
   static_assert(U % J == 0 && NT % 32 == 0, "16 units per thread");
 
   int c, t, row, colt, barrier, k1;
@@ -505,9 +538,7 @@ struct MidTile {
     base = tile_addr;
     rowb = tile_addr + row * ROWB + c * 16;
   }
-  __device__ __forceinline__ void sync() const {
-    asm volatile("bar.sync %0, %1;" ::"r"(barrier), "n"(NT) : "memory");
-  }
+  __device__ __forceinline__ void sync() const { group_sync<NT>(barrier); }
   // Natural unit x of this thread's row as a load left it.
   __device__ __forceinline__ uint32_t nat(int x) const { return rowb + x * (C * 16); }
   // Slot (kx, c) in a row.
@@ -518,12 +549,11 @@ struct MidTile {
   // After the exchange: unit s of butterfly i's input t, and its row and interleave (l0 is
   // lane bit 4 now).
   static constexpr int unit_of(int i, int tt) {
-    return C == 2 ? i * 8 + tt : (i >> 1) * 8 + tt * 2 + (i & 1);
+    return (i / HC) * 8 + tt * HC + i % HC;
   }
   __device__ __forceinline__ uint32_t out(int i, int k2) const {
-    const int l0 = (threadIdx.x >> 4) & 1, row0 = row & ~1;
-    const int r = row0 + (C == 2 ? i : i >> 1), cc = C == 2 ? l0 : (i & 1) * 2 + l0;
-    return base + r * ROWB + slot(k1 + 16 * k2, cc);
+    const int l0 = (threadIdx.x >> 4) & 1;
+    return base + ((row & ~1) + i / HC) * ROWB + slot(k1 + 16 * k2, (i % HC) * 2 + l0);
   }
 
   // v[e] = unit t + R2 e of the row on entry; on exit v[i J + j'] = transform at row output
@@ -531,24 +561,29 @@ struct MidTile {
   // after_read() runs once the tile's last read is done by this thread.
   template <class F>
   __device__ __forceinline__ void forward(Pair (&v)[U], F &&after_read) const {
-    uint32_t r[64];
     PDft<16>::run(v);
+    if constexpr (R2 == 1) {  // a row is one thread's
 #pragma unroll
-    for (int k = 0; k < 16; ++k) put_pair(r, tm_col1(k, 0), tm_col1(k, 1), v[k]);
-    __syncwarp();
-    tm_st_rows(tm, r);  // lanes (l4 .. l0)
-    tm_ld_frag(tm, r);  // lanes (l2 l1 l0 k3 k2)
-    tm_twiddle<false>(r, tml);
-    tm_st_rows(tm, r);
-    tm_ld_frag(tm, r);  // lanes (l0 k3 k2 k1 k0)
+      for (int k = 0; k < 16; ++k) sts_pair(base + row * ROWB + slot(k, c), v[k]);
+    } else {
+      uint32_t r[64];
 #pragma unroll
-    for (int i = 0; i < B2; ++i) {
-      Pair x[R2];
+      for (int k = 0; k < 16; ++k) put_pair(r, tm_col1(k, 0), tm_col1(k, 1), v[k]);
+      __syncwarp();
+      tm_st_rows(tm, r);  // lanes (l4 .. l0)
+      tm_ld_frag(tm, r);  // lanes (l2 l1 l0 k3 k2)
+      tm_twiddle<false>(r, tml);
+      tm_st_rows(tm, r);
+      tm_ld_frag(tm, r);  // lanes (l0 k3 k2 k1 k0)
 #pragma unroll
-      for (int tt = 0; tt < R2; ++tt) x[tt] = get_pair(r, tm_frag2(unit_of(i, tt), 0), tm_frag2(unit_of(i, tt), 1));
-      PDft<R2>::run(x);
+      for (int i = 0; i < B2; ++i) {
+        Pair x[R2];
 #pragma unroll
-      for (int k = 0; k < R2; ++k) sts_pair(out(i, k), x[k]);
+        for (int tt = 0; tt < R2; ++tt) x[tt] = get_pair(r, tm_frag2(unit_of(i, tt), 0), tm_frag2(unit_of(i, tt), 1));
+        PDft<R2>::run(x);
+#pragma unroll
+        for (int k = 0; k < R2; ++k) sts_pair(out(i, k), x[k]);
+      }
     }
     sync();
 #pragma unroll
@@ -565,7 +600,6 @@ struct MidTile {
   // read is done.
   template <class F>
   __device__ __forceinline__ void inverse(Pair (&v)[U], F &&after_read) const {
-    uint32_t r[64];
 #pragma unroll
     for (int i = 0; i < B3; ++i) {
       PDft<J>::run(v + i * J);
@@ -573,6 +607,18 @@ struct MidTile {
       for (int j = 0; j < J; ++j) sts_pair(col(i, j), v[i * J + j]);
     }
     sync();
+    if constexpr (R2 == 1) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = lds_pair(base + row * ROWB + slot(k, c));
+      after_read();
+    } else {
+      back_along_rows(v, after_read);
+    }
+    PDft<16>::run(v);
+  }
+  template <class F>
+  __device__ __forceinline__ void back_along_rows(Pair (&v)[U], F &&after_read) const {
+    uint32_t r[64];
 #pragma unroll
     for (int i = 0; i < B2; ++i)
 #pragma unroll
@@ -593,7 +639,6 @@ struct MidTile {
     tm_ld_rows(tm, r);
 #pragma unroll
     for (int k = 0; k < 16; ++k) v[k] = get_pair(r, tm_col1(k, 0), tm_col1(k, 1));
-    PDft<16>::run(v);
   }
 
   // Twiddle table (4 KB) in shared memory, by a thread's place between the two trips: entry
@@ -604,7 +649,7 @@ struct MidTile {
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
       const int m = i >> 4, q = i & 15;
       const int s = (m >> 2) << 2 | q >> 2, k = (q & 3) << 2 | (m & 3);  // s = (l4 l3 l2 l1)
-      const int tt = C == 2 ? s & 7 : (s >> 1) & 3;
+      const int tt = (s / HC) % R2;
       const float2 w = __ldg(tw512 + tt * k * (512 / N));
       sts_pair(tw + i * 16, Pair{pk(w.x, w.x), pk(-w.y, -w.y)});
     }

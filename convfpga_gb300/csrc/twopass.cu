@@ -1,4 +1,4 @@
-// Launchers of the two-pass 3D transform (twopass.cuh) for N = 128 and 256, and its scratch
+// Launchers of the two-pass 3D transform (twopass.cuh) for N = 32 to 256, and its scratch
 // cubes. One persistent CTA per SM; launches read their operands through plain pointers, and
 // only the runs of tile order go through a tensor map.
 #define CONVGPU_PASS_LAUNCH_IMPL
@@ -7,10 +7,11 @@
 #include "twopass.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace convgpu {
 
-bool tp_size(int n) { return n == 128 || n == 256; }
+bool tp_size(int n) { return n == 32 || n == 64 || n == 128 || n == 256; }
 
 namespace {
 
@@ -27,23 +28,33 @@ cudaError_t launch(K kern, int &done, int smem, int threads, long long tiles, cu
   if (tiles <= 0 || tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const cudaError_t e = set_smem_once(kern, smem, done);
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)std::min<long long>(tiles, sm_count()), threads, smem, s>>>(args...);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)std::min<long long>(tiles, sm_count()));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 template <int N>
 bool encode_tiles(CUtensorMap *m, const void *cubes, int nvol) {
   using S = TpShape<N>;
-  return encode_runs_map(m, cubes, 2 * S::C, (long long)nvol * N * S::J / S::C, (N / S::J) * (N / 2), N);
+  return encode_runs_map(m, cubes, 2 * kTpBox<N>, (long long)nvol * N * S::J / S::C,
+                         (N / S::J) * (N / 2) * (S::C / kTpBox<N>), N);
 }
 
 template <int N>
-cudaError_t fwd(const TpArgs &a, bool real, const CUtensorMap &m, cudaStream_t s) {
+cudaError_t fwd(const TpArgs &a, bool real, const CUtensorMap &m, const CUtensorMap &m2, cudaStream_t s) {
   const long long tiles = (long long)a.nvol * (N / TpShape<N>::J) * (N / 2);
   static int done[2] = {0, 0};
-  constexpr int smem = tp_outer_smem<N>(), threads = kTpThreads<N> + 32;
-  return real ? launch(k_tp_fwd<N, true>, done[1], smem, threads, tiles, s, m, a)
-              : launch(k_tp_fwd<N, false>, done[0], smem, threads, tiles, s, m, a);
+  constexpr int smem = tp_outer_smem<N>(), threads = kTpFwdThreads<N>;
+  return real ? launch(k_tp_fwd<N, true>, done[1], smem, threads, tiles, s, m, m2, a)
+              : launch(k_tp_fwd<N, false>, done[0], smem, threads, tiles, s, m, m2, a);
 }
 
 template <int N>
@@ -80,14 +91,29 @@ TpArgs args(int n, const void *src, void *dst, int nvol, const float2 *tw512) {
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-float2 *g_scratch[2] = {nullptr, nullptr};  // N = 128, 256
+float2 *g_scratch[4] = {};  // N = 32, 64, 128, 256
+
+// Calls f with N as a compile-time constant.
+template <class F>
+cudaError_t with_size(int n, F &&f) {
+  switch (n) {
+    case 32: return f(std::integral_constant<int, 32>{});
+    case 64: return f(std::integral_constant<int, 64>{});
+    case 128: return f(std::integral_constant<int, 128>{});
+    case 256: return f(std::integral_constant<int, 256>{});
+    default: return cudaErrorNotSupported;
+  }
+}
 
 }  // namespace
 
-int tp_scratch_cubes(int n) { return n == 128 ? kTpScratchCubes128 : kTpScratchCubes256; }
+int tp_scratch_cubes(int n) {
+  return n == 32 ? kTpScratchCubes32
+                 : (n == 64 ? kTpScratchCubes64 : (n == 128 ? kTpScratchCubes128 : kTpScratchCubes256));
+}
 
 float2 *tp_scratch(int n, bool may_allocate) {
-  float2 *&p = g_scratch[n == 128 ? 0 : 1];
+  float2 *&p = g_scratch[n == 32 ? 0 : (n == 64 ? 1 : (n == 128 ? 2 : 3))];
   if (!p && may_allocate) {
     void *q = nullptr;
     if (cudaMalloc(&q, (size_t)tp_scratch_cubes(n) * n * n * n * sizeof(float2)) == cudaSuccess)
@@ -106,15 +132,21 @@ void release_tp() {
 }
 
 bool tp_encode_tiles(CUtensorMap *m, const void *cubes, int n, int nvol) {
-  return n == 128 ? encode_tiles<128>(m, cubes, nvol) : (n == 256 && encode_tiles<256>(m, cubes, nvol));
+  return with_size(n, [&](auto k) {
+           return encode_tiles<decltype(k)::value>(m, cubes, nvol) ? cudaSuccess : cudaErrorNotSupported;
+         }) == cudaSuccess;
 }
 
 cudaError_t launch_tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, const float2 *tw512,
-                          cudaStream_t s) {
-  const TpArgs a = args(n, src, dst, nvol, tw512);
-  CUtensorMap m;
-  if (!tp_size(n) || !aligned16(src) || !tp_encode_tiles(&m, dst, n, nvol)) return cudaErrorNotSupported;
-  return n == 128 ? fwd<128>(a, real, m, s) : fwd<256>(a, real, m, s);
+                          cudaStream_t s, const float2 *src2, float2 *dst2, int nvol2) {
+  TpArgs a = args(n, src, dst, nvol + nvol2, tw512);
+  a.first = nvol;
+  a.src2 = src2;
+  CUtensorMap m, m2;
+  if (!tp_size(n) || !aligned16(src) || !aligned16(src2) || (real && nvol2) || !tp_encode_tiles(&m, dst, n, nvol) ||
+      !tp_encode_tiles(&m2, nvol2 ? dst2 : dst, n, nvol2 ? nvol2 : nvol))
+    return cudaErrorNotSupported;
+  return with_size(n, [&](auto k) { return fwd<decltype(k)::value>(a, real, m, m2, s); });
 }
 
 cudaError_t launch_tp_inv(int n, const float2 *src, float2 *dst, int nvol, float scale, const float2 *tw512,
@@ -123,7 +155,7 @@ cudaError_t launch_tp_inv(int n, const float2 *src, float2 *dst, int nvol, float
   a.scale = scale;
   CUtensorMap m;
   if (!tp_size(n) || !tp_encode_tiles(&m, src, n, nvol)) return cudaErrorNotSupported;
-  return n == 128 ? inv<128>(a, m, s) : inv<256>(a, m, s);
+  return with_size(n, [&](auto k) { return inv<decltype(k)::value>(a, m, s); });
 }
 
 cudaError_t launch_tp_mid(int n, int mode, const float2 *src, float2 *dst, const float2 *filt, long long filt_vol,
@@ -133,7 +165,7 @@ cudaError_t launch_tp_mid(int n, int mode, const float2 *src, float2 *dst, const
   a.filt_vol = filt_vol;
   if (!tp_size(n) || !aligned16(src) || !aligned16(dst) || (mode != TP_FWD && !aligned16(filt)))
     return cudaErrorNotSupported;
-  return n == 128 ? mid<128>(a, mode, s) : mid<256>(a, mode, s);
+  return with_size(n, [&](auto k) { return mid<decltype(k)::value>(a, mode, s); });
 }
 
 cudaError_t launch_tp_fwd_table(int n, const float2 *const *srcs, const CUtensorMap *dst_maps, int nvol,
@@ -142,7 +174,7 @@ cudaError_t launch_tp_fwd_table(int n, const float2 *const *srcs, const CUtensor
   a.srcs = srcs;
   a.maps = dst_maps;
   CUtensorMap m{};
-  return n == 128 ? fwd<128>(a, false, m, s) : (n == 256 ? fwd<256>(a, false, m, s) : cudaErrorInvalidValue);
+  return with_size(n, [&](auto k) { return fwd<decltype(k)::value>(a, false, m, m, s); });
 }
 
 cudaError_t launch_tp_inv_table(int n, const CUtensorMap *src_maps, float2 *const *dsts, int nvol, float scale,
@@ -152,7 +184,7 @@ cudaError_t launch_tp_inv_table(int n, const CUtensorMap *src_maps, float2 *cons
   a.maps = src_maps;
   a.dsts = dsts;
   CUtensorMap m{};
-  return n == 128 ? inv<128>(a, m, s) : (n == 256 ? inv<256>(a, m, s) : cudaErrorInvalidValue);
+  return with_size(n, [&](auto k) { return inv<decltype(k)::value>(a, m, s); });
 }
 
 cudaError_t launch_tp_mid_table(int n, const float2 *const *srcs, float2 *const *dsts, const float2 *const *filts,
@@ -161,7 +193,7 @@ cudaError_t launch_tp_mid_table(int n, const float2 *const *srcs, float2 *const 
   a.srcs = srcs;
   a.dsts = dsts;
   a.filts = filts;
-  return n == 128 ? mid<128>(a, TP_PAIR, s) : (n == 256 ? mid<256>(a, TP_PAIR, s) : cudaErrorInvalidValue);
+  return with_size(n, [&](auto k) { return mid<decltype(k)::value>(a, TP_PAIR, s); });
 }
 
 template <int N>
@@ -177,6 +209,8 @@ static cudaError_t prepare() {
   return e;
 }
 
-cudaError_t prepare_tp(int n) { return n == 128 ? prepare<128>() : (n == 256 ? prepare<256>() : cudaErrorInvalidValue); }
+cudaError_t prepare_tp(int n) {
+  return with_size(n, [](auto k) { return prepare<decltype(k)::value>(); });
+}
 
 }  // namespace convgpu

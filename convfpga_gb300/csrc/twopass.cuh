@@ -38,7 +38,8 @@ namespace convgpu {
 // groups of threads per CTA (one CTA per SM), B tile buffers. A group transforms one tile at
 // a time; the other B - G buffers are in flight, so a group finds its next tile landed.
 //   256: 64 KB tiles, 2 groups of 256 threads x 128 registers, 3 buffers.
-//   128: 32 KB tiles, 4 groups of 128 threads, 6 buffers.
+//   128: 32 KB tiles, 4 groups of 128 threads, 6 buffers. 64: 16 KB, 8 groups of 64, 12
+//   buffers. 32: 8 KB, 16 groups of a warp, 24 buffers.
 // One CTA of 16 compute warps per SM, since a thread holds a tile's 16 pairs (64 registers).
 // Measured, us: 4 cubes of 256^3: k_tp_fwd 187 and k_tp_inv 191 (1.07 GB each: 5.7 TB/s; two
 // CTAs of one tile each, loaded and stored from registers, took 215 and 276), k_tp_mid with
@@ -54,6 +55,17 @@ template <>
 struct TpShape<128> {
   static constexpr int J = 16, C = 4, PAD = 4, G = 4, B = 6;
 };
+template <>
+struct TpShape<64> {
+  static constexpr int J = 16, C = 8, PAD = 4, G = 8, B = 12;
+};
+template <>
+struct TpShape<32> {
+  static constexpr int J = 16, C = 16, PAD = 2, G = 16, B = 24;
+};
+// Units of a run that one TMA box row holds (128 bytes at most, for the swizzle).
+template <int N>
+constexpr int kTpBox = TpShape<N>::C < 8 ? TpShape<N>::C : 8;
 
 // The filter operand of k_tp_mid.
 enum TpMode : int {
@@ -64,6 +76,8 @@ enum TpMode : int {
 
 struct TpArgs {
   const float2 *src;   // k_tp_fwd: cubes; k_tp_mid, k_tp_inv: cubes in tile order
+  const float2 *src2;  // k_tp_fwd: cubes `first`.. come from here (and go to the second map)
+  int first;
   float2 *dst;
   const float2 *filt;  // k_tp_mid
   long long src_vol, dst_vol, filt_vol;  // elements between cubes (0: one for all)
@@ -133,9 +147,20 @@ struct TpStream {
   uint32_t bar, tiles, pitch;
   __device__ __forceinline__ uint32_t full(int n) const { return bar + ((n % G) * 4 + (n / G) % 4) * 8; }
   __device__ __forceinline__ uint32_t buf(int n) const { return tiles + (n % B) * pitch; }
+  // The outer passes' tile of load n (below zero: none is left), written before its barrier is
+  // armed and read after the wait.
+  __device__ __forceinline__ uint32_t tile_slot(int n) const { return bar + 720 + ((n % G) * 4 + (n / G) % 4) * 4; }
+  __device__ __forceinline__ void set_tile(int n, int w) const {
+    asm volatile("st.shared.s32 [%0], %1;" ::"r"(tile_slot(n)), "r"(w) : "memory");
+  }
+  __device__ __forceinline__ int tile(int n) const {
+    int w;
+    asm volatile("ld.shared.s32 %0, [%1];" : "=r"(w) : "r"(tile_slot(n)) : "memory");
+    return w;
+  }
   // A bounded wait that gave up marks the CTA: it carries on with what its buffers hold
   // (wrong output, reported through the status word), waits no more and loads no more.
-  __device__ __forceinline__ uint32_t mark() const { return bar + 192; }
+  __device__ __forceinline__ uint32_t mark() const { return bar + 704; }
   __device__ __forceinline__ bool marked() const {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(mark()) : "memory");
@@ -160,11 +185,19 @@ struct TpStream {
   }
 };
 
-// TMEM of a CTA (warp 0 allocates and frees): 64 columns per warp that shares a lane group,
+// Programmatic dependent launch: a CTA may start once every CTA of the kernel before it in the
+// stream has started to end, fills its tables and sets up its barriers, and touches nothing
+// that another kernel writes before tp_grid_wait(). It hides the launch and the set-up of
+// every pass but the first: 17 cubes of 32^3 25 us instead of 35, one of 128^3 41 instead of
+// 49. (Letting the next kernel in from the start, launch_dependents, changed nothing there
+// and cost 4 cubes of 256^3 with their filters 909 us instead of 835.)
+__device__ __forceinline__ void tp_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// TMEM of a CTA (warp 1 allocates and frees): 64 columns per warp that shares a lane group,
 // for the row exchange, and in the middle pass as many again for the filter's values.
 template <int COLS>
 __device__ __forceinline__ uint32_t tp_tmem_alloc(uint32_t slot) {
-  if (threadIdx.x < 32) {
+  if (threadIdx.x / 32 == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "n"(COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
@@ -180,7 +213,8 @@ __device__ __forceinline__ void tp_tmem_free(uint32_t tmem) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(COLS));
+  if (threadIdx.x / 32 == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(COLS));
 }
 // This warp's 64 columns of block b.
 __device__ __forceinline__ uint32_t tp_tmem_warp(uint32_t tmem, int b) {
@@ -200,6 +234,36 @@ __device__ __forceinline__ void tp_gave_up(const TpStream<B, G> &st, unsigned *s
   }
 }
 
+// Tiles of the outer passes at N = 128 and 256 are claimed in order, after each CTA's first
+// ones, not dealt out: runs of 32 or 64 bytes of neighbouring tiles share cache lines, which
+// leave L2 half filled (about 20 us after the first write) if CTAs with a fixed share of the
+// tiles drift apart. A forward pass of 32 cubes of 256^3 then took 123 us a cube and filter
+// where one of 8 took 91, and the inverse 51 a cube; claimed 85 and 42. At N = 32 and 64 runs
+// are whole lines, and the claims of so many small tiles cost more than they give (17 cubes
+// of 32^3 64 us instead of 25). One counter per size and
+// pass (kernels of one size and pass never run side by side); every tile claims one successor,
+// so the claim that counts the last tile is the last there is and sets it back to zero. The
+// middle pass between them zeroes both as well, for after a pass that gave up.
+__device__ unsigned g_tp_claims[4];
+template <int N>
+constexpr bool kTpClaims = N >= 128;
+template <int N>
+constexpr bool kTpStager = N >= 64;  // k_tp_fwd: a warp of its own stores the tiles
+template <int N>
+__device__ __forceinline__ unsigned *tp_claims(int pass) {
+  return g_tp_claims + (N == 256 ? 2 : 0) + pass;
+}
+// Tile of a CTA's load n (ntiles or above: none is left), claimed by one thread when one of
+// the launch's tiles is begun; the first `dealt` tiles of the launch are the CTAs' own, tile
+// blockIdx + n gridDim, and so are all of a short launch, over before CTAs drift.
+template <int N>
+__device__ __forceinline__ int tp_claim(int pass, int n, int dealt, int ntiles) {
+  if (ntiles < 32 * (int)gridDim.x) return (int)(blockIdx.x + n * gridDim.x);
+  const unsigned k = atomicAdd(tp_claims<N>(pass), 1u);
+  if (k == (unsigned)ntiles - 1u) atomicExch(tp_claims<N>(pass), 0u);
+  return dealt + (int)k;
+}
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -211,28 +275,39 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *m, uint32_t src,
                : "memory");
 }
 
-// Byte offset of unit c of kx's run in the staged (or landed) box of a column group: boxes
-// of N runs of C units, 16-byte chunks swizzled as the tensor map says (32 or 64 bytes), so
-// that neighbouring kx cover all banks.
+// Byte offset of unit c of kx's run in a staged (or landed) box: boxes of N runs of C units,
+// 16-byte chunks swizzled as the tensor map says (32, 64 or 128 bytes), so that neighbouring
+// kx cover all banks.
 template <int C>
 __device__ __forceinline__ uint32_t tp_run_off(int kx, int c) {
   return (uint32_t)(kx * C + (c ^ ((kx * C / 8) & (C - 1)))) * 16;
 }
 
 // Forward outer pass. REAL: the source holds N^3 floats per cube. mdst: the destination in
-// tile order, dims (2 C values of a run, tiles, runs of a tile), box (2 C, N, 1). Every group
-// has a buffer of its own, where its loads land and its exchanges happen; the next load is
-// issued when the columns are in registers. Outputs are staged in the other S = B - G
-// buffers, which the groups take in turn, and a further warp stores them: 2,048 runs of 32
-// bytes keep the TMA unit for about 1.8 us, which the tile's own buffer does not wait for.
-// (Stores from registers, one run per thread, hold the LSU pipe for 1.4 cycles a run, 80% of
-// the pass: 215 us for 4 cubes of 256^3. Staged in the tile's own buffer 195, this 187.)
+// tile order, dims (2 C values of a run, tiles, runs of a tile), box (2 C, N, 1), for the
+// first a.first cubes, mdst2 for the others (a filter and its signals in one launch).
+//
+// N = 64 to 256: every group has a buffer of its own, where its loads land and its exchanges
+// happen; the next load is issued when the columns are in registers. Outputs are staged in
+// the other S = B - G buffers, which the groups take in turn, and a further warp stores them:
+// 2,048 runs of 32 bytes keep the TMA unit for about 1.8 us, which the tile's own buffer does
+// not wait for. (Stores from registers, one run per thread, hold the LSU pipe for 1.4 cycles
+// a run, 80% of the pass: 215 us for 4 cubes of 256^3. Staged in the tile's own buffer 195,
+// this 187, 177 with claimed tiles.)
+// N = 32: outputs are staged in the tile's own buffer and stored by the group; the buffer
+// takes its next load during the group's next tile. (One warp storing for 16 groups holds
+// them up: 17 cubes under one filter 24.6 us instead of 21.8. At N = 64 it does not: 100
+// cubes 239 us instead of 258.)
+template <int N>
+constexpr int kTpFwdThreads = kTpThreads<N> + (kTpStager<N> ? 32 : 0);
+
 template <int N, bool REAL>
-__global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
-    k_tp_fwd(const __grid_constant__ CUtensorMap mdst, TpArgs a) {
+__global__ void __launch_bounds__(kTpFwdThreads<N>, 1)
+    k_tp_fwd(const __grid_constant__ CUtensorMap mdst, const __grid_constant__ CUtensorMap mdst2, TpArgs a) {
   using TT = TpOuterTile<N>;
   using S = TpShape<N>;
-  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B, SB = B - G;
+  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B, SB = B - G,
+                BX = kTpBox<N>;
   static_assert(G % SB == 0, "the groups take the staging buffers in turn");
   extern __shared__ __align__(1024) unsigned char smraw[];
   const uint32_t sm = smem_u32(smraw);
@@ -240,34 +315,73 @@ __global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
   const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + TT::kTwBytes, lin = utw0 + G * 2 * J * 16;
   const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
   const int ntiles = a.nvol * R * H;
-  const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // tiles of this CTA
-  // staged[s]: the group whose turn it is has staged its tile in buffer G + s; grant[g]: the
-  // buffer of group g's next tile has been stored (a group's own, so its waits are in order).
-  const uint32_t staged = sm + 128, grant = sm + 144;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < SB; ++s) mbar_init(staged + s * 8, TT::NT);
-    for (int i = 0; i < G; ++i) mbar_init(grant + i * 8, 1);
-    st.init();
+  constexpr bool kClaims = kTpClaims<N>, kStager = kTpStager<N>;
+  const int mine = kClaims ? 0 : ((int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0);
+  // staged[s]: the group whose turn it is has staged its tile in buffer G + s;
+  // grant[g]: the buffer of group g's next turn has been stored (a group's own, so its waits
+  // are in order). Turn n is group n % G's and buffer G + n % SB's.
+  const uint32_t staged = sm + 512, grant = sm + 576;
+  static_assert(G <= 16 && SB <= 8, "barriers in the first KB");
+  constexpr uint32_t kRow = REAL ? N * 4 : N * 8;
+  auto load = [&](int n, int w) {  // by one warp: 2 J row copies, row (j, plane) at j ROWB + plane N 8
+    const int lane = threadIdx.x & 31;
+    if (w >= ntiles) {
+      if (lane == 0) {
+        st.set_tile(n, -1);
+        mbar_arrive(st.full(n));
+      }
+      return;
+    }
+    const int vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
+    // src_vol counts values, complex or (REAL) float
+    const char *src = a.srcs ? (const char *)a.srcs[vol]
+                             : (vol < a.first ? (const char *)a.src + vol * a.src_vol * (REAL ? 4 : 8)
+                                              : (const char *)a.src2 + (vol - a.first) * a.src_vol * (REAL ? 4 : 8));
+    if (lane == 0) {
+      st.set_tile(n, w);
+      mbar_arrive_expect_tx(st.full(n), 2 * J * kRow);
+    }
+    __syncwarp();
+    for (int i = lane; i < 2 * J; i += 32) {
+      const int j = i >> 1, z = zz + (i & 1) * H;
+      bulk_load(st.buf(kStager ? n % G : n) + j * TT::ROWB + (i & 1) * (N * 8), src + ((long long)z * N + y0 + R * j) * kRow, kRow,
+                st.full(n));
+    }
+  };
+  auto store = [&](uint32_t buf, int w) {  // by one thread: the staged tile's runs
+    const int vol = w / (R * H), r = w % (R * H);
+    const CUtensorMap *m = a.maps ? a.maps + vol : (vol < a.first ? &mdst : &mdst2);
+    const int mvol = a.maps ? 0 : (vol < a.first ? vol : vol - a.first);
+    if (a.maps) tensormap_acquire(m);
+#pragma unroll
+    for (int k = 0; k < J / BX; ++k)  // box k: units k BX .. of the runs of column group k BX / C
+      tma_store_3d(m, buf + k * (N * BX * 16), 0, (mvol * (J / C) + k * BX / C) * N, r * (C / BX) + k % (C / BX));
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  };
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) {
+      for (int s = 0; s < SB; ++s) mbar_init(staged + s * 8, TT::NT);
+      for (int i = 0; i < G; ++i) mbar_init(grant + i * 8, 1);
+      st.init();
+    }
+    __syncwarp();
+    tp_grid_wait();
+    for (int n = 0; n < (kClaims ? G : min(kStager ? G : B, mine)); ++n) load(n, blockIdx.x + n * gridDim.x);
   }
   TT::fill_tw(tw, a.tw512);
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const float2 w = __ldg(a.tw512 + i * (512 / N));
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(lin + i * 8), "f"(w.x), "f"(w.y) : "memory");
   }
+  tp_grid_wait();
   __syncthreads();
   bool ok = true;
-  if (g == G) {  // the storing warp
+  if (kStager && !kClaims && g == G) {  // the storing warp, turns known
     for (int n = 0; n < mine; ++n) {
       const int s = n % SB;
       ok &= st.wait_on(staged + s * 8, (uint32_t)(n / SB) & 1u);
       if (tid == 0) {
-        const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H);
-        const CUtensorMap *m = a.maps ? a.maps + vol : &mdst;
-        if (a.maps) tensormap_acquire(m);
-#pragma unroll
-        for (int k = 0; k < J / C; ++k)
-          tma_store_3d(m, st.buf(G + s) + k * (N * C * 16), 0, ((a.maps ? 0 : vol) * (J / C) + k) * N, r);
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        store(st.buf(G + s), blockIdx.x + n * gridDim.x);
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         if (n + SB < mine) mbar_arrive(grant + (n + SB) % G * 8);
       }
@@ -277,28 +391,67 @@ __global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
     if (!ok) tp_gave_up(st, a.status);
     return;
   }
-  constexpr uint32_t kRow = REAL ? N * 4 : N * 8;
-  auto load = [&](int n) {  // by the group's first warp: 2 J row copies, row (j, plane) at j ROWB + plane N 8
-    const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
-    // src_vol counts values, complex or (REAL) float
-    const char *src = a.srcs ? (const char *)a.srcs[vol] : (const char *)a.src + vol * a.src_vol * (REAL ? 4 : 8);
-    if (tid == 0) mbar_arrive_expect_tx(st.full(n), 2 * J * kRow);
-    __syncwarp();
-    for (int i = tid; i < 2 * J; i += 32) {
-      const int j = i >> 1, z = zz + (i & 1) * H;
-      bulk_load(st.buf(g) + j * TT::ROWB + (i & 1) * (N * 8), src + ((long long)z * N + y0 + R * j) * kRow, kRow,
-                st.full(n));
+  if (kClaims && g == G) {  // the storing warp
+    unsigned alive = (1u << G) - 1u;
+    int done[SB] = {};  // phases of each staging buffer
+    for (int n0 = 0; alive; n0 += SB) {
+#pragma unroll
+      for (int s = 0; s < SB; ++s) {
+        const int n = n0 + s, turn = n % G;
+        if (!(alive >> turn & 1u)) continue;
+        ok &= st.wait(n);  // the turn's tile is known
+        const bool none = ok && st.tile(n) < 0;
+        if (!__any_sync(~0u, none)) ok &= st.wait_on(staged + s * 8, (uint32_t)(done[s]++) & 1u);
+        if (__any_sync(~0u, !ok || st.marked())) {  // a wait gave up: no more stores
+          ok = false;
+          alive = 0;
+          break;
+        }
+        const int w = st.tile(n);
+        if (w < 0) {
+          alive &= ~(1u << turn);
+        } else if (tid == 0) {
+          store(st.buf(G + s), w);
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
+        if (tid == 0) {  // the buffer's next turn that is still taken
+          for (int m = n + SB; m < n + SB + G; m += SB)
+            if (alive >> (m % G) & 1u) {
+              mbar_arrive(grant + m % G * 8);
+              break;
+            }
+        }
+        __syncwarp();
+      }
     }
-  };
-  if (tid < 32 && g < mine) load(g);
+    if (tid == 0) {
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    if (!ok) tp_gave_up(st, a.status);
+    return;
+  }
   TT tt(tid, 1 + g, tw);
-  tt.at(st.buf(g));
-  int set = 0;
-  for (int n = g; n < mine; n += G) {
-    const int r = (blockIdx.x + n * gridDim.x) % (R * H), y0 = r / H, zz = r % H;
+  int set = 0, drain = -1;  // drain: the load whose buffer the group's last store reads (N = 32)
+  for (int n = g; kClaims || n < mine; n += G) {
+    int w = blockIdx.x + n * gridDim.x;
+    if constexpr (kClaims) {
+      // the whole group carries on or stops
+      if (group_any<TT::NT>(1 + g, !st.wait(n) || !ok)) {
+        ok = false;
+        break;
+      }
+      w = st.tile(n);
+      if (w < 0) break;  // nothing left; the storing warp sees it too and passes the turn on
+      tt.at(st.buf(g));
+    } else {
+      ok &= st.wait(n);
+      tt.at(st.buf(kStager ? g : n));
+    }
+    const int r = w % (R * H), y0 = r / H, zz = r % H;
     const uint32_t utw = utw0 + (g * 2 + set) * (J * 16);
     tp_step_tw<N>(utw, lin, tid, y0, zz);
-    ok &= st.wait(n);
+    int next = 0;  // the group's next tile, claimed ahead of its use below
+    if (kClaims && tid == 0) next = tp_claim<N>(0, n + G, gridDim.x * G, ntiles);
     Pair v[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
@@ -315,23 +468,41 @@ __global__ void __launch_bounds__(kTpThreads<N> + 32, 1)
     tt.forward(v, [&] {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tt.sync();
-      if (tid < 32 && n + G < mine && !__any_sync(~0u, st.marked())) load(n + G);
+      if (tid >= 32) return;
+      const bool dead = __any_sync(~0u, st.marked());
+      if constexpr (kClaims) {
+        load(n + G, dead ? ntiles : __shfl_sync(~0u, next, 0));
+      } else if (kStager) {
+        if (n + G < mine && !dead) load(n + G, blockIdx.x + (n + G) * gridDim.x);
+      } else if (drain >= 0 && drain + B < mine && !dead) {
+        if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        __syncwarp();
+        load(drain + B, blockIdx.x + (drain + B) * gridDim.x);
+      }
     });
-    if (n >= SB) ok &= st.wait_on(grant + g * 8, (uint32_t)(n / G - (g < SB ? 1 : 0)) & 1u);
-    const uint32_t out = st.buf(G + n % SB);
+    if (kStager && n >= SB) ok &= st.wait_on(grant + g * 8, (uint32_t)(n / G - (g < SB ? 1 : 0)) & 1u);
+    const uint32_t out = kStager ? st.buf(G + n % SB) : tt.base;
 #pragma unroll
     for (int i = 0; i < TT::B3; ++i) {
       const int kx = tt.q + i * TT::NT;
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const Pair s = lds_pair(utw + j * 16);
-        sts_pair(out + (j / C) * (N * C * 16) + tp_run_off<C>(kx, j % C), pmul_tw(v[i * J + j], s.re, s.im));
+        sts_pair(out + (j / BX) * (N * BX * 16) + tp_run_off<BX>(kx, j % BX), pmul_tw(v[i * J + j], s.re, s.im));
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_arrive(staged + n % SB * 8);
+    if constexpr (kStager) {
+      mbar_arrive(staged + n % SB * 8);
+    } else {
+      tt.sync();
+      if (tid == 0) store(out, w);
+      __syncwarp();
+      drain = n;
+    }
     set ^= 1;
   }
+  if (!kStager && tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   if (!ok) tp_gave_up(st, a.status);
 }
 
@@ -341,47 +512,74 @@ template <int N>
 __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_inv(const __grid_constant__ CUtensorMap msrc, TpArgs a) {
   using TT = TpOuterTile<N>;
   using S = TpShape<N>;
-  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B;
+  constexpr int J = TT::J, R = N / J, C = S::C, H = N / 2, G = S::G, B = S::B, BX = kTpBox<N>;
   extern __shared__ __align__(1024) unsigned char smraw[];
   const uint32_t sm = smem_u32(smraw);
   const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
   const uint32_t tw = sm + 1024 + B * kTpBuf<N>, utw0 = tw + TT::kTwBytes, lin = utw0 + G * 2 * J * 16;
   const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
   const int ntiles = a.nvol * R * H;
-  const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  if (threadIdx.x == 0) st.init();
+  constexpr bool kClaims = kTpClaims<N>;
+  const int mine = kClaims ? 0 : ((int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0);
+  auto load = [&](int n, int w) {  // by one thread
+    if (w >= ntiles) {
+      st.set_tile(n, -1);
+      mbar_arrive(st.full(n));
+      return;
+    }
+    const int vol = w / (R * H), r = w % (R * H);
+    st.set_tile(n, w);
+    const CUtensorMap *m = a.maps ? a.maps + vol : &msrc;
+    if (a.maps) tensormap_acquire(m);
+    mbar_arrive_expect_tx(st.full(n), J * N * 16);
+#pragma unroll
+    for (int k = 0; k < J / BX; ++k)
+      tma_load_3d(st.buf(n) + k * (N * BX * 16), m, 0, ((a.maps ? 0 : vol) * (J / C) + k * BX / C) * N,
+                  r * (C / BX) + k % (C / BX), st.full(n));
+  };
+  if (threadIdx.x == 0) {
+    st.init();
+    tp_grid_wait();
+    for (int n = 0; n < (kClaims ? B : min(B, mine)); ++n) load(n, blockIdx.x + n * gridDim.x);
+  }
   TT::fill_tw(tw, a.tw512);
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const float2 w = __ldg(a.tw512 + i * (512 / N));
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(lin + i * 8), "f"(w.x), "f"(w.y) : "memory");
   }
+  tp_grid_wait();
   __syncthreads();
   TT tt(tid, 1 + g, tw);
-  auto load = [&](int n) {  // by one thread
-    const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H);
-    const CUtensorMap *m = a.maps ? a.maps + vol : &msrc;
-    if (a.maps) tensormap_acquire(m);
-    mbar_arrive_expect_tx(st.full(n), J * N * 16);
-#pragma unroll
-    for (int k = 0; k < J / C; ++k)
-      tma_load_3d(st.buf(n) + k * (N * C * 16), m, 0, ((a.maps ? 0 : vol) * (J / C) + k) * N, r, st.full(n));
-  };
-  if (threadIdx.x == 0)
-    for (int n = 0; n < B && n < mine; ++n) load(n);
   bool ok = true;
   int set = 0;
-  for (int n = g; n < mine; n += G) {
-    const int w = blockIdx.x + n * gridDim.x, vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
+  for (int n = g; kClaims || n < mine; n += G) {
+    int w = blockIdx.x + n * gridDim.x;
+    if constexpr (kClaims) {
+      // the whole group carries on or stops
+      if (group_any<TT::NT>(1 + g, !st.wait(n))) {
+        ok = false;
+        break;
+      }
+      w = st.tile(n);
+      if (w < 0) {  // nothing left, for the load that would follow in this buffer either
+        if (tid == 0) load(n + B, ntiles);
+        break;
+      }
+    } else {
+      ok &= st.wait(n);
+    }
+    const int vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
     const uint32_t utw = utw0 + (g * 2 + set) * (J * 16);
     tp_step_tw<N>(utw, lin, tid, y0, zz);
     tt.at(st.buf(n));
-    ok &= st.wait(n);
+    int next = 0;  // the tile that takes this buffer, claimed ahead of its use below
+    if (kClaims && tid == 0) next = tp_claim<N>(1, n + B, gridDim.x * B, ntiles);
     Pair v[16];
 #pragma unroll
     for (int i = 0; i < TT::B3; ++i)
 #pragma unroll
       for (int j = 0; j < J; ++j)
-        v[i * J + j] = lds_pair(tt.base + (j / C) * (N * C * 16) + tp_run_off<C>(tt.q + i * TT::NT, j % C));
+        v[i * J + j] = lds_pair(tt.base + (j / BX) * (N * BX * 16) + tp_run_off<BX>(tt.q + i * TT::NT, j % BX));
     tt.sync();  // every thread has its units; the step twiddles are written
 #pragma unroll
     for (int i = 0; i < TT::B3; ++i)
@@ -393,7 +591,12 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_inv(const __grid_consta
     tt.inverse(v, [&] {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tt.sync();
-      if (tid == 0 && n + B < mine && !st.marked()) load(n + B);
+      if (tid == 0) {
+        if constexpr (kClaims)
+          load(n + B, st.marked() ? ntiles : next);
+        else if (n + B < mine && !st.marked())
+          load(n + B, blockIdx.x + (n + B) * gridDim.x);
+      }
       __syncwarp();
     });
     float2 *o0 = a.dst_of(vol) + ((long long)zz * N + y0 + R * tt.row) * N, *o1 = o0 + (long long)H * N * N;
@@ -469,7 +672,7 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
   static_assert(TT::NT * G == kTpThreads<N> && TT::BYTES <= kTpBuf<N>, "one CTA shape for all passes");
   constexpr int kCols = MODE == TP_FWD ? 256 : 512;  // TMEM columns
   extern __shared__ __align__(1024) unsigned char smraw[];
-  const uint32_t sm = smem_u32(smraw), tslot = sm + 200;
+  const uint32_t sm = smem_u32(smraw), tslot = sm + 712;
   const TpStream<B, G> st{sm, sm + 1024, (uint32_t)kTpBuf<N>};
   const uint32_t tw = sm + 1024 + B * kTpBuf<N>;
   const int g = threadIdx.x / TT::NT, tid = threadIdx.x % TT::NT;
@@ -478,10 +681,6 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
   // Loads come in rounds of G (one per group, missing ones included so that n % G is the
   // group); tile of load n: its round's number / LPT.
   const int loads = (mine + G - 1) / G * G * LPT;
-  if (threadIdx.x == 0) st.init();
-  TT::fill_tw(tw, a.tw512);
-  const uint32_t tmem = tp_tmem_alloc<kCols>(tslot), park = tp_tmem_warp(tmem, 1);
-  TT tt(tid, 1 + g, tp_tmem_warp(tmem, 0), tw);
   // Tile w: cube w % nvol, tile w / nvol: the cubes' tiles against one filter run together.
   auto load = [&](int n) {  // by one thread; a missing tile's load completes at once
     const int k = (n / G / LPT) * G + n % G;  // this CTA's tile number
@@ -494,8 +693,16 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
     mbar_arrive_expect_tx(st.full(n), (uint32_t)(ELEMS * 8));
     bulk_load(st.buf(n), cube + (long long)(w / a.nvol) * ELEMS, (uint32_t)(ELEMS * 8), st.full(n));
   };
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0) {
+    st.init();
+    tp_grid_wait();
     for (int n = 0; n < B && n < loads; ++n) load(n);
+  }
+  TT::fill_tw(tw, a.tw512);
+  const uint32_t tmem = tp_tmem_alloc<kCols>(tslot), park = tp_tmem_warp(tmem, 1);
+  tp_grid_wait();
+  if (kTpClaims<N> && blockIdx.x == 0 && threadIdx.x < 2) *tp_claims<N>(threadIdx.x) = 0u;
+  TT tt(tid, 1 + g, tp_tmem_warp(tmem, 0), tw);
   bool ok = true;
   int n = g;  // this group's next load
   Pair v[16];

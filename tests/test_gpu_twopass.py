@@ -1,4 +1,4 @@
-"""The two-pass 3D transform (twopass.cuh; plan kind 4, variant 3, N = 128 and 256).
+"""The two-pass 3D transform (twopass.cuh; plan kind 4, variant 3, N = 32 to 256).
 
 Every route of it against the oracle: one filter per signal and shared, complex and real,
 batches below, at and above the scratch cubes and the shared-filter threshold, in place,
@@ -24,8 +24,8 @@ def _c64(rng, shape):
 
 @pytest.fixture
 def tp(gpu):
-    keep = {(n, k): gpu.plan_variant(n, k) for n in (128, 256) for k in (4, 7)}
-    for n in (128, 256):
+    keep = {(n, k): gpu.plan_variant(n, k) for n in (32, 64, 128, 256) for k in (4, 7)}
+    for n in (32, 64, 128, 256):
         assert gpu.plan_variant(n, 4, 3) == 3
         gpu.plan_variant(n, 7, 0)
     gpu.device_status()
@@ -41,6 +41,8 @@ def _check(ref32, ref64, out):
 
 
 @pytest.mark.parametrize("n,b,filt", [(128, b, f) for b in (1, 2, 3, 4, 7) for f in ("shared", "pairs", "real", "real_pairs")]
+                         + [(n, b, f) for n in (32, 64) for b in (2, 5) for f in ("shared", "pairs", "real", "real_pairs")]
+                         + [(32, 1100, "shared"), (32, 515, "pairs"), (64, 131, "shared")]
                          + [(256, 1, "real"), (256, 3, "shared"), (256, 5, "shared"), (256, 5, "pairs")])
 def test_routes(tp, n, b, filt):
     rng = np.random.default_rng(n + b)
@@ -101,7 +103,7 @@ def test_operands_it_does_not_take(tp):
 def test_uneven_graph(tp, in_place):
     """The graph's classes run it in table mode unless a job of the class is in place; the
     cached plan follows the buffers either way."""
-    sizes = [256, 128, 32, 128, 256, 128]
+    sizes = [256, 128, 32, 64, 128, 64, 256, 32, 128]
     offs = np.cumsum([0] + [n ** 3 for n in sizes])
     jobs = [(n, int(o), int(o), int(o)) for n, o in zip(sizes, offs)]
     for rep in range(2):

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 # N: (J rows of the outer tile, C interleaved columns of the middle tile)
-SHAPES = {32: (8, 2), 64: (8, 4), 128: (16, 4), 256: (16, 2)}
+SHAPES = {32: (16, 16), 64: (16, 8), 128: (16, 4), 256: (16, 2)}
 
 
 def _fwd(cube, j_rows, c_cols):
@@ -82,8 +82,8 @@ def _banks(units):
         assert len(set(units[at:at + 8] % 8)) == 8
 
 
-@pytest.mark.parametrize("n", [128, 256])
-def test_outer_tile_slots(n):
+@pytest.mark.parametrize("n,pad", [(32, 2), (64, 4), (128, 4), (256, 0)])
+def test_outer_tile_slots(n, pad):
     """The outer tile's row exchange (written by ex_w, read by ex_r) and its column slots are
     permutations of the tile, both sides agree, and 8 consecutive lanes of each access hit 8
     different 16-byte bank groups."""
@@ -93,22 +93,23 @@ def test_outer_tile_slots(n):
     t, row = tid % r2, tid // r2
     written, read, cols = {}, {}, set()
     for k1 in range(16):
-        u = row * n + k1 * r2 + (t ^ (k1 & sw))
+        u = row * (n + pad) + k1 * r2 + (t ^ (k1 & sw))
         _banks(u)
         written.update({int(a): (int(b), k1, int(c)) for a, b, c in zip(u, row, t)})
     for i in range(16 // r2):
         for tt in range(r2):
             k1 = t + i * r2
-            u = row * n + k1 * r2 + (tt ^ (k1 & sw))
+            u = row * (n + pad) + k1 * r2 + (tt ^ (k1 & sw))
             _banks(u)
             read.update({int(a): (int(b), int(c), tt) for a, b, c in zip(u, row, k1)})
-    assert written == read and sorted(written) == list(range(n * j_rows))
+    rows = {j * (n + pad) + x for j in range(j_rows) for x in range(n)}
+    assert written == read and set(written) == rows
     for i in range(16 // j_rows):
         for j in range(j_rows):
-            u = j * n + tid + i * nt
+            u = j * (n + pad) + tid + i * nt
             _banks(u)
             cols.update(u.tolist())
-    assert cols == set(range(n * j_rows))
+    assert cols == rows
 
 
 def _trip(regs, col_of, reg_of):
@@ -125,7 +126,7 @@ def _trip(regs, col_of, reg_of):
     return out
 
 
-@pytest.mark.parametrize("n", [128, 256])
+@pytest.mark.parametrize("n", [64, 128, 256])
 def test_middle_tile_exchange(n):
     """Two trips through TMEM take unit (k1) of lane (l4..l0) to lane (l0, k1), register
     s = (l4 l3 l2 l1); the twiddles between them are those of (t, k1); the shared-memory slots
@@ -154,14 +155,15 @@ def test_middle_tile_exchange(n):
                 for h in range(2):
                     assert b[(lane, frag2(s, w) + h)] == (s << 1 | lane >> 4, lane & 15, w, h)
     # lane before = (row, t, c) = 16 row + C t + c; butterfly i's input t is unit_of(i, t)
-    unit_of = lambda i, t: i * 8 + t if c_cols == 2 else (i >> 1) * 8 + t * 2 + (i & 1)
+    hc = c_cols // 2
+    unit_of = lambda i, t: (i // hc) * 8 + t * hc + i % hc
     slots = set()
     for i in range(16 // r2):
         for k2 in range(r2):
             u = []
             for lane in range(32):
                 l0 = lane >> 4
-                row, c = (i, l0) if c_cols == 2 else (i >> 1, (i & 1) * 2 + l0)
+                row, c = i // hc, (i % hc) * 2 + l0
                 for t in range(r2):
                     assert unit_of(i, t) << 1 | l0 == 16 * row + c_cols * t + c
                 kx = (lane & 15) + 16 * k2
