@@ -58,6 +58,7 @@ struct GPlan {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaEvent_t done = nullptr;
+  unsigned long long kernels = 0;  // the graph's
   bool launched = false;
   ~GPlan() {
     if (done) cudaEventDestroy(done);
@@ -71,6 +72,18 @@ struct GPlan {
     if (d_spec) cudaFree(d_spec);
   }
 };
+
+cudaError_t count_kernels(cudaGraph_t graph, unsigned long long &kernels) {
+  size_t n = 0;
+  cudaError_t e = cudaGraphGetNodes(graph, nullptr, &n);
+  std::vector<cudaGraphNode_t> nodes(n);
+  if (e == cudaSuccess) e = cudaGraphGetNodes(graph, nodes.data(), &n);
+  for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+    cudaGraphNodeType t;
+    if ((e = cudaGraphNodeGetType(nodes[i], &t)) == cudaSuccess) kernels += t == cudaGraphNodeTypeKernel;
+  }
+  return e;
+}
 
 std::mutex g_mu;
 // key: job sizes, normalize + 2 * (form of each size, base 5)
@@ -185,6 +198,7 @@ cudaError_t build(GPlan &p, bool normalize, const Forms &forms, const float2 *tw
     if (e == cudaSuccess) e = e2;
   }
   if (e == cudaSuccess) e = cudaGraphInstantiate(&p.exec, p.graph, 0);
+  if (e == cudaSuccess) e = count_kernels(p.graph, p.kernels);
   for (auto b : br)
     if (b) cudaStreamDestroy(b);
   for (auto v : ev)
@@ -305,7 +319,7 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
     return -3;
   }
   p.launched = true;
-  count_launches(7 * p.groups.size());
+  count_launches(p.kernels);
   return 0;
 }
 
