@@ -522,6 +522,10 @@ static cudaError_t tp_inv(int n, const float2 *src, float2 *dst, int nvol, float
   return pass_tp(13, 32.0 * n * n * n * nvol, s, [&] { return launch_tp_inv(n, src, dst, nvol, scale, g.tw512, s); });
 }
 
+static cudaError_t tp_order(int n, const float2 *src, float2 *dst, cudaStream_t s) {
+  return pass_tp(8 + OP_FWD, 16.0 * n * n * n, s, [&] { return launch_tp_order(n, src, dst, s); });
+}
+
 // A shared filter's second pass runs inside every signal's middle pass (TP_PAIR) for small
 // batches, and otherwise once before them (TP_FWD, then TP_SPECTRUM): a quarter of the middle
 // pass's work for every cube against one more launch and the filter's own tiles. Measured, us,
@@ -582,6 +586,42 @@ static cudaError_t enqueue_tp(int n, const float2 *sig, const float2 *filt, floa
   return cudaSuccess;
 }
 
+static bool apart(const void *a, size_t an, const void *b, size_t bn) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x + an <= y || y + bn <= x;
+}
+
+// Signals against one spectrum in natural order: it is put into tile order first, in the last
+// scratch cube, and read once for all signals.
+// cudaErrorNotSupported, with nothing enqueued, as enqueue_tp, and for batches that the
+// three-axis passes (five launches, no reordering) take faster: between 2^21 and 2^23 points
+// those run out of L2 and the tiles make less than two rounds of the SMs, and one large cube
+// does not make up for the reordering. us, tiles / three axes: 32^3 x1 16.0 / 20.7, x17 23.0 /
+// 26.8, x100 67.4 / 61.3, x300 132 / 137; 64^3 x1 18.1 / 22.7, x8 37.5 / 42.8, x17 63.2 / 60.5,
+// x33 98 / 110; 128^3 x1 42.5 / 43.1, x2 63.3 / 60.8, x4 100 / 108, x8 166 / 200; 256^3 x1
+// 227 / 219, x2 365 / 404, x4 683 / 769.
+constexpr long long kTpSpectrumSmall = 1ll << 21, kTpSpectrumLarge = 1ll << 23;
+static cudaError_t enqueue_tp_spectrum(int n, const float2 *sig, const float2 *spec, float2 *out, unsigned how_many,
+                                       float scale, cudaStream_t s) {
+  const long long V = (long long)n * n * n;
+  const size_t bytes = (size_t)V * how_many * sizeof(float2);
+  if (V * how_many > kTpSpectrumSmall && (how_many < 2 || V * how_many < kTpSpectrumLarge)) return cudaErrorNotSupported;
+  if ((reinterpret_cast<uintptr_t>(sig) | reinterpret_cast<uintptr_t>(out)) & 15u) return cudaErrorNotSupported;
+  if (sig != out && !apart(sig, bytes, out, bytes)) return cudaErrorNotSupported;
+  float2 *scratch = tp_scratch(n, !capturing(s));
+  if (!scratch) return cudaErrorNotSupported;
+  const unsigned cubes = tp_scratch_cubes(n) - 1u;
+  float2 *tiles = scratch + cubes * V;
+  CG_TRY(tp_order(n, spec, tiles, s));
+  for (unsigned i = 0; i < how_many; i += cubes) {
+    const int k = (int)std::min(cubes, how_many - i);
+    CG_TRY(tp_fwd(n, sig + i * V, scratch, k, false, s));
+    CG_TRY(tp_mid(n, kTpSpectrum, scratch, scratch, tiles, 0, k, s));
+    CG_TRY(tp_inv(n, scratch, out + i * V, k, scale, s));
+  }
+  return cudaSuccess;
+}
+
 static int tc_of(unsigned flags) {
   // 0: FP32 kernels; 1 + split precision for the tensor-core path.
   return (flags & (kFlagTensorSplit | kFlagTensorBf16x3)) ? 1 + ((flags & kFlagTensorBf16x3) ? kTcBf16x3 : kTcTf32x3)
@@ -600,11 +640,6 @@ static size_t workspace_bytes_for(unsigned n, unsigned how_many, unsigned flags)
 // Largest batch for which a shared filter's z transform runs inside the signals' fused z
 // pass instead of as a pass of its own.
 constexpr unsigned kSharedFilterFusedMax = 2;
-
-static bool apart(const void *a, size_t an, const void *b, size_t bn) {
-  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-  return x + an <= y || y + bn <= x;
-}
 
 // The one-launch path of 16^3 cubes reads a cube's operands before it writes its output, but
 // the cubes in any order: outputs must be the signals or apart from them, and apart from
@@ -631,7 +666,12 @@ static cudaError_t enqueue_conv_device(unsigned n, const float2 *sig, const floa
     return e;
   }
   if (flags & kFlagFilterIsSpectrum) {
-    const long long sv = (flags & kFlagPerSignalFilter) ? V : 0;
+    const bool per = (flags & kFlagPerSignalFilter) != 0 && how_many > 1;
+    if (!per && use_tp((int)n, tc)) {
+      const cudaError_t e = enqueue_tp_spectrum((int)n, sig, filt, out, how_many, scale, s);
+      if (e != cudaErrorNotSupported) return e;
+    }
+    const long long sv = per ? V : 0;
     return enqueue_signals(n, sig, out, filt, sv, OP_CONV, how_many, scale, s, nullptr, tc);
   }
   const bool real = (flags & kFlagFilterReal) != 0;

@@ -88,6 +88,8 @@ cudaError_t launch_tp_mid(int n, int mode, const float2 *src, float2 *dst, const
                           int nvol, const float2 *tw512, cudaStream_t s);
 cudaError_t launch_tp_inv(int n, const float2 *src, float2 *dst, int nvol, float scale, const float2 *tw512,
                           cudaStream_t s);
+// A spectrum from natural to tile order (any 8-byte aligned source).
+cudaError_t launch_tp_order(int n, const float2 *src, float2 *dst, cudaStream_t s);
 // The same over cubes at unrelated addresses: device arrays of pointers and of tensor maps
 // (tp_encode_tiles of each cube in tile order). prepare_tp sets the kernels' attributes (call
 // it before a capture).

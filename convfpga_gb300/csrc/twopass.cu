@@ -24,12 +24,9 @@ int sm_count() {
 }
 
 template <class K, class... M>
-cudaError_t launch(K kern, int &done, int smem, int threads, long long tiles, cudaStream_t s, const M &...args) {
-  if (tiles <= 0 || tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const cudaError_t e = set_smem_once(kern, smem, done);
-  if (e != cudaSuccess) return e;
+cudaError_t launch_blocks(K kern, int smem, int threads, long long blocks, cudaStream_t s, const M &...args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)std::min<long long>(tiles, sm_count()));
+  cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = s;
@@ -39,6 +36,15 @@ cudaError_t launch(K kern, int &done, int smem, int threads, long long tiles, cu
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// Persistent: one CTA per SM at most.
+template <class K, class... M>
+cudaError_t launch(K kern, int &done, int smem, int threads, long long tiles, cudaStream_t s, const M &...args) {
+  if (tiles <= 0 || tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  const cudaError_t e = set_smem_once(kern, smem, done);
+  if (e != cudaSuccess) return e;
+  return launch_blocks(kern, smem, threads, std::min<long long>(tiles, sm_count()), s, args...);
 }
 
 template <int N>
@@ -75,6 +81,11 @@ cudaError_t mid(const TpArgs &a, int mode, cudaStream_t s) {
     case TP_FWD: return launch(k_tp_mid<N, TP_FWD>, done[2], smem, threads, tiles, s, a);
     default: return cudaErrorInvalidValue;
   }
+}
+
+template <int N>
+cudaError_t order(const float2 *src, float2 *dst, cudaStream_t s) {
+  return launch_blocks(k_tp_order<N>, 0, 256, (long long)N * N * N / 1024, s, src, dst);
 }
 
 TpArgs args(int n, const void *src, void *dst, int nvol, const float2 *tw512) {
@@ -166,6 +177,10 @@ cudaError_t launch_tp_mid(int n, int mode, const float2 *src, float2 *dst, const
   if (!tp_size(n) || !aligned16(src) || !aligned16(dst) || (mode != TP_FWD && !aligned16(filt)))
     return cudaErrorNotSupported;
   return with_size(n, [&](auto k) { return mid<decltype(k)::value>(a, mode, s); });
+}
+
+cudaError_t launch_tp_order(int n, const float2 *src, float2 *dst, cudaStream_t s) {
+  return with_size(n, [&](auto k) { return order<decltype(k)::value>(src, dst, s); });
 }
 
 cudaError_t launch_tp_fwd_table(int n, const float2 *const *srcs, const CUtensorMap *dst_maps, int nvol,

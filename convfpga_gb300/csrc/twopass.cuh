@@ -774,4 +774,33 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
   tp_tmem_free<kCols>(tmem);
 }
 
+// A spectrum in natural order -> tile order, for calls that bring their filter's spectrum.
+// Bound by the copy (16 N^3 bytes, or L2 for the small sizes; 4.7 us at N = 64, launch
+// included): a block turns 32 rows (pairs of kz, C of ky) of 32 kx into 32 runs of 16 units,
+// 256 bytes a run on either side.
+template <int N>
+__global__ void __launch_bounds__(256) k_tp_order(const float2 *src, float2 *dst) {
+  constexpr int J = TpShape<N>::J, C = TpShape<N>::C, R = N / J, H = N / 2, KZ = 16 / C;
+  __shared__ float2 rows[32][33];
+  int b = blockIdx.x;
+  const int x0 = b % (N / 32) * 32;
+  b /= N / 32;
+  const int kz0 = b % (H / KZ) * KZ;
+  b /= H / KZ;
+  const int k2 = b % R, g = b / R;
+  const int lane = threadIdx.x & 31;
+  tp_grid_wait();
+  for (int i = threadIdx.x >> 5; i < 32; i += 8) {
+    const int u = i >> 1, kz = 2 * (kz0 + u / C) + (i & 1), ky = g * C + u % C + J * k2;
+    rows[i][lane] = __ldg(src + ((long long)kz * N + ky) * N + x0 + lane);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 512; i += 256) {
+    const int x = i >> 4, u = i & 15;
+    const float2 p = rows[2 * u][x], q = rows[2 * u + 1][x];
+    stg_unit(dst + (((long long)g * N + x0 + x) * (R * H * C) + (k2 * H + kz0) * C + u) * 2,
+             Pair{pk(p.x, q.x), pk(p.y, q.y)});
+  }
+}
+
 }  // namespace convgpu

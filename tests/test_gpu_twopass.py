@@ -67,6 +67,26 @@ def test_routes(tp, n, b, filt):
         _check(ref, ref64, inplace[i])
 
 
+@pytest.mark.parametrize("n,b,off", [(32, 2, 0), (32, 515, 1), (64, 1, 0), (64, 5, 1), (64, 9, 0), (128, 1, 1),
+                                     (128, 33, 0), (256, 1, 0), (256, 4, 1)])
+def test_given_spectrum(tp, n, b, off):
+    """Signals against a spectrum in natural order, at 16- and 8-byte alignment, apart and in place."""
+    rng = np.random.default_rng(n + b)
+    sig, f = _c64(rng, (b, n, n, n)), _c64(rng, (n, n, n))
+    spec = torch.empty(n ** 3 + off, dtype=torch.complex64, device="cuda")[off:]
+    spec.copy_(torch.from_numpy(np.fft.fftn(f.astype(np.complex128)).astype(np.complex64)).flatten())
+    s = torch.from_numpy(sig).cuda()
+    o = torch.empty_like(s)
+    flags = tp.FILTER_IS_SPECTRUM | tp.NORMALIZE
+    tp.conv3d_device(n, s, spec, o, b, flags)
+    tp.conv3d_device(n, s, spec, s, b, flags)
+    torch.cuda.synchronize()
+    assert torch.equal(o, s)
+    for i in {0, b // 2, b - 1}:
+        _check(conv3d(sig[i:i + 1], f, "fp32", normalize=True, engine="pocketfft")[0],
+               conv3d(sig[i:i + 1], f, "fp64", normalize=True, engine="pocketfft")[0], o[i].cpu().numpy())
+
+
 def test_filters_in_the_outputs(tp):
     """The filters are read before any output is written, chunk by chunk or not."""
     n, b = 128, 5
