@@ -404,13 +404,13 @@ static bool use_half(unsigned n, bool real, int tc) {
 // (C+2)/(2C) share of a full spectrum's bytes (C = 16 columns per tile below N = 256, 8 above).
 static cudaError_t pass_half(int n, int axis, int op, const void *src, float2 *dst, const float2 *filt,
                              long long filt_vol, int nvol, float scale, cudaStream_t s) {
-  NvtxRange nv(axis == 0 ? "x-fwd half" : (axis == 1 ? "y-fwd half" : (op == OP_CONV ? "z-conv half" : "z-fwd half")));
+  NvtxRange nv(axis == 0 ? "x-fwd half" : (axis == 1 ? "y-fwd half" : (op == OP_FWD ? "z-fwd half" : "z-conv half")));
   PassRec r{axis * 4 + op, 0.0, nullptr, nullptr};
   if (g_prof) {
     const double v = (double)n * n * n, h = (double)n * n * half_spectrum_pitch(n);
     const double cols = n >= 256 ? 8.0 : 16.0;
     r.bytes = nvol * (axis == 0 ? 4.0 * v + 8.0 * h
-                                : (op == OP_CONV ? 16.0 * v + 8.0 * v * (cols + 2.0) / (2.0 * cols) : 16.0 * h));
+                                : (op != OP_FWD ? 16.0 * v + 8.0 * v * (cols + 2.0) / (2.0 * cols) : 16.0 * h));
     cudaEventCreate(&r.a);
     cudaEventCreate(&r.b);
     cudaEventRecord(r.a, s);
@@ -423,12 +423,16 @@ static cudaError_t pass_half(int n, int axis, int op, const void *src, float2 *d
   return e;
 }
 
+// The fused z pass against half spectra: at N = 512 it transforms them along z itself
+// (pairs512.cuh), elsewhere a pass of the filter's own does before (herm.cuh).
+static int half_op(int n) { return n == 512 ? OP_CONV_FZ : OP_CONV; }
+
 // Half spectra of `count` real filters (N^3 floats each) into spec (N^2 W values each):
-// x pass of the real rows, then y and z passes over the half width.
+// x pass of the real rows, then y and (unless it is fused) z passes over the half width.
 static cudaError_t enqueue_filter_half(int n, const float *filt, float2 *spec, int count, cudaStream_t s) {
   CG_TRY(pass_half(n, 0, OP_FWD, filt, spec, nullptr, 0, count, 1.f, s));
   CG_TRY(pass_half(n, 1, OP_FWD, spec, spec, nullptr, 0, count, 1.f, s));
-  CG_TRY(pass_half(n, 2, OP_FWD, spec, spec, nullptr, 0, count, 1.f, s));
+  if (half_op(n) == OP_CONV) CG_TRY(pass_half(n, 2, OP_FWD, spec, spec, nullptr, 0, count, 1.f, s));
   return cudaSuccess;
 }
 
@@ -463,7 +467,7 @@ static cudaError_t enqueue_signals(int n, const float2 *sig, float2 *out, const 
     CG_TRY(pass(n, 1, OP_FWD, out, out, nullptr, 0, nsig, 1.f, s, tc));
   }
   if (half)
-    CG_TRY(pass_half(n, 2, OP_CONV, out, out, spec, spec_vol, nsig, 1.f, s));
+    CG_TRY(pass_half(n, 2, half_op(n), out, out, spec, spec_vol, nsig, 1.f, s));
   else
     CG_TRY(pass(n, 2, fop, out, out, spec, spec_vol, nsig, 1.f, s, tc));
   if (mid) cudaEventRecord(mid, s);
@@ -1487,7 +1491,7 @@ int bridge_autotune(const unsigned *sizes, unsigned count, int write_cache) {
         if (half_spectrum_pitch(n) > 0) {
           for (int v = 0; v < 2 && err == cudaSuccess; ++v) {
             auto run = [&]() {
-              return v ? launch_axis_pass_half(n, 2, OP_CONV, data, data, spec, 0, nvol, 1.f, g.tw512, s)
+              return v ? launch_axis_pass_half(n, 2, half_op(n), data, data, spec, 0, nvol, 1.f, g.tw512, s)
                        : launch_axis_pass(n, 2, OP_CONV, data, data, spec, 0, nvol, 1.f, g.tw512, s);
             };
             for (int w = 0; w < 2 && err == cudaSuccess; ++w) err = run();

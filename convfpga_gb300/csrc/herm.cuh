@@ -18,7 +18,8 @@
 // an even width so the box's inner bytes are a multiple of 16), so the half spectrum is
 // read once for two signal tiles: a signal convolution reads (C+2)/(2C) of a full
 // spectrum's bytes. Threads 0 .. C*T-1 transform tile A, the rest tile B, each tile being
-// its own exchange buffer as in k_strided_tma.
+// its own exchange buffer as in k_strided_tma. (N = 512 has a kernel of its own, which also
+// transforms the filter along z: k_zpair, pairs512.cuh.)
 #pragma once
 
 #include "passes.cuh"
@@ -34,11 +35,11 @@ constexpr int zconv_half_smem_bytes() {
   return 128 + (2 * N * COLS + N * (COLS + 2)) * 8 + N * 8;
 }
 
-// CTAs per SM that shared memory allows (26 KB at N = 64, about 52 KB at 128 and 256,
-// 111 KB at 512): registers are held to that occupancy too.
+// CTAs per SM that shared memory allows (26 KB at N = 64, about 52 KB at 128 and 256):
+// registers are held to that occupancy too.
 template <int N>
 constexpr int zconv_half_min_blocks() {
-  return N <= 64 ? 8 : (N <= 256 ? 4 : 2);
+  return N <= 64 ? 8 : 4;
 }
 
 template <int N, int E, int COLS, class Plan>

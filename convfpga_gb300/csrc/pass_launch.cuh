@@ -10,11 +10,13 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 
 #include "herm.cuh"
 #include "passes.cuh"
+#include "pairs512.cuh"
 
 namespace convgpu {
 
@@ -61,6 +63,9 @@ bool encode_runs_map(CUtensorMap *m, const void *base, int vals, long long tiles
 // As encode_cube_map over planes of N rows of `width` complex values (row pitch = width).
 bool encode_pitched_map(CUtensorMap *m, const void *base, int width, int n, long long nplanes, int axis, int cols);
 
+// The device's tile counter of pairs512.cuh's kernels (calls on one device are in stream order).
+unsigned *zpair_claims();
+
 template <int N>
 cudaError_t launch_size(const PassReq &r);
 template <int N>
@@ -78,6 +83,14 @@ static cudaError_t set_smem_once(K kern, int smem, int &done) {
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e == cudaSuccess) done = dev + 1;
   return e;
+}
+
+static inline int sm_count() {
+  static int of[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  if (of[dev] == 0 && cudaDeviceGetAttribute(&of[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+  return of[dev];
 }
 
 // Register-gather kernels (shape variant 0): any 8-byte aligned operands.
@@ -125,12 +138,43 @@ static cudaError_t launch_rows(const PassReq &r) {
   return cudaGetLastError();
 }
 
+// Fused z pass of N = 512 (pairs512.cuh): against half spectra of pitch half_pitch(512) with
+// their z transform (HALF, FZ), or full filters with (FZ) or without it.
+template <bool HALF, bool FZ>
+static cudaError_t launch_zpair(const PassReq &r) {
+  using S = ZPairShape<HALF>;
+  constexpr int N = S::N;
+  auto kern = k_zpair<HALF, FZ>;
+  static int done = 0;
+  cudaError_t e = set_smem_once(kern, S::kSmem, done);
+  if (e != cudaSuccess) return e;
+  CUtensorMap ms, mf;
+  const long long fplanes = r.a.filt_vol_elems ? (long long)r.nvol * N : (long long)N;
+  if (!encode_cube_map(&ms, r.a.src, N, (long long)r.nvol * N, 2, S::C) ||
+      !encode_pitched_map(&mf, r.a.filt, HALF ? half_pitch(N) : N, N, fplanes, 2, S::FC))
+    return cudaErrorNotSupported;
+  const long long tiles = (long long)r.nvol * N * S::GROUPS;
+  if (tiles <= 0 || tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  const unsigned blocks = (unsigned)std::min<long long>((tiles + S::G - 1) / S::G, sm_count());
+  unsigned *claims = zpair_claims();
+  if (!claims) return cudaErrorNotSupported;
+  e = cudaMemsetAsync(claims, 0, sizeof(unsigned), r.s);
+  if (e != cudaSuccess) return e;
+  kern<<<blocks, S::NT * S::G, S::kSmem, r.s>>>(ms, mf, r.a, r.nvol, claims);
+  return cudaGetLastError();
+}
+
 // TMA y / z pass. Returns cudaErrorNotSupported when a tensor map cannot be built.
 template <int N, int V, int OP>
 static cudaError_t launch_strided(const PassReq &r) {
   using S = Shape<N, V>;
   constexpr int E = S::E, COLS = S::SC;
   constexpr bool HAS_F = (OP == OP_CONV || OP == OP_CONV_FZ);
+  if constexpr (N == 512 && HAS_F)
+    if (r.mode != kModeTable && r.axis == 2) {
+      if ((reinterpret_cast<uintptr_t>(r.a.dst) & 15u) != 0) return cudaErrorNotSupported;
+      return launch_zpair<false, OP == OP_CONV_FZ>(r);
+    }
   constexpr int smem = tma_pass_smem_bytes<N, COLS, OP>();
   auto kern = k_strided_tma<N, E, COLS, OP, typename S::Plan>;
   static int done = 0;
@@ -228,6 +272,18 @@ static cudaError_t launch_half(const PassReq &r) {
     if ((reinterpret_cast<uintptr_t>(a.dst) & 15u) != 0) return cudaErrorNotSupported;
     if (r.axis == 0) {
       if (!r.real_src || r.op != OP_FWD) return cudaErrorInvalidValue;
+      if constexpr (N == 512) {
+        // two rows as one complex row, where the copies' alignment allows it
+        if ((reinterpret_cast<uintptr_t>(a.src) & 15u) == 0) {
+          static int done = 0;
+          const cudaError_t e = set_smem_once(k_rows_real_pair, RowsRealPair::kSmem, done);
+          if (e != cudaSuccess) return e;
+          const long long blocks = (long long)r.nplanes * N / RowsRealPair::kRows;
+          if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+          k_rows_real_pair<<<(unsigned)blocks, RowsRealPair::WARPS * 32, RowsRealPair::kSmem, r.s>>>(a);
+          return cudaGetLastError();
+        }
+      }
       PassReq q = r;
       q.a.out_cols = W;
       return r.variant ? launch_rows_real<N, 1>(q) : launch_rows_real<N, 0>(q);
@@ -250,7 +306,9 @@ static cudaError_t launch_half(const PassReq &r) {
       kern<<<(unsigned)blocks, COLS * (N / E), smem, r.s>>>(m, m, a, r.axis);
       return cudaGetLastError();
     }
-    if (r.op == OP_CONV && r.axis == 2) {
+    if constexpr (N == 512) {
+      return r.op == OP_CONV_FZ && r.axis == 2 ? launch_zpair<true, true>(r) : cudaErrorInvalidValue;
+    } else if (r.op == OP_CONV && r.axis == 2) {
       auto kern = k_zconv_half<N, E, COLS, typename S::Plan>;
       constexpr int smem = zconv_half_smem_bytes<N, COLS>();
       static int done = 0;

@@ -23,6 +23,7 @@ namespace convgpu {
 // gave up). Word 1: the dependency-wait limit that tests may lower (tma.cuh:
 // dep_wait_limit; 0 = every wait's own limit). Kernels get the address of word 0.
 __device__ unsigned int g_device_words[2] = {0u, 0u};
+__device__ unsigned int g_zpair_claims[1];
 
 extern template cudaError_t launch_size<16>(const PassReq &);
 extern template cudaError_t launch_size<32>(const PassReq &);
@@ -154,19 +155,29 @@ bool encode_table_map(CUtensorMap *m, const void *cube, int n, int kind) {
 }
 
 // ------------------------------------------------------------------ status word
-unsigned int *device_status_address() {
-  constexpr int kMaxDev = 64;
-  static std::atomic<unsigned int *> cache[kMaxDev];
+// Address of one of this file's device arrays on the current device, kept per device.
+template <class Symbol>
+static unsigned int *address_of(const Symbol &symbol, std::atomic<unsigned int *> (&cache)[64]) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   unsigned int *p = cache[dev].load();
   if (!p) {
     void *q = nullptr;
-    if (cudaGetSymbolAddress(&q, g_device_words) != cudaSuccess) return nullptr;
+    if (cudaGetSymbolAddress(&q, symbol) != cudaSuccess) return nullptr;
     p = static_cast<unsigned int *>(q);
     cache[dev].store(p);
   }
   return p;
+}
+
+unsigned int *device_status_address() {
+  static std::atomic<unsigned int *> cache[64];
+  return address_of(g_device_words, cache);
+}
+
+unsigned int *zpair_claims() {
+  static std::atomic<unsigned int *> cache[64];
+  return address_of(g_zpair_claims, cache);
 }
 
 unsigned int read_and_clear_device_status() {

@@ -15,14 +15,6 @@ bool tp_size(int n) { return n == 32 || n == 64 || n == 128 || n == 256; }
 
 namespace {
 
-int sm_count() {
-  static int of[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
-  if (of[dev] == 0 && cudaDeviceGetAttribute(&of[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
-  return of[dev];
-}
-
 template <class K, class... M>
 cudaError_t launch_blocks(K kern, int smem, int threads, long long blocks, cudaStream_t s, const M &...args) {
   cudaLaunchConfig_t cfg{};
