@@ -50,7 +50,7 @@ struct ZPairShape {
 // The 16 x 16 transform of a column of units by 16 threads, thread t of them; ROWB: bytes
 // between units. Slot of (k1, t) between the stages is 16 k1 + t.
 template <int ROWB>
-struct ZColumn {
+struct UnitColumn {
   uint32_t base, tw, tw2;  // the column's unit 0; W_256^(t k1) at k1 16 + t; radix-2 twiddles, by n
   int t;
   __device__ __forceinline__ uint32_t at(int n) const { return base + n * ROWB; }
@@ -96,6 +96,9 @@ struct ZColumn {
     for (int k = 0; k < 16; ++k) v[k] = lds_pair(at(16 * t + k));
   }
 };
+
+// A kernel, not a memset: a memset may be queued on a copy engine behind large transfers.
+static __global__ void k_zpair_clear(unsigned *claims) { *claims = 0u; }
 
 // msig: the signals, box {C, 1, 256}; mfilt: the filter's columns, box {FC, 1, 256}.
 template <bool HALF, bool FZ>
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(ZPairShape<HALF>::NT *ZPairShape<HALF>::G, 1)
     if (tid == 0) next = (int)(gridDim.x * G + atomicAdd(claims, 1u));
     if constexpr (FZ) {
       const bool mine = tid < FC * 16;  // whole warps
-      const ZColumn<FC * 16> f{fbuf + (uint32_t)(tid % FC) * 16, tw, tw2, tid / FC};
+      const UnitColumn<FC * 16> f{fbuf + (uint32_t)(tid % FC) * 16, tw, tw2, tid / FC};
       if (mine) {
         f.load(v, fbuf + (uint32_t)(tid % FC) * 8, FC * 8, 1.f);
         f.stage1(v);
@@ -183,7 +186,7 @@ __global__ void __launch_bounds__(ZPairShape<HALF>::NT *ZPairShape<HALF>::G, 1)
       group_barrier();
       if (mine) f.write1(v);  // output k = t + 16 k2 to slot k
     }
-    const ZColumn<C * 16> s{sbuf + (uint32_t)c * 16, tw, tw2, t};
+    const UnitColumn<C * 16> s{sbuf + (uint32_t)c * 16, tw, tw2, t};
     ok &= ss.wait(n);
     s.load(v, sbuf + (uint32_t)c * 8, C * 8, sgn);
     s.stage1(v);

@@ -158,8 +158,7 @@ static cudaError_t launch_zpair(const PassReq &r) {
   const unsigned blocks = (unsigned)std::min<long long>((tiles + S::G - 1) / S::G, sm_count());
   unsigned *claims = zpair_claims();
   if (!claims) return cudaErrorNotSupported;
-  e = cudaMemsetAsync(claims, 0, sizeof(unsigned), r.s);
-  if (e != cudaSuccess) return e;
+  k_zpair_clear<<<1, 1, 0, r.s>>>(claims);
   kern<<<blocks, S::NT * S::G, S::kSmem, r.s>>>(ms, mf, r.a, r.nvol, claims);
   return cudaGetLastError();
 }

@@ -195,6 +195,10 @@ __device__ __forceinline__ float lds_f(uint32_t a) {
   return v;
 }
 
+__device__ __forceinline__ void stg_unit(float2 *p, Pair a) {
+  asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a.re), "l"(a.im) : "memory");
+}
+
 // Barrier of a group of NT threads: named, or its warp's.
 template <int NT>
 __device__ __forceinline__ void group_sync(int id) {

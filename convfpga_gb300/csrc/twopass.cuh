@@ -120,10 +120,6 @@ template <int N>
 constexpr int tp_mid_smem() {
   return 1024 + TpShape<N>::B * kTpBuf<N> + TpMidTile<N>::kTwBytes;
 }
-__device__ __forceinline__ void stg_unit(float2 *p, Pair a) {
-  asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a.re), "l"(a.im) : "memory");
-}
-
 // Step twiddles of outer tile (y0, zz): entry j' = {W_N^(y0 j'), W_N^(y0 j' + zz)} as
 // {c0, c1, s0, s1}; written by the group's first J threads into one of its two sets, since
 // slow threads may still read the previous tile's.

@@ -1,9 +1,10 @@
-// Launchers of the L2-staged fused x + y pass for N = 128, 256 and 512 (xyl2.cuh) and of its
+// Launchers of the L2-staged fused x + y pass for N = 128, 256 (xyl2.cuh) and 512 (xy512.cuh) and of its
 // tensor-core form for N = 256 (xyl2_tc.cuh): scratch ring per size and dependency counters
 // (grow-only, per process), counters cleared on the stream before every launch, one
 // persistent grid of as many CTAs as fit.
 #define CONVGPU_PASS_LAUNCH_IMPL
 #include "pass_launch.cuh"
+#include "xy512.cuh"
 #include "xyl2.cuh"
 #include "xyl2_tc.cuh"
 
@@ -87,18 +88,15 @@ cudaError_t prepare_xy_l2(int n) {
   Scratch *ring;
   if (n == 256) return xy_l2_setup<256>(0, ps, sms, ring);
   if (n == 128) return xy_l2_setup<128>(0, ps, sms, ring);
-  if (n == 512) return xy_l2_setup<512>(0, ps, sms, ring);
   return cudaErrorInvalidValue;
 }
 
 size_t xy_l2_counter_bytes(int n, int ncubes) { return (2ull * n * ncubes + 2) * sizeof(unsigned); }
 
-// The source rows map of the pass: 2D rows (box {N, C}) for N <= 256; for N = 512 rows
-// viewed as (256, 2, rows) with box {256, 2, C}, since a box is at most 256 long.
+// The source rows map of the pass (box {N, C}).
 static bool encode_xy_rows(CUtensorMap *m, const void *src, int n, long long rows) {
   if (n == 256) return encode_rows_map(m, src, 256, rows, XyL2Cfg<256>::C);
   if (n == 128) return encode_rows_map(m, src, 128, rows, XyL2Cfg<128>::C);
-  if (n == 512) return encode_rows512_map(m, src, rows, XyL2Cfg<512>::C);
   return false;
 }
 
@@ -116,17 +114,41 @@ static cudaError_t launch_common(const CUtensorMap *msrc_or_null, const CUtensor
   cudaError_t e = xy_l2_setup<N>(ctr ? 0 : nplanes, ps, sms, ring);
   if (e != cudaSuccess) return e;
   if (!ctr) ctr = reinterpret_cast<unsigned *>(g_ctr.p);
-  CUtensorMap mscr;
-  if (!encode_cube_map(&mscr, ring->p, N, Cfg::RING, 1, Cfg::C)) return cudaErrorNotSupported;
-  const CUtensorMap &msrc = msrc_or_null ? *msrc_or_null : mscr;  // unused in table mode
+  const CUtensorMap unused{};
+  const CUtensorMap &msrc = msrc_or_null ? *msrc_or_null : unused;  // table mode has its own
   auto kern = rmaps ? (inverse ? k_xy_l2<N, true, true> : k_xy_l2<N, false, true>)
                     : (inverse ? k_xy_l2<N, true, false> : k_xy_l2<N, false, false>);
   const long long ncount = 2LL * nplanes + 2;
   k_xyl2_clear<<<(unsigned)std::min<long long>((ncount + 255) / 256, 64), 256, 0, s>>>(ctr, ncount);
   const long long items = 2LL * nplanes * (N / Cfg::C);
   const unsigned grid = (unsigned)std::min<long long>(items, (long long)ps * sms);
-  kern<<<grid, kXyL2Threads, xyl2_smem<N>(), s>>>(msrc, mscr, reinterpret_cast<float2 *>(ring->p), dst, nplanes,
-                                                   scale, tw512, ctr, status, Cfg::LAG, rmaps, dsts);
+  kern<<<grid, kXyL2Threads, xyl2_smem<N>(), s>>>(msrc, reinterpret_cast<float2 *>(ring->p), dst, nplanes, scale, tw512,
+                                                   ctr, status, Cfg::LAG, rmaps, dsts);
+  return cudaGetLastError();
+}
+
+// The N = 512 form (xy512.cuh).
+static cudaError_t launch_xy512(const float2 *src, float2 *dst, int nplanes, bool inverse, float scale,
+                                const float2 *tw512, unsigned *status, cudaStream_t s) {
+  using S = Xy512;
+  using Cfg = XyL2Cfg<512>;
+  if (nplanes > 1 << 23) return cudaErrorInvalidConfiguration;  // 2^31 items
+  Scratch &ring = g_ring[2];
+  cudaError_t e = ring.ensure((size_t)S::N * S::N * sizeof(float2) * Cfg::RING);
+  if (e != cudaSuccess) return e;
+  const long long ncount = 2LL * nplanes + 2;
+  if ((e = g_ctr.ensure(std::max<size_t>(ncount * sizeof(unsigned), 64 << 10))) != cudaSuccess) return e;
+  static int done[2] = {0, 0};
+  auto kern = inverse ? k_xy512<true> : k_xy512<false>;
+  if ((e = set_smem_once(kern, S::kSmem, done[inverse])) != cudaSuccess) return e;
+  CUtensorMap msrc, mscr;
+  if (!encode_rows512_map(&msrc, src, (long long)nplanes * S::N, S::C) ||
+      !encode_cube_map(&mscr, ring.p, S::N, Cfg::RING, 1, S::C))
+    return cudaErrorNotSupported;
+  unsigned *ctr = reinterpret_cast<unsigned *>(g_ctr.p);
+  k_xyl2_clear<<<(unsigned)std::min<long long>((ncount + 255) / 256, 64), 256, 0, s>>>(ctr, ncount);
+  kern<<<S::CTAS * sm_count(), S::NT, S::kSmem, s>>>(msrc, mscr, reinterpret_cast<float2 *>(ring.p), dst, nplanes, scale,
+                                                      tw512, ctr, status);
   return cudaGetLastError();
 }
 
@@ -139,12 +161,12 @@ cudaError_t launch_xy_l2(int n, const float2 *src, float2 *dst, int nplanes, boo
                          const float2 *tw512, unsigned *status, cudaStream_t s) {
   if (nplanes <= 0) return cudaSuccess;
   if ((reinterpret_cast<uintptr_t>(dst) & 15u) != 0) return cudaErrorNotSupported;
+  if (n == 512) return launch_xy512(src, dst, nplanes, inverse, scale, tw512, status, s);
   CUtensorMap msrc;
   if (!encode_xy_rows(&msrc, src, n, (long long)nplanes * n)) return cudaErrorNotSupported;
   switch (n) {
     case 256: return launch_common<256>(&msrc, nullptr, nullptr, dst, nplanes, inverse, scale, tw512, status, nullptr, s);
     case 128: return launch_common<128>(&msrc, nullptr, nullptr, dst, nplanes, inverse, scale, tw512, status, nullptr, s);
-    case 512: return launch_common<512>(&msrc, nullptr, nullptr, dst, nplanes, inverse, scale, tw512, status, nullptr, s);
     default: return cudaErrorNotSupported;
   }
 }
@@ -207,7 +229,6 @@ cudaError_t launch_xy_l2_table(int n, const CUtensorMap *rmaps, float2 *const *d
   switch (n) {
     case 256: return launch_common<256>(nullptr, rmaps, dsts, nullptr, 256 * ncubes, inverse, scale, tw512, status, ctr, s);
     case 128: return launch_common<128>(nullptr, rmaps, dsts, nullptr, 128 * ncubes, inverse, scale, tw512, status, ctr, s);
-    case 512: return launch_common<512>(nullptr, rmaps, dsts, nullptr, 512 * ncubes, inverse, scale, tw512, status, ctr, s);
     default: return cudaErrorInvalidValue;
   }
 }

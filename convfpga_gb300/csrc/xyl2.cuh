@@ -1,7 +1,7 @@
-// Fused x + y pass for N = 128, 256 and 512 staged through L2: the x-transformed plane
+// Fused x + y pass for N = 128 and 256 staged through L2: the x-transformed plane
 // goes to a small ring of scratch planes instead of back to HBM, and the y transform reads
-// it from there. (Written for N = 256 below; N = 128 uses 16-row / 16-column items and
-// N = 512 4-row / 4-column items, see XyL2Cfg.)
+// it from there. (Written for N = 256 below; N = 128 uses 16-row / 16-column items, see
+// XyL2Cfg; N = 512 has a kernel of its own on the same schedule, xy512.cuh.)
 // A plane then crosses HBM once (read + write) instead of twice, as in the reference's
 // on-chip plane transpose (kernels/conv3D.cl:118-232, transpose + fft3db).
 //
@@ -11,8 +11,7 @@
 //            slot p % R;
 //   Y(p, c): y transform of columns 8c..8c+7 of plane p (one contiguous bulk copy from the
 //            scratch slot, which holds a plane as N / 8 column tiles of 8 columns x N rows;
-//            the tile is its own exchange buffer), written to the destination plane. (At
-//            N = 512 the slot is row-major and the columns come as a TMA box.)
+//            the tile is its own exchange buffer), written to the destination plane.
 // Order: X items of plane b and Y items of plane b - L, for b = 0, 1, ... (lag L planes).
 // Dependencies:
 //   Y(p, *) loads slot p % R only after all 32 X(p, *) items have stored (per-plane
@@ -127,31 +126,6 @@ __device__ __forceinline__ float2 stage_tw(const TwRT128 &tw, int r, int k) {
   return tw.t[r * 16 + k];
 }
 
-// Y items' exchange slot for N = 512 (4 columns per item): ColSlot<4> with the position's
-// low 2 bits XOR bits 4..5. A warp holds 8 consecutive pencil threads t x 4 columns; the
-// first stage's stores (positions 16t + j), the later stages' loads (t + 32e) and the
-// second stage's stores ((t/16)*256 + t%16 + 16j) then spread over all 32 banks (two
-// wavefronts) instead of 8 lanes per bank pair.
-struct ColSwz4 {
-  int c;
-  __device__ __forceinline__ int operator()(int n) const { return (n ^ ((n >> 4) & 3)) * 4 + c; }
-};
-
-// Twiddles of a 16 x 16 x 2 plan (N = 512): entries 0..255 hold W_512^(2*r*k) at r*16 + k
-// (second stage, NS = 16, R = 16: a warp reads consecutive entries), entries 256..767 hold
-// W_512^j (third stage, NS = 256, R = 2).
-struct TwRT512 {
-  const float2 *t;
-};
-template <int N, int NS, int R>
-__device__ __forceinline__ float2 stage_tw(const TwRT512 &tw, int r, int k) {
-  static_assert(N == 512 && ((NS == 16 && R == 16) || (NS == 256 && R == 2)), "TwRT512 serves a 16 x 16 x 2 plan");
-  if constexpr (NS == 16)
-    return tw.t[r * 16 + k];
-  else
-    return tw.t[256 + r * k];
-}
-
 // Per-size shape of the L2-staged pass. C: rows per X item = columns per Y item (each
 // item is C*N = 2048 points for 128 threads of 16 points); LAG / RING: planes between a
 // plane's X and Y items, and scratch planes (R > L; both chosen by timing: a shorter lag
@@ -194,33 +168,11 @@ struct XyL2Cfg<128> {
     tma_load_2d(d, m, 0, row0, bar);
   }
 };
+// N = 512: xy512.cuh.
 template <>
 struct XyL2Cfg<512> {
-  // 256 items per plane: the ~2,400 items the CTAs hold span ~10 planes. The ring is 18
-  // planes of 2 MiB (36 MiB, as for the other sizes); lag / ring 8 / 16 and 14 / 24 time
-  // no better.
-  static constexpr int C = 4, LAG = 10, RING = 18, TWN = 768;
-  // Row-major ring planes: with 4-column tiles a warp's stores of one row would touch 8
-  // lines instead of 2 (measured 2% slower at 512^3).
-  static constexpr bool TILED = false;
-  using Plan = Radices<16, 16, 2>;
-  using Tw = TwRT512;
-  static __device__ __forceinline__ float2 tw_entry(const float2 *tw512, int i) {
-    return i < 256 ? tw512[2 * ((i >> 4) * (i & 15))] : tw512[i - 256];
-  }
-  // a row's 512 slots: the low 4 bits XOR bits 4..7 (one row per warp, 32 threads)
-  static __device__ __forceinline__ SwzRow xslot(int c) { return SwzRow{c * 512}; }
-  static __device__ __forceinline__ ColSwz4 yslot(int c) { return ColSwz4{c}; }
-  // rows map viewed as (256, 2, rows): one box lands C whole rows
-  static __device__ __forceinline__ void load_x(uint32_t d, const CUtensorMap *m, int row0, uint32_t bar) {
-    tma_load_3d(d, m, 0, 0, row0, bar);
-  }
-  // C columns of a row-major ring plane; a box is at most 256 long: rows 0..255 and
-  // 256..511
-  static __device__ __forceinline__ void load_y(uint32_t d, const CUtensorMap *m, int x0, int slot, uint32_t bar) {
-    tma_load_3d(d, m, x0, 0, slot, bar);
-    tma_load_3d(d + 256 * C * 8, m, x0, 256, slot, bar);
-  }
+  static constexpr int C = 8, LAG = 10, RING = 16;
+  static constexpr bool TILED = false;  // row-major ring planes
 };
 // Dynamic shared memory: barrier (128 B), tile (TMA target and exchange buffer), the
 // twiddle table, the next item index: 18-23 KB, so registers (64 per thread) bound the
@@ -230,20 +182,17 @@ constexpr int xyl2_smem() {
   return 128 + XyL2Cfg<N>::C * N * 8 + XyL2Cfg<N>::TWN * 8 + 16;
 }
 
-// msrc: 2D map over the source rows (box {N, C}); scratch: Cfg::RING planes of N x N;
-// mscr: 3D map over them (box {C, N, 1}), used where the ring planes are row-major.
+// msrc: 2D map over the source rows (box {N, C}); scratch: Cfg::RING planes of N x N.
 // ctr: 2 * np counters (X stores done, Y reads done) and the work counter at ctr[2 * np],
 // all zero at launch.
 // TABLE: the planes belong to np / N cubes at unrelated addresses; plane p is plane p % N
 // of cube p / N, whose rows map is rmaps[p / N] (in device memory) and whose output base
 // is dsts[p / N]; msrc and dst are unused (and rmaps, dsts otherwise).
 template <int N, bool INV, bool TABLE>
-__global__ void __launch_bounds__(kXyL2Threads, 8) k_xy_l2(const __grid_constant__ CUtensorMap msrc,
-                                                           const __grid_constant__ CUtensorMap mscr, float2 *scratch,
-                                                           float2 *dst, long long np, float scale,
-                                                           const float2 *tw512, unsigned *ctr, unsigned *status,
-                                                           int lag_planes, const CUtensorMap *rmaps,
-                                                           float2 *const *dsts) {
+__global__ void __launch_bounds__(kXyL2Threads, 8)
+    k_xy_l2(const __grid_constant__ CUtensorMap msrc, float2 *scratch, float2 *dst, long long np, float scale,
+            const float2 *tw512, unsigned *ctr, unsigned *status, int lag_planes, const CUtensorMap *rmaps,
+            float2 *const *dsts) {
   using Cfg = XyL2Cfg<N>;
   constexpr int E = 16, T = N / E, C = Cfg::C, ITEMS = N / C, RING = Cfg::RING;
   static_assert(C * T == kXyL2Threads, "an item is one pencil tile per thread group");
@@ -282,11 +231,8 @@ __global__ void __launch_bounds__(kXyL2Threads, 8) k_xy_l2(const __grid_constant
         if (!wait_count(xdone + p, ITEMS, spin)) ok = false;
         asm volatile("fence.proxy.async.global;" ::: "memory");  // generic stores -> TMA reads
         mbar_arrive_expect_tx(bar, (uint32_t)(C * N * 8));
-        if constexpr (Cfg::TILED)  // the column tile is one contiguous block
-          bulk_load(smem_u32(tile), scratch + (long long)slot * N * N + (long long)tl * N * C, (uint32_t)(C * N * 8),
-                    bar);
-        else
-          Cfg::load_y(smem_u32(tile), &mscr, tl * C, slot, bar);
+        // the column tile is one contiguous block
+        bulk_load(smem_u32(tile), scratch + (long long)slot * N * N + (long long)tl * N * C, (uint32_t)(C * N * 8), bar);
       } else if constexpr (TABLE) {
         const unsigned long long q = (unsigned long long)p;
         const CUtensorMap *m = rmaps + q / N;
@@ -350,18 +296,12 @@ __global__ void __launch_bounds__(kXyL2Threads, 8) k_xy_l2(const __grid_constant
         if (threadIdx.x == 0 && !wait_count(yread + (p - RING), ITEMS, spin)) ok = false;
         __syncthreads();
       }
-      if constexpr (Cfg::TILED) {
-        // column tile x / C of the slot holds its C columns of every row contiguously
-        float2 *o = scratch + (long long)slot * N * N + (tl * C + c) * C;
+      // column tile x / C of the slot holds its C columns of every row contiguously
+      float2 *o = scratch + (long long)slot * N * N + (tl * C + c) * C;
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const int x = t + e * T;
-          o[(x / C) * (N * C) + (x % C)] = v[e];
-        }
-      } else {
-        float2 *o = scratch + (long long)slot * N * N + (long long)(tl * C + c) * N + t;
-#pragma unroll
-        for (int e = 0; e < E; ++e) o[e * T] = v[e];
+      for (int e = 0; e < E; ++e) {
+        const int x = t + e * T;
+        o[(x / C) * (N * C) + (x % C)] = v[e];
       }
       __syncthreads();  // every thread's stores issued
       // The barrier orders every thread's stores before this release (cumulativity); a
