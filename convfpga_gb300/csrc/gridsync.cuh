@@ -1,0 +1,42 @@
+// Barrier of a cooperative launch (small cubes in one launch).
+#pragma once
+
+#include "tma.cuh"
+
+namespace convgpu {
+
+constexpr unsigned kStatusQueueTimeout = 2u;
+constexpr uint32_t kSpinLimit = 1u << 22;
+
+__device__ __forceinline__ int ld_acquire(const int *p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Barrier k (k = 1, 2) of a launch waits until its counter reaches k * gridDim.x; every
+// launch uses its own counter slot, zeroed before use.
+// spin: the probe limit, read by the caller at kernel start (dep_wait_limit) so that the
+// read stays off the barrier's critical path.
+__device__ __forceinline__ bool small_grid_barrier(unsigned *slot, unsigned target, unsigned *status, uint32_t spin) {
+  __shared__ int s_ok;
+  __syncthreads();  // this block's stores for the level are done
+  if (threadIdx.x == 0) {
+    __threadfence();  // ... and visible device-wide before the arrival
+    atomicAdd(slot, 1u);
+    int ok = 0;
+    for (uint32_t i = 0; i < spin; ++i) {
+      if ((unsigned)ld_acquire(reinterpret_cast<const int *>(slot)) >= target) {
+        ok = 1;
+        break;
+      }
+      __nanosleep(32);
+    }
+    if (!ok && status) atomicOr(status, kStatusQueueTimeout);
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+}  // namespace convgpu

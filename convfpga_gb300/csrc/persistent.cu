@@ -38,12 +38,11 @@
 #include <vector>
 
 #include "engine_internal.h"
+#include "gridsync.cuh"
 #include "passes.cuh"
 
 namespace convgpu {
 
-constexpr unsigned kStatusQueueTimeout = 2u;
-constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr int kPThreads = 256;
 constexpr int kPasses = 7;
 constexpr int kPTwOffset = 65536;                      // twiddles after two 32 KiB tiles
@@ -212,12 +211,6 @@ __device__ __noinline__ void run_tile(const UJob &j, int pass, int tile, unsigne
   for (int e = 0; e < E; ++e) dst[base + (long long)(t + e * T) * stride] = v[e];
 }
 
-__device__ __forceinline__ int ld_acquire(const int *p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ void red_release_add(int *p, int v) {
   asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -296,37 +289,15 @@ __global__ void __launch_bounds__(kPThreads, 3) k_persistent_queue(const UJob *_
 }
 
 // ------------------------------------------------------------------ small cubes, one launch
-// One convolution of a small cube (N <= 64) as a single cooperative launch in three
+// One convolution of a small cube (N <= 64) as a single cooperative launch, where neither the
+// one-CTA form of N = 16 (cube16.cu) nor the tile form of N = 32 and 64 (k_tp_one, twopass.cuh,
+// which wants a cube of scratch) takes the call, in three
 // dependency levels: x+y of the filter's and the signal's planes (each block holds its
 // planes in shared memory between the two transforms), the fused z pass, inverse y+x;
 // each level's items spread over the grid, a grid barrier between levels. A 64^3 cube is 2 MiB and stays in L2, so separate launches are bound by
 // launch gaps, not by HBM. The cooperative launch makes every block resident, so the
 // barrier cannot wait on a block that never runs; each wait is still bounded and one that
 // gives up sets kStatusQueueTimeout.
-// Barrier k (k = 1, 2) of a launch waits until its counter reaches k * gridDim.x; every
-// launch uses its own counter slot, zeroed before use.
-// spin: the probe limit, read by the caller at kernel start (dep_wait_limit) so that the
-// read stays off the barrier's critical path.
-__device__ __forceinline__ bool small_grid_barrier(unsigned *slot, unsigned target, unsigned *status, uint32_t spin) {
-  __shared__ int s_ok;
-  __syncthreads();  // this block's stores for the level are done
-  if (threadIdx.x == 0) {
-    __threadfence();  // ... and visible device-wide before the arrival
-    atomicAdd(slot, 1u);
-    int ok = 0;
-    for (uint32_t i = 0; i < spin; ++i) {
-      if ((unsigned)ld_acquire(reinterpret_cast<const int *>(slot)) >= target) {
-        ok = 1;
-        break;
-      }
-      __nanosleep(32);
-    }
-    if (!ok && status) atomicOr(status, kStatusQueueTimeout);
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
 
 // Column n-slots of plane-column x of plane q in P consecutive N x N planes (row-major).
 struct PlaneCol {
@@ -463,6 +434,7 @@ std::mutex g_pmu;
 std::map<std::vector<int>, std::unique_ptr<PPlan>> g_plans;
 unsigned *g_small_slots = nullptr;  // barrier counters of the small-cube launches (a ring)
 unsigned long long g_small_next = 0;
+float2 *g_small_tiles = nullptr;  // a 64^3 cube's worth, for the signal in tile order
 std::string g_perr;
 
 cudaError_t build_plan(PPlan &p, const float2 *tw512, unsigned *status) {
@@ -580,7 +552,9 @@ void release_uneven_plans() {
   std::lock_guard<std::mutex> lk(g_pmu);
   g_plans.clear();
   if (g_small_slots) cudaFree(g_small_slots);
+  if (g_small_tiles) cudaFree(g_small_tiles);
   g_small_slots = nullptr;
+  g_small_tiles = nullptr;
   g_small_next = 0;
 }
 
@@ -602,6 +576,18 @@ cudaError_t launch_small_conv(int n, const float2 *sig, const float2 *filt, floa
     if ((e = cudaMemsetAsync(g_small_slots, 0, kSlots * sizeof(unsigned), s)) != cudaSuccess) return e;
   }
   unsigned *slot = g_small_slots + (g_small_next++ % kSlots);
+  if (n > 16) {  // in tiles, with a cube of scratch (not allocated while a graph is captured)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (!g_small_tiles && cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
+      void *p = nullptr;
+      if (cudaMalloc(&p, (size_t)64 * 64 * 64 * sizeof(float2)) == cudaSuccess) g_small_tiles = static_cast<float2 *>(p);
+      cudaGetLastError();
+    }
+    if (g_small_tiles) {
+      e = launch_tp_one(n, sig, filt, out, spec, g_small_tiles, scale, real, tw512, slot, status, s);
+      if (e != cudaErrorNotSupported) return e;
+    }
+  }
   void (*kern)(UJob, unsigned *, const float2 *, unsigned *, int) =
       n == 16 ? k_small_conv<16> : (n == 32 ? k_small_conv<32> : k_small_conv<64>);
   // attribute and grid per size, set once per device: the grid is the resident blocks, at

@@ -175,6 +175,23 @@ cudaError_t launch_tp_order(int n, const float2 *src, float2 *dst, cudaStream_t 
   return with_size(n, [&](auto k) { return order<decltype(k)::value>(src, dst, s); });
 }
 
+cudaError_t launch_tp_one(int n, const float2 *sig, const float2 *filt, float2 *out, float2 *ftiles, float2 *stiles,
+                          float scale, bool real, const float2 *tw512, unsigned *slot, unsigned *status,
+                          cudaStream_t s) {
+  void *a[] = {&sig, &filt, &out, &ftiles, &stiles, &scale, &tw512, &slot, &status};
+  auto go = [&](auto k) {
+    constexpr int N = decltype(k)::value;
+    static_assert(tp_one_smem<N>() <= 48 << 10, "no attribute needed");
+    const void *kern = real ? (const void *)k_tp_one<N, true> : (const void *)k_tp_one<N, false>;
+    return cudaLaunchCooperativeKernel(kern, dim3(N / TpShape<N>::J * (N / 2)), dim3(kTpOneThreads<N>), a,
+                                       tp_one_smem<N>(), s);
+  };
+  if (sm_count() < 128) return cudaErrorNotSupported;  // every CTA resident, one a SM
+  if (n == 32) return go(std::integral_constant<int, 32>{});
+  if (n == 64) return go(std::integral_constant<int, 64>{});
+  return cudaErrorNotSupported;
+}
+
 cudaError_t launch_tp_fwd_table(int n, const float2 *const *srcs, const CUtensorMap *dst_maps, int nvol,
                                 const float2 *tw512, cudaStream_t s) {
   TpArgs a = args(n, nullptr, nullptr, nvol, tw512);

@@ -30,6 +30,7 @@
 // own engine with transposes between (kernels/conv3D.cl:71-420).
 #pragma once
 
+#include "gridsync.cuh"
 #include "tilefft.cuh"
 #include "tilestream.cuh"
 
@@ -730,6 +731,133 @@ __global__ void __launch_bounds__(256) k_tp_order(const float2 *src, float2 *dst
     const float2 p = rows[2 * u][x], q = rows[2 * u + 1][x];
     stg_unit(dst + (((long long)g * N + x0 + x) * (R * H * C) + (k2 * H + kz0) * C + u) * 2,
              Pair{pk(p.x, q.x), pk(p.y, q.y)});
+  }
+}
+
+// One convolution of a small cube in one cooperative launch: the three passes on one tile a
+// CTA, grid barriers between them. Two groups per CTA, the filter's and the signal's, which
+// hand over through shared memory at the product. Tiles are read and written straight from
+// registers: latency is all there is (L2 round trips, exchanges, two barriers). One cube of 64^3
+// 16.4 us, of 32^3 12.3, where whole planes and z tiles a block (persistent.cu) took 22.5 and
+// 16.4.
+template <int N>
+constexpr int kTpOneThreads = 2 * TpOuterTile<N>::NT;
+template <int N>
+constexpr int tp_one_smem() {
+  return 1024 + 2 * kTpBuf<N> + TpOuterTile<N>::kTwBytes + TpMidTile<N>::kTwBytes + TpShape<N>::J * 16 + N * 8;
+}
+
+__device__ __forceinline__ Pair ldcg_unit(const float2 *p) {
+  Pair a;
+  asm volatile("ld.global.cg.v2.b64 {%0, %1}, [%2];" : "=l"(a.re), "=l"(a.im) : "l"(p) : "memory");
+  return a;
+}
+
+template <int N, bool REAL>
+__global__ void __launch_bounds__(kTpOneThreads<N>, 1)
+    k_tp_one(const float2 *sig, const float2 *filt, float2 *out, float2 *ftiles, float2 *stiles, float scale,
+             const float2 *tw512, unsigned *slot, unsigned *status) {
+  using OT = TpOuterTile<N>;
+  using MT = TpMidTile<N>;
+  constexpr int J = OT::J, R = N / J, C = MT::C, H = N / 2, NT = OT::NT, TILE = R * H * C;
+  constexpr bool kTmem = MT::R2 > 1;
+  static_assert(MT::NT == NT && N * J / C == R * H, "a tile of either kind per CTA and group");
+  extern __shared__ __align__(1024) unsigned char smraw[];
+  const uint32_t sm = smem_u32(smraw), tiles = sm + 1024, tw = tiles + 2 * kTpBuf<N>, mtw = tw + OT::kTwBytes,
+                 utw = mtw + MT::kTwBytes, lin = utw + J * 16;
+  const int g = threadIdx.x / NT, tid = threadIdx.x % NT, w = blockIdx.x, y0 = w / H, zz = w % H;
+  const uint32_t spin = dep_wait_limit(status, kSpinLimit), buf = tiles + g * kTpBuf<N>;
+  OT ot(tid, 1 + g, tw);
+  ot.at(buf);
+  Pair v[16];
+  {
+    const long long row = ((long long)zz * N + y0 + R * ot.row) * N + ot.t;
+    if (REAL && g == 0) {
+      const float *p = reinterpret_cast<const float *>(filt) + row, *q = p + (long long)H * N * N;
+      float a[16], b[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) a[e] = __ldcg(p + OT::R2 * e), b[e] = __ldcg(q + OT::R2 * e);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] = {pk(a[e] + b[e], a[e] - b[e]), 0ull};
+    } else {
+      const float2 *p = (g ? sig : filt) + row, *q = p + (long long)H * N * N;
+      float2 a[16], b[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) a[e] = __ldcg(p + OT::R2 * e), b[e] = __ldcg(q + OT::R2 * e);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] = {pk(a[e].x + b[e].x, a[e].x - b[e].x), pk(a[e].y + b[e].y, a[e].y - b[e].y)};
+    }
+  }
+  OT::fill_tw(tw, tw512);
+  MT::fill_tw(mtw, tw512);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    const float2 u = __ldg(tw512 + i * (512 / N));
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(lin + i * 8), "f"(u.x), "f"(u.y) : "memory");
+  }
+  uint32_t tmem = 0;
+  if constexpr (kTmem) tmem = tp_tmem_alloc<64>(sm);
+  __syncthreads();
+  tp_step_tw<N>(utw, lin, threadIdx.x, y0, zz);
+  __syncthreads();
+  // unit of output (kx, j') in tile order
+  auto unit = [&](int kx, int j) { return ((long long)((j / C) * N + kx) * TILE + w * C + j % C) * 2; };
+  ot.forward(v, [] {});
+  {
+    float2 *o = g ? stiles : ftiles;
+#pragma unroll
+    for (int i = 0; i < OT::B3; ++i)
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const Pair s = lds_pair(utw + j * 16);
+        stg_unit(o + unit(ot.q + i * NT, j), pmul_tw(v[i * J + j], s.re, s.im));
+      }
+  }
+  bool ok = small_grid_barrier(slot, gridDim.x, status, spin);
+  if (ok) {
+    MT mt(tid, 1 + g, kTmem ? tp_tmem_warp(tmem, 0) : 0u, mtw);
+    mt.at(buf);
+    float2 *tile = (g ? stiles : ftiles) + (long long)w * TILE * 2;
+    auto nat = [&](int e) { return ((mt.row * H + mt.t + MT::R2 * e) * C + mt.c) * 2; };
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] = ldcg_unit(tile + nat(e));
+    mt.forward(v, [] {});
+    __syncthreads();
+    if (g == 0) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) sts_pair(tiles + (k * NT + tid) * 16, v[k]);
+    }
+    __syncthreads();
+    if (g == 1) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = pswap(pmul(v[k], lds_pair(tiles + (k * NT + tid) * 16)));
+      mt.inverse(v, [] {});
+#pragma unroll
+      for (int e = 0; e < 16; ++e) stg_unit(tile + nat(e), pswap(v[e]));
+    }
+    ok = small_grid_barrier(slot, 2u * gridDim.x, status, spin);
+    // the last to pass leaves the counter at zero, for a replay of a captured launch
+    if (ok && threadIdx.x == 0 && atomicAdd(slot, 1u) == 3u * gridDim.x - 1u) atomicExch(slot, 0u);
+  }
+  if constexpr (kTmem) tp_tmem_free<64>(tmem);
+  if (!ok || g == 0) return;
+#pragma unroll
+  for (int i = 0; i < OT::B3; ++i)
+#pragma unroll
+    for (int j = 0; j < J; ++j) v[i * J + j] = ldcg_unit(stiles + unit(ot.q + i * NT, j));
+#pragma unroll
+  for (int i = 0; i < OT::B3; ++i)
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const Pair s = lds_pair(utw + j * 16);
+      v[i * J + j] = pmul_tw(pswap(v[i * J + j]), s.re, s.im);
+    }
+  ot.inverse(v, [] {});
+  float2 *o0 = out + ((long long)zz * N + y0 + R * ot.row) * N + ot.t, *o1 = o0 + (long long)H * N * N;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const Pair p = v[e];  // swapped: re holds im
+    o0[OT::R2 * e] = make_float2((lo_of(p.im) + hi_of(p.im)) * scale, (lo_of(p.re) + hi_of(p.re)) * scale);
+    o1[OT::R2 * e] = make_float2((lo_of(p.im) - hi_of(p.im)) * scale, (lo_of(p.re) - hi_of(p.re)) * scale);
   }
 }
 
