@@ -17,10 +17,10 @@
 //                         x-fwd -> y-fwd                       (z done inside CONV_FZ)
 //   signal:               x-fwd -> y-fwd -> z[fwd, (.)F, inv] -> y-inv -> x-inv(scale)
 // With the fused pass in the plan (N = 128, 256, 512), x-fwd -> y-fwd and y-inv -> x-inv
-// each run as one L2-staged launch. With the two-pass transform in the plan (N = 128, 256)
+// each run as one L2-staged launch. With the two-pass transform in the plan (N = 32 to 256)
 // the passes are instead tiles of x and part of y, then tiles of the rest of y and z with the
-// product, then the mirror of the first (enqueue_tp). One cube of N <= 64 runs all of it in one cooperative
-// launch (persistent.cu: launch_small_conv).
+// product, then the mirror of the first (enqueue_tp). Cubes of N = 16, and one cube of N = 32
+// or 64, run all of it in one launch (cube16.cu, persistent.cu: launch_small_conv).
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 

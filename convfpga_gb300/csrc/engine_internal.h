@@ -107,8 +107,8 @@ cudaError_t launch_tp_mid_table(int n, const float2 *const *srcs, float2 *const 
 cudaError_t launch_tp_inv_table(int n, const CUtensorMap *src_maps, float2 *const *dsts, int nvol, float scale,
                                 const float2 *tw512, cudaStream_t s);
 // The process's scratch cubes in tile order, tp_scratch_cubes(n) of them (512 MiB, 256 at
-// N = 64, 128 at N = 32): the signals a call transforms at a time. Fewer cost more in launches than L2 gives back: a
-// call of 16 cubes of 128^3 took 403 us by 4, 357 by 8 and 339 at once. Null when not
+// N = 64, 128 at N = 32): the signals a call transforms at a time. Fewer cost more in launches
+// than L2 gives back: a call of 16 cubes of 128^3 took 403 us by 4, 357 by 8 and 339 at once. Null when not
 // allocated and not (or not to be) allocatable.
 constexpr int kTpScratchCubes32 = 512, kTpScratchCubes64 = 128, kTpScratchCubes128 = 32, kTpScratchCubes256 = 4;
 int tp_scratch_cubes(int n);

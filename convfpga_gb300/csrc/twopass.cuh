@@ -26,8 +26,8 @@
 // A spectrum in tile order holds, in tile (g, kx), unit (k2 N/2 + kz') C + c: the pairs
 // (kz = 2 kz' and 2 kz' + 1) at ky = g C + c + J k2.
 //
-// Persistent CTAs take tiles in order through a few buffers in shared memory. The reference streams each axis through its
-// own engine with transposes between (kernels/conv3D.cl:71-420).
+// Persistent CTAs take tiles in order through a few buffers in shared memory. The reference
+// streams each axis through its own engine with transposes between (kernels/conv3D.cl:71-420).
 #pragma once
 
 #include "gridsync.cuh"
@@ -43,10 +43,12 @@ namespace convgpu {
 //   128: 32 KB tiles, 4 groups of 128 threads, 6 buffers. 64: 16 KB, 8 groups of 64, 12
 //   buffers. 32: 8 KB, 16 groups of a warp, 24 buffers.
 // One CTA of 16 compute warps per SM, since a thread holds a tile's 16 pairs (64 registers).
-// Measured, us: 4 cubes of 256^3: k_tp_fwd 187 and k_tp_inv 191 (1.07 GB each: 5.7 TB/s; two
+// Measured, us: 4 cubes of 256^3: k_tp_fwd 177 and k_tp_inv 180 (1.07 GB each: 6.0 TB/s; two
 // CTAs of one tile each, loaded and stored from registers, took 215 and 276), k_tp_mid with
-// a filter per cube 287 (1.6 GB: 5.6 TB/s), so 850 for a batch with its filters, against
-// 1,083 for the L2-staged x+y passes and the fused z pass.
+// a filter per cube 285 (1.6 GB: 5.6 TB/s), so 808 for a batch with its filters, against
+// 1,083 for the L2-staged x+y passes and the fused z pass. At N = 64 a pass of 33 cubes takes
+// 30 to 39: 128 KB of tiles per SM take some 6.3 us whatever the size, and 33 cubes are 3.5
+// rounds of that.
 template <int N>
 struct TpShape;
 template <>
@@ -121,6 +123,7 @@ template <int N>
 constexpr int tp_mid_smem() {
   return 1024 + TpShape<N>::B * kTpBuf<N> + TpMidTile<N>::kTwBytes;
 }
+
 // Step twiddles of outer tile (y0, zz): entry j' = {W_N^(y0 j'), W_N^(y0 j' + zz)} as
 // {c0, c1, s0, s1}; written by the group's first J threads into one of its two sets, since
 // slow threads may still read the previous tile's.

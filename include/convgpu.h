@@ -55,7 +55,7 @@ extern "C" {
  * filter, and the result equals that of the same filter given as complex values with
  * zero imaginary parts. Not with CONVGPU_FILTER_IS_SPECTRUM. The reference takes complex
  * filters only; its real Gaussian filters are stored with zero imaginary parts.
- * Calls of N = 128 and 256 on the FP32 path also hold 512 MiB of scratch cubes per size,
+ * Calls of N = 32 to 256 on the FP32 path also hold scratch cubes (128, 256, 512 and 512 MiB),
  * allocated by the first such call and kept until fpga_final; without them (no memory) the
  * calls run the passes of the other plan variants. A call captured into a graph allocates
  * none, so make one call of its size before the capture.
@@ -114,7 +114,7 @@ typedef struct {
 /* Convolutions of different power-of-two sizes in one call (one filter per job),
  * on device pointers. Extends fpgaf_conv3D_svm_batch to uneven sizes.
  * Default: one CUDA graph, cached per sequence of job sizes, in which every size class is
- * a branch of seven launches (one per pass) over all jobs of that size; tensor maps are
+ * a branch of one to seven launches over all jobs of that size; tensor maps are
  * rebuilt only when a job's buffers move. CONVGPU_UNEVEN_QUEUE runs the batch as one
  * persistent launch fed by a device work queue of (job, pass, tile) items (at most
  * 4096 jobs), also replayed from a cached graph. Graphs and filter-spectrum workspaces
@@ -167,16 +167,17 @@ int convgpu_autotune(const unsigned *sizes, unsigned count, int write_cache);
 /* Plan-table entry of cube size N for pass kind (0 x pass, 1 y/z passes, 2 fused z pass,
  * 3 fused z pass with the filter's z transform, 4 x and y: 0 separate passes; N = 256:
  * 1 one pass staged through an L2-resident scratch ring, 2 one pass on 8-CTA clusters;
- * N = 128 and 512: 1 one pass staged through an L2-resident scratch ring; N = 128 and 256,
- * the default there: 3 the two-pass 3D transform, for calls whose cubes are 16-byte aligned
- * and whose outputs are the signals or do not overlap them (other calls run 1);
+ * N = 128 and 512: 1 one pass staged through an L2-resident scratch ring; N = 32 to 256, the
+ * default there: 3 the two-pass 3D transform, for calls whose cubes are 16-byte aligned and
+ * whose outputs are the signals or do not overlap them, and for spectra given by the caller
+ * where it is faster (other calls run 1 at N = 128 and 256, else 0);
  * 5 tensor-core kernels of CONVGPU_TENSOR_SPLIT, N = 256: 0 tcgen05 (TMEM accumulators),
  * 1 mma.sync; 6 x and y passes of the tcgen05 split path, N = 256: 0 separate passes, 1 one
  * pass staged through the L2-resident scratch ring; 7 spectra of real filters
  * (CONVGPU_FILTER_REAL, FP32 path, N >= 64): 0 full spectra, 1 Hermitian half spectra, kx up
  * to N/2 only, with a fused z pass that serves a column tile and its mirror from one read):
- * sets it to set_to (0 or 1; 0..2 for kind 4, 0..3 with N = 128 or 256) when set_to >= 0, and returns the current
- * variant (or a negative CONVGPU_E* code). */
+ * sets it to set_to (0 or 1; 0..2 for kind 4, 0..3 with N = 32 to 256) when set_to >= 0, and
+ * returns the current variant (or a negative CONVGPU_E* code). */
 int convgpu_plan_variant(unsigned N, int kind, int set_to);
 
 /* Waits for the device, then returns and clears the library's device status word in
