@@ -513,7 +513,7 @@ static cudaError_t pass_tp(int slot, double bytes, cudaStream_t s, F &&launch) {
 }
 static cudaError_t tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, cudaStream_t s,
                           const float2 *src2 = nullptr, float2 *dst2 = nullptr, int nvol2 = 0) {
-  return pass_tp(12, (real ? 28.0 : 32.0) * n * n * n * (nvol + nvol2), s,
+  return pass_tp(12, ((real ? 28.0 : 32.0) * nvol + 32.0 * nvol2) * n * n * n, s,
                  [&] { return launch_tp_fwd(n, src, dst, nvol, real, g.tw512, s, src2, dst2, nvol2); });
 }
 static cudaError_t tp_mid(int n, int mode, const float2 *src, float2 *dst, const float2 *filt, long long filt_vol,
@@ -560,8 +560,8 @@ static cudaError_t enqueue_tp(int n, const float2 *sig, const float2 *filt, floa
   const uintptr_t fbytes = (uintptr_t)V * (per_signal ? how_many : 1) * (real ? 4 : 8);
   const bool filters_apart = fu + fbytes <= ou || ou + bytes <= fu;
   if (direct) {
-    if (!real && filters_apart) {
-      CG_TRY(tp_fwd(n, filt, ws, how_many, false, s, sig, out, how_many));
+    if (filters_apart) {
+      CG_TRY(tp_fwd(n, filt, ws, how_many, real, s, sig, out, how_many));
     } else {
       CG_TRY(tp_fwd(n, filt, ws, how_many, real, s));
       CG_TRY(tp_fwd(n, sig, out, how_many, false, s));
@@ -572,18 +572,14 @@ static cudaError_t enqueue_tp(int n, const float2 *sig, const float2 *filt, floa
   }
   const unsigned chunk = std::min<unsigned>(how_many, tp_scratch_cubes(n));
   const bool spectrum = !per_signal && how_many > kTpSharedPairCubes && V * how_many > kTpSharedPairPoints;
-  // All filters go with the first chunk of signals (into the scratch), in one launch unless
-  // they are real.
+  // All filters go with the first chunk of signals (into the scratch), in one launch.
   const int nf = per_signal ? (int)how_many : 1;
-  if (real)
-    CG_TRY(tp_fwd(n, filt, ws, nf, true, s));
-  else
-    CG_TRY(tp_fwd(n, filt, ws, nf, false, s, sig, scratch, (int)chunk));
+  CG_TRY(tp_fwd(n, filt, ws, nf, real, s, sig, scratch, (int)chunk));
   if (spectrum) CG_TRY(tp_mid(n, kTpFwd, ws, ws, nullptr, 0, 1, s));
   for (unsigned i = 0; i < how_many; i += chunk) {
     const int k = (int)std::min(chunk, how_many - i);
     const float2 *f = per_signal ? ws + i * V : ws;
-    if (real || i > 0) CG_TRY(tp_fwd(n, sig + i * V, scratch, k, false, s));
+    if (i > 0) CG_TRY(tp_fwd(n, sig + i * V, scratch, k, false, s));
     CG_TRY(tp_mid(n, spectrum ? kTpSpectrum : kTpPair, scratch, scratch, f, per_signal ? V : 0, k, s));
     CG_TRY(tp_inv(n, scratch, out + i * V, k, scale, s));
   }

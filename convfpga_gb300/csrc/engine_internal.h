@@ -80,7 +80,7 @@ constexpr int kTpPair = 0, kTpSpectrum = 1, kTpFwd = 2;
 // Forward outer pass (cubes, or N^3 floats each with `real`, to tile order), middle pass, and
 // inverse outer pass (tile order to cubes). src and dst of the outer passes must not
 // overlap; the middle pass may write over its source or its filters. The forward pass can
-// take a second set of (complex) cubes along. cudaErrorNotSupported
+// take a second set of cubes along, complex in any case. cudaErrorNotSupported
 // when an operand is not 16-byte aligned.
 cudaError_t launch_tp_fwd(int n, const void *src, float2 *dst, int nvol, bool real, const float2 *tw512,
                           cudaStream_t s, const float2 *src2 = nullptr, float2 *dst2 = nullptr, int nvol2 = 0);

@@ -146,7 +146,7 @@ cudaError_t launch_tp_fwd(int n, const void *src, float2 *dst, int nvol, bool re
   a.first = nvol;
   a.src2 = src2;
   CUtensorMap m, m2;
-  if (!tp_size(n) || !aligned16(src) || !aligned16(src2) || (real && nvol2) || !tp_encode_tiles(&m, dst, n, nvol) ||
+  if (!tp_size(n) || !aligned16(src) || !aligned16(src2) || !tp_encode_tiles(&m, dst, n, nvol) ||
       !tp_encode_tiles(&m2, nvol2 ? dst2 : dst, n, nvol2 ? nvol2 : nvol))
     return cudaErrorNotSupported;
   return with_size(n, [&](auto k) { return fwd<decltype(k)::value>(a, real, m, m2, s); });

@@ -217,7 +217,8 @@ __device__ __forceinline__ uint32_t tp_run_off(int kx, int c) {
   return (uint32_t)(kx * C + (c ^ ((kx * C / 8) & (C - 1)))) * 16;
 }
 
-// Forward outer pass. REAL: the source holds N^3 floats per cube. mdst: the destination in
+// Forward outer pass. REAL: the first a.first cubes hold N^3 floats each (real filters), the
+// others complex values. mdst: the destination in
 // tile order, dims (2 C values of a run, tiles, runs of a tile), box (2 C, N, 1), for the
 // first a.first cubes, mdst2 for the others (a filter and its signals in one launch).
 //
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(kTpFwdThreads<N>, 1)
   // are in order). Turn n is group n % G's and buffer G + n % SB's.
   const uint32_t staged = sm + 512, grant = sm + 576;
   static_assert(G <= 16 && SB <= 8, "barriers in the first KB");
-  constexpr uint32_t kRow = REAL ? N * 4 : N * 8;
+  auto real = [&](int vol) { return REAL && vol < a.first; };  // this cube's rows are floats
   auto load = [&](int n, int w) {  // by one warp: 2 J row copies, row (j, plane) at j ROWB + plane N 8
     const int lane = threadIdx.x & 31;
     if (w >= ntiles) {
@@ -267,18 +268,19 @@ __global__ void __launch_bounds__(kTpFwdThreads<N>, 1)
       return;
     }
     const int vol = w / (R * H), r = w % (R * H), y0 = r / H, zz = r % H;
-    // src_vol counts values, complex or (REAL) float
+    // src_vol counts values, complex or float
+    const uint32_t row = real(vol) ? N * 4 : N * 8;
     const char *src = a.srcs ? (const char *)a.srcs[vol]
                              : (vol < a.first ? (const char *)a.src + vol * a.src_vol * (REAL ? 4 : 8)
-                                              : (const char *)a.src2 + (vol - a.first) * a.src_vol * (REAL ? 4 : 8));
+                                              : (const char *)a.src2 + (vol - a.first) * a.src_vol * 8);
     if (lane == 0) {
       st.set_tile(n, w);
-      mbar_arrive_expect_tx(st.full(n), 2 * J * kRow);
+      mbar_arrive_expect_tx(st.full(n), 2 * J * row);
     }
     __syncwarp();
     for (int i = lane; i < 2 * J; i += 32) {
       const int j = i >> 1, z = zz + (i & 1) * H;
-      bulk_load(st.buf(kStager ? n % G : n) + j * TT::ROWB + (i & 1) * (N * 8), src + ((long long)z * N + y0 + R * j) * kRow, kRow,
+      bulk_load(st.buf(kStager ? n % G : n) + j * TT::ROWB + (i & 1) * (N * 8), src + ((long long)z * N + y0 + R * j) * row, row,
                 st.full(n));
     }
   };
@@ -387,13 +389,17 @@ __global__ void __launch_bounds__(kTpFwdThreads<N>, 1)
     int next = 0;  // the group's next tile, claimed ahead of its use below
     if (kClaims && tid == 0) next = tp_claim<N>(0, n + G, gridDim.x * G, ntiles);
     Pair v[16];
+    if (real(w / (R * H))) {
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const int x = tt.t + TT::R2 * e;
-      if constexpr (REAL) {
+      for (int e = 0; e < 16; ++e) {
+        const int x = tt.t + TT::R2 * e;
         const float p = lds_f(tt.rowb + x * 4), q = lds_f(tt.rowb + N * 8 + x * 4);
         v[e] = {pk(p + q, p - q), 0ull};
-      } else {
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const int x = tt.t + TT::R2 * e;
         const float2 p = lds_f2(tt.rowb + x * 8), q = lds_f2(tt.rowb + N * 8 + x * 8);
         v[e] = {pk(p.x + q.x, p.x - q.x), pk(p.y + q.y, p.y - q.y)};
       }
