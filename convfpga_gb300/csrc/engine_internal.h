@@ -122,6 +122,8 @@ cudaError_t launch_cube16(const float2 *sig, const void *filt, float2 *out, int 
                           bool spectrum, float scale, cudaStream_t s);
 cudaError_t launch_cube16_table(const float2 *const *sigs, const float2 *const *filts, float2 *const *outs, int cubes,
                                 float scale, cudaStream_t s);
+// Forward transforms of 16^3 cubes in one launch; dst is src or apart from it.
+cudaError_t launch_spectrum16(const float2 *src, float2 *dst, int cubes, cudaStream_t s);
 cudaError_t prepare_cube16();
 // Fused x + y pass over `nplanes` planes (N = 128, 256, 512; cudaErrorNotSupported otherwise
 // or when tensor maps cannot describe the operands). Plan kind kKindXy, N = 256: variant 1
