@@ -248,7 +248,8 @@ NOALLOC_SCRATCH_ELEMS = 1 << 21
 def conv3d_device_noalloc(n: int, sig, filt, out, how_many: int, flags: int = 0, stream=None) -> None:
     """Like conv3d_device, for callers that cannot allocate device memory: its scratch
     is a fixed 16 MiB array inside the library (NOALLOC_SCRATCH_ELEMS complex values),
-    shared by all calls (overlapping calls race). Raises on error."""
+    shared by all calls (overlapping calls race, unless the filter is given as a spectrum,
+    which takes no scratch). Raises on error."""
     rc = load_library().convgpu_conv3d_device_noalloc(n, _dev_ptr(sig), _dev_ptr(filt), _dev_ptr(out), how_many,
                                                       flags, _stream_ptr(stream))
     _check(rc, "convgpu_conv3d_device_noalloc")

@@ -15,10 +15,12 @@
 namespace convgpu {
 
 // Launches one per-axis pass over `nvol` cubes of size n (axis 0 = x, 1 = y, 2 = z).
-// op: OP_FWD / OP_INV / OP_CONV / OP_CONV_FZ (passes.cuh). src may equal dst.
+// op: OP_FWD / OP_INV / OP_CONV / OP_CONV_FZ (passes.cuh). src may equal dst. `unordered`: the
+// caller does not keep other launches from running beside this one (no CallOrder), so it uses
+// no counter that they share.
 cudaError_t launch_axis_pass(int n, int axis, int op, const float2 *src, float2 *dst, const float2 *filt,
                              long long filt_vol_elems, int nvol, float scale, const float2 *tw512,
-                             cudaStream_t s);
+                             cudaStream_t s, bool unordered = false);
 
 // x pass of `nvol` cubes of real data (N^3 floats each) into complex dst: the first pass of
 // a real filter's transform (CONVGPU_FILTER_REAL).
@@ -139,7 +141,7 @@ cudaError_t launch_axis_pass_planes(int n, int axis, int op, const float2 *src, 
 // launch_axis_pass with an explicit shape variant (the autotuner times both).
 cudaError_t launch_axis_pass_variant(int n, int axis, int op, const float2 *src, float2 *dst, const float2 *filt,
                                      long long filt_vol_elems, int nvol, float scale, const float2 *tw512,
-                                     cudaStream_t s, int variant);
+                                     cudaStream_t s, int variant, bool unordered = false);
 
 // Table-mode launches (one launch over cubes at unrelated addresses): per-volume tensor
 // maps of the source (and, for the fused z pass, of the filter spectrum) and per-volume

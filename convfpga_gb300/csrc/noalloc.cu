@@ -24,7 +24,8 @@
 // same array, which keeps the previous call's contents; nothing in it has to start at
 // zero, because each call's first filter pass writes every element that call later
 // reads. Calls that overlap on the GPU (different streams, or host threads without
-// ordering) race on the array.
+// ordering) race on the array; calls with CONVGPU_FILTER_IS_SPECTRUM share no written
+// memory with any other call (launch_axis_pass's `unordered`) and may overlap.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -116,7 +117,7 @@ int conv_device_noalloc(unsigned n, const void *d_sig, const void *d_filt, void 
   auto run = [&](int axis, int op, const float2 *src, float2 *dst, const float2 *f, long long fv, int nvol,
                  float sc) {
     if (e != cudaSuccess) return;
-    e = launch_axis_pass((int)n, axis, op, src, dst, f, fv, nvol, sc, d->tw512, s);
+    e = launch_axis_pass((int)n, axis, op, src, dst, f, fv, nvol, sc, d->tw512, s, true);
     if (e == cudaSuccess) ++launches;
   };
   if (flags & kIsSpectrum) {

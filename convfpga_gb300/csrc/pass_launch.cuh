@@ -47,6 +47,7 @@ struct PassReq {
   int variant;  // shape variant 0 / 1
   bool real_src;  // x pass of real rows (a.src holds floats): k_rows_real
   int half;       // Hermitian half-spectrum layout of pitch half_pitch(N) (herm.cuh), else 0
+  bool unordered;  // other launches may run beside this one: it shares no counter with them
   PassArgs a;
   cudaStream_t s;
 };
@@ -63,7 +64,7 @@ bool encode_runs_map(CUtensorMap *m, const void *base, int vals, long long tiles
 // As encode_cube_map over planes of N rows of `width` complex values (row pitch = width).
 bool encode_pitched_map(CUtensorMap *m, const void *base, int width, int n, long long nplanes, int axis, int cols);
 
-// The device's tile counter of pairs512.cuh's kernels (calls on one device are in stream order).
+// The device's tile counter of pairs512.cuh's kernels, for calls that the engine orders.
 unsigned *zpair_claims();
 
 template <int N>
@@ -169,8 +170,11 @@ static cudaError_t launch_strided(const PassReq &r) {
   using S = Shape<N, V>;
   constexpr int E = S::E, COLS = S::SC;
   constexpr bool HAS_F = (OP == OP_CONV || OP == OP_CONV_FZ);
+  // The tiles of k_zpair are claimed from one counter of the device. A launch that others may run
+  // beside keeps to k_strided_tma, which shares nothing: a no-allocation call of one 512^3 cube
+  // takes 2,180 us so, and 2,239 with k_zpair on fixed shares of the tiles.
   if constexpr (N == 512 && HAS_F)
-    if (r.mode != kModeTable && r.axis == 2) {
+    if (r.mode != kModeTable && r.axis == 2 && !r.unordered) {
       if ((reinterpret_cast<uintptr_t>(r.a.dst) & 15u) != 0) return cudaErrorNotSupported;
       return launch_zpair<false, OP == OP_CONV_FZ>(r);
     }

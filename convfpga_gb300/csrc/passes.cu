@@ -268,7 +268,7 @@ static PassArgs make_args(int n, const float2 *src, float2 *dst, const float2 *f
 // ------------------------------------------------------------------ entry points
 cudaError_t launch_axis_pass_variant(int n, int axis, int op, const float2 *src, float2 *dst, const float2 *filt,
                                      long long filt_vol_elems, int nvol, float scale, const float2 *tw512,
-                                     cudaStream_t s, int variant) {
+                                     cudaStream_t s, int variant, bool unordered) {
   if (nvol <= 0) return cudaSuccess;
   if ((op == OP_CONV || op == OP_CONV_FZ) && axis != 2) return cudaErrorInvalidValue;
   if (size_index(n) < 0) return cudaErrorInvalidValue;
@@ -279,6 +279,7 @@ cudaError_t launch_axis_pass_variant(int n, int axis, int op, const float2 *src,
   r.nvol = nvol;
   r.nplanes = nvol * n;
   r.variant = variant;
+  r.unordered = unordered;
   r.a = make_args(n, src, dst, filt, filt_vol_elems, scale, tw512);
   r.s = s;
   return dispatch(n, r);
@@ -286,9 +287,9 @@ cudaError_t launch_axis_pass_variant(int n, int axis, int op, const float2 *src,
 
 cudaError_t launch_axis_pass(int n, int axis, int op, const float2 *src, float2 *dst, const float2 *filt,
                              long long filt_vol_elems, int nvol, float scale, const float2 *tw512,
-                             cudaStream_t s) {
+                             cudaStream_t s, bool unordered) {
   return launch_axis_pass_variant(n, axis, op, src, dst, filt, filt_vol_elems, nvol, scale, tw512, s,
-                                  get_pass_variant(n, pass_kind(axis, op)));
+                                  get_pass_variant(n, pass_kind(axis, op)), unordered);
 }
 
 cudaError_t launch_axis_pass_planes(int n, int axis, int op, const float2 *src, float2 *dst, int nplanes, float scale,

@@ -76,7 +76,9 @@ int convgpu_conv3d_device(unsigned N, const float2 *d_sig, const float2 *d_filte
  * CONVGPU_EINVAL. CONVGPU_TENSOR_SPLIT returns CONVGPU_EUNSUPPORTED.
  * The first call on a device sets that device up (looks up the array's address and
  * fills a twiddle table), so make it before any stream capture. All calls share the
- * array: calls that overlap on the GPU race. Like convgpu_conv3d_device it returns once
+ * array: calls that overlap on the GPU race, except that calls with
+ * CONVGPU_FILTER_IS_SPECTRUM use none of it and may overlap any other call. Like
+ * convgpu_conv3d_device it returns once
  * the work is enqueued; a kernel that gives up a bounded wait reports it through
  * convgpu_device_status, not through this call's return code. */
 #define CONVGPU_NOALLOC_SCRATCH_ELEMS (1u << 21)
