@@ -93,7 +93,8 @@ cudaError_t launch_tp_inv(int n, const float2 *src, float2 *dst, int nvol, float
 // A spectrum from natural to tile order (any 8-byte aligned source).
 cudaError_t launch_tp_order(int n, const float2 *src, float2 *dst, cudaStream_t s);
 // One convolution of a cube of N = 32 or 64 in one cooperative launch: the filter (N^3 floats
-// with `real`) and the signal go through ftiles and stiles, N^3 each. slot: a zeroed counter.
+// with `real`) and the signal go through ftiles and stiles, N^3 each. slot: two zero words,
+// zero again after the launch.
 cudaError_t launch_tp_one(int n, const float2 *sig, const float2 *filt, float2 *out, float2 *ftiles, float2 *stiles,
                           float scale, bool real, const float2 *tw512, unsigned *slot, unsigned *status,
                           cudaStream_t s);

@@ -14,8 +14,8 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
   return v;
 }
 
-// Barrier k (k = 1, 2) of a launch waits until its counter reaches k * gridDim.x; every
-// launch uses its own counter slot, zeroed before use.
+// Barrier k (k = 1, 2) of a launch waits until slot[0] reaches k * gridDim.x. Both words of
+// slot are zero at launch and, by small_grid_leave, again at its end.
 // spin: the probe limit, read by the caller at kernel start (dep_wait_limit) so that the
 // read stays off the barrier's critical path.
 __device__ __forceinline__ bool small_grid_barrier(unsigned *slot, unsigned target, unsigned *status, uint32_t spin) {
@@ -37,6 +37,18 @@ __device__ __forceinline__ bool small_grid_barrier(unsigned *slot, unsigned targ
   }
   __syncthreads();
   return s_ok != 0;
+}
+
+// By every CTA, after its last barrier or the one that gave up (ok: none did): the last to leave
+// sets both words back to zero, so that a launch that gave up leaves nothing to the next one
+// or to a replay of itself. A barrier that was passed has seen this CTA's arrival; one that
+// gave up may not have.
+__device__ __forceinline__ void small_grid_leave(unsigned *slot, bool ok) {
+  if (threadIdx.x != 0) return;
+  if (!ok) __threadfence();
+  if (atomicAdd(slot + 1, 1u) != gridDim.x - 1) return;
+  atomicExch(slot, 0u);
+  atomicExch(slot + 1, 0u);
 }
 
 }  // namespace convgpu

@@ -393,12 +393,16 @@ __global__ void __launch_bounds__(kPThreads, 3) k_small_conv(UJob j, unsigned *s
       xy_planes_small<N, false>(j.sig + (w - NI) * PL, j.out + (w - NI) * PL, 1.f, smraw, tw512);
     __syncthreads();
   }
-  if (!small_grid_barrier(slot, gridDim.x, status, spin)) return;
-  for (int w = blockIdx.x; w < ptiles(N); w += gridDim.x) {
-    run_tile<N>(j, 4, w, smraw, tw512);
-    __syncthreads();
+  bool ok = small_grid_barrier(slot, gridDim.x, status, spin);
+  if (ok) {
+    for (int w = blockIdx.x; w < ptiles(N); w += gridDim.x) {
+      run_tile<N>(j, 4, w, smraw, tw512);
+      __syncthreads();
+    }
+    ok = small_grid_barrier(slot, 2u * gridDim.x, status, spin);
   }
-  if (!small_grid_barrier(slot, 2u * gridDim.x, status, spin)) return;
+  small_grid_leave(slot, ok);
+  if (!ok) return;
   for (int w = blockIdx.x; w < NI; w += gridDim.x) {
     xy_planes_small<N, true>(j.out + w * PL, j.out + w * PL, j.scale, smraw, tw512);
     __syncthreads();
@@ -432,8 +436,7 @@ struct PPlan {
 
 std::mutex g_pmu;
 std::map<std::vector<int>, std::unique_ptr<PPlan>> g_plans;
-unsigned *g_small_slots = nullptr;  // barrier counters of the small-cube launches (a ring)
-unsigned long long g_small_next = 0;
+unsigned *g_small_slot = nullptr;  // barrier words of the small-cube launches (gridsync.cuh)
 float2 *g_small_tiles = nullptr;  // a 64^3 cube's worth, for the signal in tile order
 std::string g_perr;
 
@@ -551,11 +554,10 @@ int uneven_persistent(const UnevenJob *jobs, unsigned njobs, const void *d_sig, 
 void release_uneven_plans() {
   std::lock_guard<std::mutex> lk(g_pmu);
   g_plans.clear();
-  if (g_small_slots) cudaFree(g_small_slots);
+  if (g_small_slot) cudaFree(g_small_slot);
   if (g_small_tiles) cudaFree(g_small_tiles);
-  g_small_slots = nullptr;
+  g_small_slot = nullptr;
   g_small_tiles = nullptr;
-  g_small_next = 0;
 }
 
 // One convolution of an N^3 cube (N = 16, 32 or 64) in one cooperative launch: sig and
@@ -564,21 +566,26 @@ void release_uneven_plans() {
 // cudaErrorNotSupported for other N or when the grid cannot be co-resident.
 cudaError_t launch_small_conv(int n, const float2 *sig, const float2 *filt, float2 *out, float2 *spec, float scale,
                               bool real, const float2 *tw512, unsigned *status, cudaStream_t s) {
-  constexpr int kSlots = 1024;
   if (n != 16 && n != 32 && n != 64) return cudaErrorNotSupported;
   std::lock_guard<std::mutex> lk(g_pmu);
-  cudaError_t e;
-  if (!g_small_slots) {
-    if ((e = cudaMalloc(&g_small_slots, kSlots * sizeof(unsigned))) != cudaSuccess) return e;
-    g_small_next = 0;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &cs);
+  if (e != cudaSuccess) return e;
+  const bool captured = cs != cudaStreamCaptureStatusNone;  // nothing is allocated then
+  // One slot serves all launches, in graphs or not: calls share the workspace and so never run
+  // side by side, and every launch leaves the slot at zero.
+  if (!g_small_slot) {
+    if (captured) return cudaErrorNotSupported;
+    if ((e = cudaMalloc(&g_small_slot, 2 * sizeof(unsigned))) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(g_small_slot, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) {
+      cudaFree(g_small_slot);
+      g_small_slot = nullptr;
+      return e;
+    }
   }
-  if (g_small_next % kSlots == 0) {  // a fresh (or wrapped) ring: every slot back to zero
-    if ((e = cudaMemsetAsync(g_small_slots, 0, kSlots * sizeof(unsigned), s)) != cudaSuccess) return e;
-  }
-  unsigned *slot = g_small_slots + (g_small_next++ % kSlots);
-  if (n > 16) {  // in tiles, with a cube of scratch (not allocated while a graph is captured)
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (!g_small_tiles && cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
+  unsigned *slot = g_small_slot;
+  if (n > 16) {  // in tiles, with a cube of scratch
+    if (!g_small_tiles && !captured) {
       void *p = nullptr;
       if (cudaMalloc(&p, (size_t)64 * 64 * 64 * sizeof(float2)) == cudaSuccess) g_small_tiles = static_cast<float2 *>(p);
       cudaGetLastError();

@@ -844,9 +844,8 @@ __global__ void __launch_bounds__(kTpOneThreads<N>, 1)
       for (int e = 0; e < 16; ++e) stg_unit(tile + nat(e), pswap(v[e]));
     }
     ok = small_grid_barrier(slot, 2u * gridDim.x, status, spin);
-    // the last to pass leaves the counter at zero, for a replay of a captured launch
-    if (ok && threadIdx.x == 0 && atomicAdd(slot, 1u) == 3u * gridDim.x - 1u) atomicExch(slot, 0u);
   }
+  small_grid_leave(slot, ok);
   if constexpr (kTmem) tp_tmem_free<64>(tmem);
   if (!ok || g == 0) return;
 #pragma unroll
