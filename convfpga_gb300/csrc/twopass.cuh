@@ -717,7 +717,8 @@ __global__ void __launch_bounds__(kTpThreads<N>, 1) k_tp_mid(TpArgs a) {
 // A spectrum in natural order -> tile order, for calls that bring their filter's spectrum.
 // Bound by the copy (16 N^3 bytes, or L2 for the small sizes; 4.7 us at N = 64, launch
 // included): a block turns 32 rows (pairs of kz, C of ky) of 32 kx into 32 runs of 16 units,
-// 256 bytes a run on either side.
+// 256 bytes a run on either side. The spectrum may be what the kernel before writes, while this
+// one is resident already, so it is read from L2, after the wait and not as read-only data.
 template <int N>
 __global__ void __launch_bounds__(256) k_tp_order(const float2 *src, float2 *dst) {
   constexpr int J = TpShape<N>::J, C = TpShape<N>::C, R = N / J, H = N / 2, KZ = 16 / C;
@@ -732,7 +733,12 @@ __global__ void __launch_bounds__(256) k_tp_order(const float2 *src, float2 *dst
   tp_grid_wait();
   for (int i = threadIdx.x >> 5; i < 32; i += 8) {
     const int u = i >> 1, kz = 2 * (kz0 + u / C) + (i & 1), ky = g * C + u % C + J * k2;
-    rows[i][lane] = __ldg(src + ((long long)kz * N + ky) * N + x0 + lane);
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];"
+                 : "=f"(v.x), "=f"(v.y)
+                 : "l"(src + ((long long)kz * N + ky) * N + x0 + lane)
+                 : "memory");
+    rows[i][lane] = v;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 512; i += 256) {

@@ -45,3 +45,35 @@ def test_noalloc_with_a_spectrum_beside_other_calls(gpu, n, beside):
     calls[0](n, s, spec[0], s, 1, gpu.FILTER_IS_SPECTRUM | gpu.NORMALIZE, streams[0])
     torch.cuda.synchronize()
     assert float(torch.linalg.vector_norm(s - filt[0]) / torch.linalg.vector_norm(filt[0])) < 1e-6
+
+
+@pytest.mark.parametrize("n,b", [(32, 2), (64, 1), (64, 33), (128, 1), (128, 8), (256, 3)])
+def test_spectrum_written_just_before_it_is_used(gpu, n, b):
+    """filter_spectrum_device, then the convolution with that spectrum, on a new filter each time
+    and with no wait between: as with a wait, bit for bit."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n + b)
+    keep = gpu.plan_variant(n, 4)
+    gpu.plan_variant(n, 4, 3)
+
+    def cubes(k):
+        return torch.view_as_complex(torch.randn((k, n, n, n, 2), generator=gen, device="cuda"))
+
+    sig, filts = cubes(b), cubes(6)
+    spec, flags = torch.empty_like(filts[0]), gpu.FILTER_IS_SPECTRUM | gpu.NORMALIZE
+    outs, want = [torch.empty_like(sig) for _ in filts], torch.empty_like(sig)
+    gpu.device_status()
+    gpu.conv3d_device(n, sig, filts[0], want, b, flags)  # any allocation happens here
+    torch.cuda.synchronize()
+    for f, o in zip(filts, outs):
+        gpu.filter_spectrum_device(n, f, spec, 1)
+        gpu.conv3d_device(n, sig, spec, o, b, flags)
+    torch.cuda.synchronize()
+    for f, o in zip(filts, outs):
+        gpu.filter_spectrum_device(n, f, spec, 1)
+        torch.cuda.synchronize()
+        gpu.conv3d_device(n, sig, spec, want, b, flags)
+        torch.cuda.synchronize()
+        assert torch.equal(o, want)
+    gpu.plan_variant(n, 4, keep)
+    assert gpu.device_status() == 0
