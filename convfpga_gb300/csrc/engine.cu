@@ -628,10 +628,15 @@ static int tc_of(unsigned flags) {
                                                           : 0;
 }
 
+// One small cube (N <= 64, 2 MiB, L2-resident): the whole convolution in one cooperative
+// launch instead of seven launches separated by launch gaps. It keeps the filter as N^3 values
+// in the workspace, real filters too.
+static bool small_one(unsigned n, unsigned how_many, int tc) { return how_many == 1 && tc == 0 && n <= 64; }
+
 static size_t workspace_bytes_for(unsigned n, unsigned how_many, unsigned flags) {
   size_t vol = (size_t)n * n * n * sizeof(float2);
   if (flags & kFlagFilterIsSpectrum) return 0;
-  if (use_half(n, (flags & kFlagFilterReal) != 0, tc_of(flags)))
+  if (use_half(n, (flags & kFlagFilterReal) != 0, tc_of(flags)) && !small_one(n, how_many, tc_of(flags)))
     vol = (size_t)n * n * half_spectrum_pitch((int)n) * sizeof(float2);  // a half spectrum per filter
   if (flags & kFlagPerSignalFilter) return vol * how_many;
   return vol;
@@ -675,9 +680,7 @@ static cudaError_t enqueue_conv_device(unsigned n, const float2 *sig, const floa
     return enqueue_signals(n, sig, out, filt, sv, OP_CONV, how_many, scale, s, nullptr, tc);
   }
   const bool real = (flags & kFlagFilterReal) != 0;
-  // One small cube (N <= 64, 2 MiB, L2-resident): the whole convolution in one cooperative
-  // launch instead of seven launches separated by launch gaps.
-  if (how_many == 1 && tc == 0 && n <= 64) {
+  if (small_one(n, how_many, tc)) {
     const cudaError_t e =
         launch_small_conv((int)n, sig, filt, out, ws, scale, real, g.tw512, device_status_address(), s);
     if (e == cudaSuccess) {
