@@ -166,6 +166,9 @@ void release_xy_l2();
 // prepare_xy_l2 allocates the size's scratch ring and sets the kernel attributes (call it
 // before a capture).
 cudaError_t prepare_xy_l2(int n);
+// Whether the L2-staged pass of size n has its scratch ring and its counters for `nplanes`
+// planes, allocating them unless stream s is captured into a graph.
+bool xy_l2_ready(int n, int nplanes, cudaStream_t s);
 size_t xy_l2_counter_bytes(int n, int ncubes);
 bool encode_xy_table_map(CUtensorMap *m, const void *cube, int n);
 cudaError_t launch_xy_l2_table(int n, const CUtensorMap *rmaps, float2 *const *dsts, int ncubes, bool inverse,

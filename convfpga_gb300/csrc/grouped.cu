@@ -252,10 +252,16 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
       }
       if (apart) return filters_apart(n) ? kXyTiles : kXyTilesOrdered;
     }
-    return n >= 128 && (v == 1 || v == kXyTwoPass) ? kXyStaged : kXySeparate;
+    if (n < 128 || (v != 1 && v != kXyTwoPass)) return kXySeparate;
+    if (v == kXyTwoPass && prepare_xy_l2(n) != cudaSuccess) {  // no memory for its ring
+      cudaGetLastError();
+      return kXySeparate;
+    }
+    return kXyStaged;
   };
   Forms forms;
-  for (int n : {32, 64, 128, 256}) forms.of[Forms::index(n)] = form(n);
+  for (int n : {32, 64, 128, 256})
+    if (std::find(sizes.begin(), sizes.end(), n) != sizes.end()) forms.of[Forms::index(n)] = form(n);
   // 16^3 jobs run whole, in any order
   forms.of[0] = filters_apart(16) ? kWhole : kXySeparate;
   int form_key = 0;

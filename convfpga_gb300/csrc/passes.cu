@@ -411,7 +411,12 @@ cudaError_t launch_axis_pass_tc(int n, int axis, int op, const float2 *src, floa
 cudaError_t launch_xy_pass(int n, const float2 *src, float2 *dst, int nplanes, bool inverse, float scale,
                            const float2 *tw512, cudaStream_t s, int variant) {
   if (!g_use_tma) return cudaErrorNotSupported;
-  if (variant == kXyTwoPass) variant = 1;  // a call the two-pass transform does not take
+  if (variant == kXyTwoPass) {
+    // A call the two-pass transform does not take: the staged pass, unless it would have to
+    // allocate while a graph is captured, or cannot (the separate passes need no scratch).
+    if ((n != 128 && n != 256) || !xy_l2_ready(n, nplanes, s)) return cudaErrorNotSupported;
+    variant = 1;
+  }
   if (n == 128 || n == 512)
     return variant == 1 ? launch_xy_l2(n, src, dst, nplanes, inverse, scale, tw512, device_status_address(), s)
                         : cudaErrorNotSupported;

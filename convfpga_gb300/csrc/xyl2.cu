@@ -91,6 +91,19 @@ cudaError_t prepare_xy_l2(int n) {
   return cudaErrorInvalidValue;
 }
 
+bool xy_l2_ready(int n, int nplanes, cudaStream_t s) {
+  const size_t plane = (size_t)n * n * sizeof(float2), counters = (2ull * nplanes + 2) * sizeof(unsigned);
+  const size_t ring = plane * (n == 256 ? XyL2Cfg<256>::RING : (n == 128 ? XyL2Cfg<128>::RING : XyL2Cfg<512>::RING));
+  Scratch &r = g_ring[n == 256 ? 0 : (n == 128 ? 1 : 2)];
+  if (r.bytes >= ring && g_ctr.bytes >= counters) return true;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+      r.ensure(ring) == cudaSuccess && g_ctr.ensure(std::max<size_t>(counters, 64 << 10)) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
+}
+
 size_t xy_l2_counter_bytes(int n, int ncubes) { return (2ull * n * ncubes + 2) * sizeof(unsigned); }
 
 // The source rows map of the pass (box {N, C}).

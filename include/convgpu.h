@@ -58,7 +58,8 @@ extern "C" {
  * Calls of N = 32 to 256 on the FP32 path also hold scratch cubes (128, 256, 512 and 512 MiB),
  * allocated by the first such call and kept until fpga_final; without them (no memory) the
  * calls run the passes of the other plan variants. A call captured into a graph allocates
- * none, so make one call of its size before the capture.
+ * none of them, so make one call of its size before the capture. (A call with a given spectrum
+ * needs no workspace either and can be the first of its size; it then runs separate passes.)
  * d_sig may equal d_out (in place). The library's per-device workspace is shared by
  * all calls: calls on different streams must not overlap. */
 int convgpu_conv3d_device(unsigned N, const float2 *d_sig, const float2 *d_filter, float2 *d_out,
