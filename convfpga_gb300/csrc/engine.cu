@@ -79,6 +79,12 @@ static std::atomic<unsigned> g_fail_allocs{0};
 
 void fail_next_allocations(unsigned count) { g_fail_allocs.store(count); }
 
+bool allocation_fails_on_purpose() {
+  for (unsigned f = g_fail_allocs.load(); f > 0;)
+    if (g_fail_allocs.compare_exchange_weak(f, f - 1)) return true;
+  return false;
+}
+
 // Grow-only device buffer. Growing synchronises the device first, so work still in
 // flight on the old block never sees it freed.
 struct DevBuf {
@@ -92,8 +98,7 @@ struct DevBuf {
       p = nullptr;
       bytes = 0;
     }
-    for (unsigned f = g_fail_allocs.load(); f > 0;)
-      if (g_fail_allocs.compare_exchange_weak(f, f - 1)) return cudaErrorMemoryAllocation;
+    if (allocation_fails_on_purpose()) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc(&p, b);
     if (e == cudaSuccess) bytes = b;
     return e;

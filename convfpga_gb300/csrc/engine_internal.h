@@ -210,5 +210,8 @@ int conv_device_noalloc(unsigned n, const void *d_sig, const void *d_filt, void 
 
 // Counts kernel launches issued by this library (host-side, monotonic).
 void count_launches(unsigned long long k);
+// Testing hook: whether an allocation of device buffers is to fail on purpose; takes one of
+// those still to fail.
+bool allocation_fails_on_purpose();
 
 }  // namespace convgpu

@@ -438,6 +438,7 @@ std::mutex g_pmu;
 std::map<std::vector<int>, std::unique_ptr<PPlan>> g_plans;
 unsigned *g_small_slot = nullptr;  // barrier words of the small-cube launches (gridsync.cuh)
 float2 *g_small_tiles = nullptr;  // a 64^3 cube's worth, for the signal in tile order
+bool g_small_none = false;        // it could not be allocated
 std::string g_perr;
 
 cudaError_t build_plan(PPlan &p, const float2 *tw512, unsigned *status) {
@@ -558,6 +559,7 @@ void release_uneven_plans() {
   if (g_small_tiles) cudaFree(g_small_tiles);
   g_small_slot = nullptr;
   g_small_tiles = nullptr;
+  g_small_none = false;
 }
 
 // One convolution of an N^3 cube (N = 16, 32 or 64) in one cooperative launch: sig and
@@ -585,10 +587,14 @@ cudaError_t launch_small_conv(int n, const float2 *sig, const float2 *filt, floa
   }
   unsigned *slot = g_small_slot;
   if (n > 16) {  // in tiles, with a cube of scratch
-    if (!g_small_tiles && !captured) {
+    if (!g_small_tiles && !g_small_none && !captured) {
       void *p = nullptr;
-      if (cudaMalloc(&p, (size_t)64 * 64 * 64 * sizeof(float2)) == cudaSuccess) g_small_tiles = static_cast<float2 *>(p);
-      cudaGetLastError();
+      if (!allocation_fails_on_purpose() && cudaMalloc(&p, (size_t)64 * 64 * 64 * sizeof(float2)) == cudaSuccess) {
+        g_small_tiles = static_cast<float2 *>(p);
+      } else {
+        cudaGetLastError();
+        g_small_none = true;
+      }
     }
     if (g_small_tiles) {
       e = launch_tp_one(n, sig, filt, out, spec, g_small_tiles, scale, real, tw512, slot, status, s);

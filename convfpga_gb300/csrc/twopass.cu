@@ -94,7 +94,12 @@ TpArgs args(int n, const void *src, void *dst, int nvol, const float2 *tw512) {
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-float2 *g_scratch[4] = {};  // N = 32, 64, 128, 256
+// N = 32, 64, 128, 256. One that could not be allocated is not asked for again, call by call,
+// before release_tp.
+struct TpScratch {
+  float2 *p = nullptr;
+  bool none = false;
+} g_scratch[4];
 
 // Calls f with N as a compile-time constant.
 template <class F>
@@ -116,21 +121,24 @@ int tp_scratch_cubes(int n) {
 }
 
 float2 *tp_scratch(int n, bool may_allocate) {
-  float2 *&p = g_scratch[n == 32 ? 0 : (n == 64 ? 1 : (n == 128 ? 2 : 3))];
-  if (!p && may_allocate) {
+  TpScratch &t = g_scratch[n == 32 ? 0 : (n == 64 ? 1 : (n == 128 ? 2 : 3))];
+  if (!t.p && !t.none && may_allocate) {
     void *q = nullptr;
-    if (cudaMalloc(&q, (size_t)tp_scratch_cubes(n) * n * n * n * sizeof(float2)) == cudaSuccess)
-      p = static_cast<float2 *>(q);
-    else
+    if (!allocation_fails_on_purpose() &&
+        cudaMalloc(&q, (size_t)tp_scratch_cubes(n) * n * n * n * sizeof(float2)) == cudaSuccess) {
+      t.p = static_cast<float2 *>(q);
+    } else {
       cudaGetLastError();
+      t.none = true;
+    }
   }
-  return p;
+  return t.p;
 }
 
 void release_tp() {
-  for (auto &p : g_scratch) {
-    if (p) cudaFree(p);
-    p = nullptr;
+  for (auto &t : g_scratch) {
+    if (t.p) cudaFree(t.p);
+    t = TpScratch{};
   }
 }
 

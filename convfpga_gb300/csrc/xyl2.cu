@@ -3,6 +3,7 @@
 // (grow-only, per process), counters cleared on the stream before every launch, one
 // persistent grid of as many CTAs as fit.
 #define CONVGPU_PASS_LAUNCH_IMPL
+#include "engine_internal.h"
 #include "pass_launch.cuh"
 #include "xy512.cuh"
 #include "xyl2.cuh"
@@ -28,6 +29,7 @@ struct Scratch {
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
+    if (allocation_fails_on_purpose()) return cudaErrorMemoryAllocation;
     const cudaError_t e = cudaMalloc(&p, want);
     if (e == cudaSuccess) bytes = want;
     return e;
@@ -39,9 +41,11 @@ struct Scratch {
   }
 };
 Scratch g_ring[3], g_ctr;  // scratch rings of N = 256, 128 and 512; the process's counters
+bool g_ring_none = false;  // xy_l2_ready could not allocate
 }  // namespace
 
 void release_xy_l2() {
+  g_ring_none = false;
   for (auto &r : g_ring) r.release();
   g_ctr.release();
 }
@@ -97,10 +101,13 @@ bool xy_l2_ready(int n, int nplanes, cudaStream_t s) {
   Scratch &r = g_ring[n == 256 ? 0 : (n == 128 ? 1 : 2)];
   if (r.bytes >= ring && g_ctr.bytes >= counters) return true;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
-      r.ensure(ring) == cudaSuccess && g_ctr.ensure(std::max<size_t>(counters, 64 << 10)) == cudaSuccess)
-    return true;
+  if (g_ring_none || cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  if (r.ensure(ring) == cudaSuccess && g_ctr.ensure(std::max<size_t>(counters, 64 << 10)) == cudaSuccess) return true;
   cudaGetLastError();
+  g_ring_none = true;  // not asked for again, call by call, before release_xy_l2
   return false;
 }
 

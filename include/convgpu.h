@@ -209,10 +209,11 @@ int convgpu_device_status(unsigned *status);
  * Waits for the device before it changes the limit; graphs captured earlier read the new
  * limit when they run.
  *
- * convgpu_debug_fail_allocations: the next `count` allocations of the library's
- * grow-only device buffers (workspace, host-pipeline staging) fail as out of memory; the
- * call that meets one returns CONVGPU_ENOMEM or an fpga_t with valid == 0, and later
- * calls allocate again. */
+ * convgpu_debug_fail_allocations: the next `count` allocations of the library's device
+ * buffers (workspace, host-pipeline staging, scratch) fail as out of memory; the call that
+ * meets one returns CONVGPU_ENOMEM or an fpga_t with valid == 0, and later calls allocate
+ * again. A call that can do without the buffer (scratch cubes, the staged pass's ring when
+ * it is not named in the plan) does, and so do later ones until fpga_final. */
 int convgpu_debug_dependency_wait_limit(int probes);
 int convgpu_debug_fail_allocations(unsigned count);
 
