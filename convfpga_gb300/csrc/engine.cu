@@ -559,7 +559,7 @@ static cudaError_t enqueue_tp(int n, const float2 *sig, const float2 *filt, floa
   if (overlap && su != ou) return cudaErrorNotSupported;
   const bool pairs = per_signal || how_many == 1;  // every filter serves one signal
   const bool direct = pairs && !overlap;
-  float2 *scratch = tp_scratch(n, !capturing(s));
+  float2 *scratch = direct ? nullptr : tp_scratch(n, !capturing(s));
   if (!direct && !scratch) return cudaErrorNotSupported;
   // Filters are read before any output is written: a caller may convolve into them.
   const uintptr_t fbytes = (uintptr_t)V * (per_signal ? how_many : 1) * (real ? 4 : 8);

@@ -124,3 +124,21 @@ def test_uneven_in_place_without_the_ring(fresh, n):
     torch.cuda.synchronize()
     assert cg.device_status() == 0
     assert rel_l2(conv3d(sig[None], f, "fp64", normalize=True, engine="pocketfft")[0], s.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("n,b", [(32, 3), (64, 2), (128, 2), (256, 1)])
+def test_calls_that_need_no_scratch_ask_for_none(fresh, n, b):
+    """A filter per signal, outputs apart: the failure waits for the first call in place."""
+    cg, rng = fresh, np.random.default_rng(n)
+    sig, f = _c64(rng, (b, n, n, n)), _c64(rng, (b, n, n, n))
+    s, d = torch.from_numpy(sig).cuda(), torch.from_numpy(f).cuda()
+    o = torch.empty_like(s)
+    cg.plan_variant(n, XY, 0)
+    cg.conv3d_device(n, s, d, o, b, cg.FILTER_PER_SIGNAL)  # allocates the workspace
+    torch.cuda.synchronize()
+    cg.plan_variant(n, XY, 3)
+    cg.debug_fail_allocations(2 if n >= 128 else 1)
+    assert _launches(cg, lambda: cg.conv3d_device(n, s, d, o, b, cg.FILTER_PER_SIGNAL)) == 3
+    assert rel_l2(conv3d(sig[:1], f[0], "fp64", engine="pocketfft")[0], o[0].cpu().numpy()) < 1e-6
+    assert _launches(cg, lambda: cg.conv3d_device(n, s, d, s, b, cg.FILTER_PER_SIGNAL)) > 3
+    assert rel_l2(conv3d(sig[:1], f[0], "fp64", engine="pocketfft")[0], s[0].cpu().numpy()) < 1e-6
