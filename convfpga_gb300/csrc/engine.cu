@@ -79,6 +79,15 @@ static std::atomic<unsigned> g_fail_allocs{0};
 
 void fail_next_allocations(unsigned count) { g_fail_allocs.store(count); }
 
+cudaError_t allocate(void **p, size_t bytes) {
+  auto once = [&] { return allocation_fails_on_purpose() ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes); };
+  cudaError_t e = once();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  if (give_back_tp()) e = once();
+  return e;
+}
+
 bool allocation_fails_on_purpose() {
   for (unsigned f = g_fail_allocs.load(); f > 0;)
     if (g_fail_allocs.compare_exchange_weak(f, f - 1)) return true;
@@ -98,8 +107,7 @@ struct DevBuf {
       p = nullptr;
       bytes = 0;
     }
-    if (allocation_fails_on_purpose()) return cudaErrorMemoryAllocation;
-    cudaError_t e = cudaMalloc(&p, b);
+    const cudaError_t e = allocate(&p, b);
     if (e == cudaSuccess) bytes = b;
     return e;
   }

@@ -116,6 +116,8 @@ cudaError_t launch_tp_inv_table(int n, const CUtensorMap *src_maps, float2 *cons
 constexpr int kTpScratchCubes32 = 512, kTpScratchCubes64 = 128, kTpScratchCubes128 = 32, kTpScratchCubes256 = 4;
 int tp_scratch_cubes(int n);
 float2 *tp_scratch(int n, bool may_allocate);
+// Frees the scratch cubes that no captured call holds; later calls do without. False if none.
+bool give_back_tp();
 void release_tp();
 // Convolutions of 16^3 cubes in one launch, one CTA per cube (cube16.cu): filt holds one filter
 // (N^3 floats with `real`) for all or, with per_signal, one per cube, or spectra. A cube's
@@ -213,5 +215,8 @@ void count_launches(unsigned long long k);
 // Testing hook: whether an allocation of device buffers is to fail on purpose; takes one of
 // those still to fail.
 bool allocation_fails_on_purpose();
+// cudaMalloc of a buffer that a call cannot do without: when memory is short, the two-pass
+// transform's scratch cubes, which it can, make room.
+cudaError_t allocate(void **p, size_t bytes);
 
 }  // namespace convgpu

@@ -149,7 +149,7 @@ cudaError_t build(GPlan &p, bool normalize, const Forms &forms, const float2 *tw
     spec += (size_t)p.sizes[j] * p.sizes[j] * p.sizes[j];
   }
   cudaError_t e;
-  if ((e = cudaMalloc(&p.d_spec, spec * sizeof(float2))) != cudaSuccess) return e;
+  if ((e = allocate((void **)&p.d_spec, spec * sizeof(float2))) != cudaSuccess) return e;
   for (auto &g : p.groups) {
     const size_t k = g.jobs.size();
     g.h_maps.resize(kKinds * k);

@@ -465,7 +465,7 @@ cudaError_t build_plan(PPlan &p, const float2 *tw512, unsigned *status) {
   if ((e = cudaMalloc(&p.d_jobs, sizeof(UJob) * nj)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&p.d_items, sizeof(uint32_t) * items.size())) != cudaSuccess) return e;
   if ((e = cudaMalloc(&p.d_counters, sizeof(int) * (nj * kPasses + 1))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&p.d_spec, sizeof(float2) * p.spec_elems)) != cudaSuccess) return e;
+  if ((e = allocate((void **)&p.d_spec, sizeof(float2) * p.spec_elems)) != cudaSuccess) return e;
   if ((e = cudaMemcpy(p.d_items, items.data(), sizeof(uint32_t) * items.size(), cudaMemcpyHostToDevice)) !=
       cudaSuccess)
     return e;

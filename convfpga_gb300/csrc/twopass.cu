@@ -98,7 +98,8 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 // before release_tp.
 struct TpScratch {
   float2 *p = nullptr;
-  bool none = false;
+  bool none = false;      // not to be had, or given back
+  bool captured = false;  // a graph may hold it
 } g_scratch[4];
 
 // Calls f with N as a compile-time constant.
@@ -132,7 +133,21 @@ float2 *tp_scratch(int n, bool may_allocate) {
       t.none = true;
     }
   }
+  t.captured |= t.p && !may_allocate;
   return t.p;
+}
+
+bool give_back_tp() {
+  bool any = false;
+  for (auto &t : g_scratch) {
+    if (!t.p || t.captured) continue;
+    if (!any) cudaDeviceSynchronize();
+    any = true;
+    cudaFree(t.p);
+    t.p = nullptr;
+    t.none = true;
+  }
+  return any;
 }
 
 void release_tp() {

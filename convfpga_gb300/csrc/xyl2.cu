@@ -29,8 +29,7 @@ struct Scratch {
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
-    if (allocation_fails_on_purpose()) return cudaErrorMemoryAllocation;
-    const cudaError_t e = cudaMalloc(&p, want);
+    const cudaError_t e = allocate(&p, want);
     if (e == cudaSuccess) bytes = want;
     return e;
   }

@@ -57,8 +57,9 @@ extern "C" {
  * filters only; its real Gaussian filters are stored with zero imaginary parts.
  * Calls of N = 32 to 256 on the FP32 path also hold scratch cubes (128, 256, 512 and 512 MiB),
  * unless every filter serves one signal and the outputs are apart from the signals. They are
- * allocated by the first such call and kept until fpga_final; without them (no memory) the
- * calls run the passes of the other plan variants. A call captured into a graph allocates
+ * allocated by the first such call and kept until fpga_final, or until a buffer that a call
+ * cannot do without finds no other memory (and no captured call holds them); without them
+ * the calls run the passes of the other plan variants. A call captured into a graph allocates
  * none of them, so make one call of its size before the capture. (A call with a given spectrum
  * needs no workspace either and can be the first of its size; it then runs separate passes.)
  * d_sig may equal d_out (in place). The library's per-device workspace is shared by

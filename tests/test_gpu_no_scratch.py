@@ -142,3 +142,42 @@ def test_calls_that_need_no_scratch_ask_for_none(fresh, n, b):
     assert rel_l2(conv3d(sig[:1], f[0], "fp64", engine="pocketfft")[0], o[0].cpu().numpy()) < 1e-6
     assert _launches(cg, lambda: cg.conv3d_device(n, s, d, s, b, cg.FILTER_PER_SIGNAL)) > 3
     assert rel_l2(conv3d(sig[:1], f[0], "fp64", engine="pocketfft")[0], s[0].cpu().numpy()) < 1e-6
+
+
+def test_scratch_makes_room_for_what_a_call_needs(fresh):
+    """A workspace that finds no memory takes that of the scratch cubes; later calls do without
+    them. Scratch cubes that a captured call holds stay."""
+    cg, n = fresh, 128
+    rng = np.random.default_rng(n)
+    sig, f = _c64(rng, (5, n, n, n)), _c64(rng, (5, n, n, n))
+    s, d = torch.from_numpy(sig).cuda(), torch.from_numpy(f).cuda()
+    o = torch.empty_like(s)
+
+    def shared(stream=None):
+        cg.conv3d_device(n, s, d, o, 3, 0, stream)  # through the scratch cubes; one filter of workspace
+
+    def check(i, fi):
+        assert rel_l2(conv3d(sig[i:i + 1], f[fi], "fp64", engine="pocketfft")[0], o[i].cpu().numpy()) < 1e-6
+
+    assert _launches(cg, shared) == 3
+    check(2, 0)
+    cg.debug_fail_allocations(1)
+    cg.conv3d_device(n, s, d, o, 5, cg.FILTER_PER_SIGNAL)  # five filters of workspace
+    torch.cuda.synchronize()
+    check(4, 4)
+    assert _launches(cg, shared) > 3
+    check(2, 0)
+    _renew(cg)
+    assert _launches(cg, shared) == 3
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        shared(torch.cuda.current_stream())
+    o.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    check(2, 0)
+    cg.debug_fail_allocations(1)
+    with pytest.raises(cg.ConvGpuError):
+        cg.conv3d_device(n, s, d, o, 5, cg.FILTER_PER_SIGNAL)
+    assert _launches(cg, shared) == 3
+    check(2, 0)
