@@ -14,6 +14,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "engine_internal.h"
 #include "herm.cuh"
 #include "passes.cuh"
 #include "pairs512.cuh"
@@ -160,6 +161,7 @@ static cudaError_t launch_zpair(const PassReq &r) {
   unsigned *claims = zpair_claims();
   if (!claims) return cudaErrorNotSupported;
   k_zpair_clear<<<1, 1, 0, r.s>>>(claims);
+  count_launches(1);  // besides the pass, which the caller counts
   kern<<<blocks, S::NT * S::G, S::kSmem, r.s>>>(ms, mf, r.a, r.nvol, claims);
   return cudaGetLastError();
 }

@@ -3,7 +3,6 @@
 // (grow-only, per process), counters cleared on the stream before every launch, one
 // persistent grid of as many CTAs as fit.
 #define CONVGPU_PASS_LAUNCH_IMPL
-#include "engine_internal.h"
 #include "pass_launch.cuh"
 #include "xy512.cuh"
 #include "xyl2.cuh"
