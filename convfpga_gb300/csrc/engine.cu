@@ -1598,9 +1598,13 @@ int bridge_autotune(const unsigned *sizes, unsigned count, int write_cache) {
       const int axis = k == kKindRows ? 0 : (k == kKindStrided ? 1 : 2);
       const int op = k == kKindConv ? OP_CONV : (k == kKindConvFz ? OP_CONV_FZ : OP_FWD);
       const long long fv = k == kKindConvFz ? (long long)V : 0;
-      for (int v = 0; v < 2 && err == cudaSuccess; ++v) {
+      // N = 512: the fused z pass is one kernel in every ordered call (pairs512.cuh). Kind 2 chooses
+      // for the calls that are not, which bring spectra; kind 3 has nothing to choose.
+      const bool unordered = n == 512 && k == kKindConv;
+      const int forms = n == 512 && k == kKindConvFz ? 1 : 2;
+      for (int v = 0; v < forms && err == cudaSuccess; ++v) {
         auto run = [&]() {
-          return launch_axis_pass_variant(n, axis, op, data, data, spec, fv, nvol, 1.f, g.tw512, s, v);
+          return launch_axis_pass_variant(n, axis, op, data, data, spec, fv, nvol, 1.f, g.tw512, s, v, unordered);
         };
         for (int w = 0; w < 2 && err == cudaSuccess; ++w) err = run();
         cudaEventRecord(e0, s);
@@ -1612,7 +1616,7 @@ int bridge_autotune(const unsigned *sizes, unsigned count, int write_cache) {
         row.us[v][k] = 1000.0 * ms / 5.0;
         count_launches(7);
       }
-      row.choice[k] = row.us[1][k] < row.us[0][k] ? 1 : 0;
+      row.choice[k] = forms == 2 && row.us[1][k] < row.us[0][k] ? 1 : 0;
       set_pass_variant(n, k, row.choice[k]);
     }
     g_tuned.erase(std::remove_if(g_tuned.begin(), g_tuned.end(), [&](const TuneRow &t) { return t.n == n; }),

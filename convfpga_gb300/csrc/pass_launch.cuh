@@ -166,20 +166,12 @@ static cudaError_t launch_zpair(const PassReq &r) {
   return cudaGetLastError();
 }
 
-// TMA y / z pass. Returns cudaErrorNotSupported when a tensor map cannot be built.
+// k_strided_tma. Returns cudaErrorNotSupported when a tensor map cannot be built.
 template <int N, int V, int OP>
-static cudaError_t launch_strided(const PassReq &r) {
+static cudaError_t launch_strided_tma(const PassReq &r) {
   using S = Shape<N, V>;
   constexpr int E = S::E, COLS = S::SC;
   constexpr bool HAS_F = (OP == OP_CONV || OP == OP_CONV_FZ);
-  // The tiles of k_zpair are claimed from one counter of the device. A launch that others may run
-  // beside keeps to k_strided_tma, which shares nothing: a no-allocation call of one 512^3 cube
-  // takes 2,180 us so, and 2,239 with k_zpair on fixed shares of the tiles.
-  if constexpr (N == 512 && HAS_F)
-    if (r.mode != kModeTable && r.axis == 2 && !r.unordered) {
-      if ((reinterpret_cast<uintptr_t>(r.a.dst) & 15u) != 0) return cudaErrorNotSupported;
-      return launch_zpair<false, OP == OP_CONV_FZ>(r);
-    }
   constexpr int smem = tma_pass_smem_bytes<N, COLS, OP>();
   auto kern = k_strided_tma<N, E, COLS, OP, typename S::Plan>;
   static int done = 0;
@@ -207,6 +199,28 @@ static cudaError_t launch_strided(const PassReq &r) {
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   kern<<<(unsigned)blocks, COLS * (N / E), smem, r.s>>>(msrc, mfilt, a, r.axis);
   return cudaGetLastError();
+}
+
+// Shapes of k_strided_tma that no call reaches: at N = 512 the filter's z transform is fused in
+// k_zpair's calls and in table mode (variant 0), while unordered calls bring spectra.
+template <int N, int V, int OP>
+constexpr bool kNoStrided = N == 512 && V == 1 && OP == OP_CONV_FZ;
+
+// TMA y / z pass. Returns cudaErrorNotSupported when a tensor map cannot be built.
+template <int N, int V, int OP>
+static cudaError_t launch_strided(const PassReq &r) {
+  // The tiles of k_zpair are claimed from one counter of the device. A launch that others may run
+  // beside keeps to k_strided_tma, which shares nothing: a no-allocation call of one 512^3 cube
+  // takes 2,180 us so, and 2,239 with k_zpair on fixed shares of the tiles.
+  if constexpr (N == 512 && (OP == OP_CONV || OP == OP_CONV_FZ))
+    if (r.mode != kModeTable && r.axis == 2 && !r.unordered) {
+      if ((reinterpret_cast<uintptr_t>(r.a.dst) & 15u) != 0) return cudaErrorNotSupported;
+      return launch_zpair<false, OP == OP_CONV_FZ>(r);
+    }
+  if constexpr (kNoStrided<N, V, OP>)
+    return cudaErrorNotSupported;
+  else
+    return launch_strided_tma<N, V, OP>(r);
 }
 
 template <int N, int V>
@@ -358,7 +372,8 @@ static cudaError_t prepare_variant() {
   set(k_strided_tma<N, E, COLS, OP_FWD, typename S::Plan>, tma_pass_smem_bytes<N, COLS, OP_FWD>());
   set(k_strided_tma<N, E, COLS, OP_INV, typename S::Plan>, tma_pass_smem_bytes<N, COLS, OP_INV>());
   set(k_strided_tma<N, E, COLS, OP_CONV, typename S::Plan>, tma_pass_smem_bytes<N, COLS, OP_CONV>());
-  set(k_strided_tma<N, E, COLS, OP_CONV_FZ, typename S::Plan>, tma_pass_smem_bytes<N, COLS, OP_CONV_FZ>());
+  if constexpr (!kNoStrided<N, V, OP_CONV_FZ>)
+    set(k_strided_tma<N, E, COLS, OP_CONV_FZ, typename S::Plan>, tma_pass_smem_bytes<N, COLS, OP_CONV_FZ>());
   return e;
 }
 

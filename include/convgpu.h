@@ -170,7 +170,9 @@ int convgpu_synchronize(void);
 int convgpu_autotune(const unsigned *sizes, unsigned count, int write_cache);
 
 /* Plan-table entry of cube size N for pass kind (0 x pass, 1 y/z passes, 2 fused z pass,
- * 3 fused z pass with the filter's z transform, 4 x and y: 0 separate passes; N = 256:
+ * 3 fused z pass with the filter's z transform (N = 512: 2 chooses for
+ * convgpu_conv3d_device_noalloc alone and 3 nothing, since the other calls have one kernel);
+ * 4 x and y: 0 separate passes; N = 256:
  * 1 one pass staged through an L2-resident scratch ring, 2 one pass on 8-CTA clusters;
  * N = 128 and 512: 1 one pass staged through an L2-resident scratch ring; N = 32 to 256, the
  * default there: 3 the two-pass 3D transform, for calls whose cubes are 16-byte aligned and
