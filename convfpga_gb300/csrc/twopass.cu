@@ -27,7 +27,9 @@ cudaError_t launch_blocks(K kern, int smem, int threads, long long blocks, cudaS
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch's check
+  return e;
 }
 
 // Persistent: one CTA per SM at most.
