@@ -413,8 +413,15 @@ cudaError_t launch_xy_pass(int n, const float2 *src, float2 *dst, int nplanes, b
   if (!g_use_tma) return cudaErrorNotSupported;
   if (variant == kXyTwoPass) {
     // A call the two-pass transform does not take: the staged pass, unless it would have to
-    // allocate while a graph is captured, or cannot (the separate passes need no scratch).
-    if ((n != 128 && n != 256) || !xy_l2_ready(n, nplanes, s)) return cudaErrorNotSupported;
+    // allocate while a graph is captured, or cannot (the separate passes need no scratch), or
+    // the cubes stay in L2 between separate passes. us, staged / separate, with the autotuned
+    // shapes and with the default ones: spectra of 128^3 x2 39.2 / 33.2 and 39.2 / 36.6, x5
+    // 77.2 / 75.9 and 78.7 / 77.5, x6 92.7 / 96.6 and 93.0 / 98.0, x8 118.5 / 132.1 and 118.9 /
+    // 132.6; signals with a spectrum each x5 143.8 / 141.2 and 145.1 / 145.7, x6 166.0 / 181.1 and
+    // 167.7 / 182.5; spectra of 256^3 x1 120.8 / 128.9 and 119.0 / 127.7.
+    constexpr int kSeparate128 = 5 * 128;
+    if (n == 128 ? nplanes <= kSeparate128 : n != 256) return cudaErrorNotSupported;
+    if (!xy_l2_ready(n, nplanes, s)) return cudaErrorNotSupported;
     variant = 1;
   }
   if (n == 128 || n == 512)

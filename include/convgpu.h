@@ -177,7 +177,7 @@ int convgpu_autotune(const unsigned *sizes, unsigned count, int write_cache);
  * N = 128 and 512: 1 one pass staged through an L2-resident scratch ring; N = 32 to 256, the
  * default there: 3 the two-pass 3D transform, for calls whose cubes are 16-byte aligned and
  * whose outputs are the signals or do not overlap them, and for spectra given by the caller
- * where it is faster (other calls run 1 at N = 128 and 256, else 0);
+ * where it is faster (other calls run 1 at N = 256 and, from six cubes, 128, else 0);
  * 5 tensor-core kernels of CONVGPU_TENSOR_SPLIT, N = 256: 0 tcgen05 (TMEM accumulators),
  * 1 mma.sync; 6 x and y passes of the tcgen05 split path, N = 256: 0 separate passes, 1 one
  * pass staged through the L2-resident scratch ring; 7 spectra of real filters
