@@ -546,8 +546,9 @@ static cudaError_t tp_order(int n, const float2 *src, float2 *dst, cudaStream_t 
 // A shared filter's second pass runs inside every signal's middle pass (TP_PAIR) for small
 // batches, and otherwise once before them (TP_FWD, then TP_SPECTRUM): a quarter of the middle
 // pass's work for every cube against one more launch and the filter's own tiles. Measured, us,
-// inside / once: 32^3 x17 22.0 / 24.6, x100 63.4 / 64.5, x300 128.3 / 125.1; 64^3 x8 38.8 /
-// 41.1, x17 64.8 / 64.7, x100 253.7 / 239.2; 128^3 x4 106.1 / 104.3; 256^3 x3 582.5 / 584.0.
+// inside / once: 32^3 x17 21.8 / 25.0, x100 66.3 / 68.7, x300 130.3 / 130.7; 64^3 x8 39.7 /
+// 41.8, x17 64.6 / 65.1, x33 100.3 / 98.4, x100 249.7 / 237.7; 128^3 x4 104.1 / 105.9, x8 174.9 /
+// 172.7; 256^3 x3 528 / 544, x4 677 / 683.
 constexpr unsigned kTpSharedPairCubes = 3;
 constexpr long long kTpSharedPairPoints = 1ll << 22;
 
@@ -609,16 +610,27 @@ static bool apart(const void *a, size_t an, const void *b, size_t bn) {
 // cudaErrorNotSupported, with nothing enqueued, as enqueue_tp, and for batches that the
 // three-axis passes (five launches, no reordering) take faster: between 2^21 and 2^23 points
 // those run out of L2 and the tiles make less than two rounds of the SMs, and one large cube
-// does not make up for the reordering. us, tiles / three axes: 32^3 x1 16.0 / 20.7, x17 23.0 /
-// 26.8, x100 67.4 / 61.3, x300 132 / 137; 64^3 x1 18.1 / 22.7, x8 37.5 / 42.8, x17 63.2 / 60.5,
-// x33 98 / 110; 128^3 x1 42.5 / 43.1, x2 63.3 / 60.8, x4 100 / 108, x8 166 / 200; 256^3 x1
-// 227 / 219, x2 365 / 404, x4 683 / 769.
+// does not make up for the reordering. At N = 32 the line is earlier, where the tiles of an SM
+// go from nine to ten, and later at the other end. us, tiles / three axes with the autotuned
+// shapes: 64^3 x1 17.7 / 22.6, x8 37.8 / 43.1, x12 52.2 / 49.3, x17 63.2 / 61.9, x20 71.4 / 72.0,
+// x24 79.0 / 82.0, x31 95.3 / 101.1, x33 97.9 / 107.5; 128^3 x1 42.5 / 43.2, x2 63.1 / 62.7, x3
+// 82.1 / 84.6, x4 100.4 / 109.4; 256^3 x1 226.6 / 217.5, x2 367 / 405, x4 683 / 773. At N = 32,
+// with the default shapes after them: x1 15.9 / 20.5, x40 34.4 / 36.9 / 36.9, x46 36.1 / 36.9 /
+// 36.9, x48 39.0 / 36.9 / 36.9, x57 42.5 / 42.9 / 39.0, x64 46.0 / 47.1 / 43.8, x100 66.5 / 58.6 /
+// 57.2, x256 119.1 / 120.7 / 116.1 (in place 118.3 / 116.0 / 110.4), x300 131.3 / 137.2 / 132.6,
+// x400 164.2 / 189.6 / 185.2. (Between 20 and 31 cubes of 64^3 the tiles are the faster form too.)
 constexpr long long kTpSpectrumSmall = 1ll << 21, kTpSpectrumLarge = 1ll << 23;
+constexpr long long kTpSpectrumSmall32 = 47ll << 15, kTpSpectrumLarge32 = 300ll << 15;
+static bool tp_spectrum_faster(int n, unsigned how_many) {
+  const long long points = (long long)n * n * n * how_many;
+  return points <= (n == 32 ? kTpSpectrumSmall32 : kTpSpectrumSmall) ||
+         (how_many >= 2 && points >= (n == 32 ? kTpSpectrumLarge32 : kTpSpectrumLarge));
+}
 static cudaError_t enqueue_tp_spectrum(int n, const float2 *sig, const float2 *spec, float2 *out, unsigned how_many,
                                        float scale, cudaStream_t s) {
   const long long V = (long long)n * n * n;
   const size_t bytes = (size_t)V * how_many * sizeof(float2);
-  if (V * how_many > kTpSpectrumSmall && (how_many < 2 || V * how_many < kTpSpectrumLarge)) return cudaErrorNotSupported;
+  if (!tp_spectrum_faster(n, how_many)) return cudaErrorNotSupported;
   if ((reinterpret_cast<uintptr_t>(sig) | reinterpret_cast<uintptr_t>(out)) & 15u) return cudaErrorNotSupported;
   if (sig != out && !apart(sig, bytes, out, bytes)) return cudaErrorNotSupported;
   float2 *scratch = tp_scratch(n, !capturing(s));
