@@ -178,19 +178,19 @@ cudaError_t build(GPlan &p, bool normalize, const Forms &forms, const float2 *tw
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    // Large classes of the two-pass transform run one after another, before the others: a CTA
-    // of theirs holds an SM and a fixed share of the tiles, so kernels beside it would leave
-    // some CTAs waiting for an SM. Classes below 128 (a few percent of the points of a
-    // mixed batch) run side by side after them.
+    // Classes of the two-pass transform run one after another: a CTA of theirs holds an SM, so
+    // two side by side leave each other's CTAs waiting (two cubes of 256^3, four of 128^3, ten
+    // of 64^3 and of 32^3: 725 us side by side, 666 in turn). The others, and a class of 32^3,
+    // whose launches are short, run beside them, a branch each.
+    auto in_turn = [](const SizeGroup &g) { return tiles(g.xy) && g.n > 32; };
     auto scale_of = [&](int n) { return normalize ? (float)(1.0 / ((double)n * n * n)) : 1.0f; };
-    for (auto &g : p.groups)
-      if (tiles(g.xy) && g.n >= 128 && e == cudaSuccess) e = enqueue_group(g, scale_of(g.n), tw512, cap);
     cudaEventRecord(ev.back(), cap);
+    for (auto &g : p.groups)
+      if (in_turn(g) && e == cudaSuccess) e = enqueue_group(g, scale_of(g.n), tw512, cap);
     for (size_t gi = 0; gi < p.groups.size() && e == cudaSuccess; ++gi) {
-      if (tiles(p.groups[gi].xy) && p.groups[gi].n >= 128) continue;
-      const float scale = scale_of(p.groups[gi].n);
+      if (in_turn(p.groups[gi])) continue;
       cudaStreamWaitEvent(br[gi], ev.back(), 0);
-      e = enqueue_group(p.groups[gi], scale, tw512, br[gi]);
+      e = enqueue_group(p.groups[gi], scale_of(p.groups[gi].n), tw512, br[gi]);
       cudaEventRecord(ev[gi], br[gi]);
       cudaStreamWaitEvent(cap, ev[gi], 0);
     }
@@ -226,33 +226,53 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
       }
   }
   std::lock_guard<std::mutex> lk(g_mu);
+  // What decides a class's form: its jobs, whether their signals are apart from their outputs,
+  // and whether no filter lies among the outputs (by the ranges they span).
+  struct Class {
+    int jobs = 0;
+    bool apart = true;
+    uintptr_t flo = ~(uintptr_t)0, fhi = 0, olo = ~(uintptr_t)0, ohi = 0;
+    bool filters_apart() const { return fhi <= olo || ohi <= flo; }
+  } cls[6];
+  for (unsigned j = 0; j < njobs; ++j) {
+    Class &c = cls[Forms::index(sizes[j])];
+    const uintptr_t bytes = (uintptr_t)sizes[j] * sizes[j] * sizes[j] * sizeof(float2),
+                    su = reinterpret_cast<uintptr_t>(ptrs[3 * j]), f = reinterpret_cast<uintptr_t>(ptrs[3 * j + 1]),
+                    o = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
+    ++c.jobs;
+    if (su < o + bytes && o < su + bytes) c.apart = false;
+    c.flo = std::min(c.flo, f), c.fhi = std::max(c.fhi, f + bytes);
+    c.olo = std::min(c.olo, o), c.ohi = std::max(c.ohi, o + bytes);
+  }
+  auto of_size = [&](int n) { return cls[Forms::index(n)].jobs; };
+  int classes = 0;  // sizes present, 16 aside
+  for (int i = 1; i < 6; ++i) classes += cls[i].jobs > 0;
+  // Whether tiles are the faster form of a class, given those beside it (the axis passes' CTAs
+  // are small and fill in beside other kernels). us, tiles / axis passes, with the autotuned
+  // shapes and the default ones: 32^3 alone x16 32.9 / 35.0 and 32.9 / 35.0, x20 38.5 / 39.1 and
+  // 37.5 / 37.1, x28 45.3 / 39.3 and 44.7 / 39.2, x50 64.5 / 52.1 and 64.0 / 51.6, x170 149.7 /
+  // 150.6 and 148.7 / 148.6, x300 224.8 / 258.4; 64^3 alone x1 22.7 / 28.8, x20 111.5 / 143.1. Beside
+  // each other both in tiles / both by axes: 64^3 x2 and 32^3 x1 35 / 40, x2 and x5 47 / 42, x4 and
+  // x20 70 / 61, x8 and x40 110 / 96. 64^3 beside 32^3 by axes: x12 and x12 104 / 100, x20 and x20
+  // 142 / 157; beside two of 128^3 x8 138 / 144, x12 158 / 170. One cube of 128^3 beside both by
+  // axes: 64^3 x4 and 32^3 x5 102 / 92, 32^3 x10 64 / 70, x40 96 / 90.
+  const bool few32 = of_size(32) <= 2 && of_size(128) + of_size(256) + of_size(512) == 0;
+  const bool tiles64 = classes == 1 || few32 || of_size(64) >= (of_size(32) ? 14 : 8);
+  auto in_tiles = [&](int n) {
+    if (n == 32) return few32 || (classes == 1 && (of_size(n) <= 20 || of_size(n) >= 170));
+    if (n == 64) return tiles64;
+    return n != 128 || of_size(n) > 1 || tiles64 || (of_size(64) < 2 && of_size(32) < 32);
+  };
   // The L2-staged variant (1) and the two-pass transform (3) have table modes. The latter
   // takes signals through their outputs, so a class with a job in place (or partly so) runs
-  // the former, as does every class when tensor maps are switched off.
-  // No filter of a class lies among its outputs (by the ranges they span).
-  auto filters_apart = [&](int n) {
-    uintptr_t flo = ~(uintptr_t)0, fhi = 0, olo = ~(uintptr_t)0, ohi = 0;
-    for (unsigned j = 0; j < njobs; ++j) {
-      if (sizes[j] != n) continue;
-      const uintptr_t bytes = (uintptr_t)n * n * n * sizeof(float2), f = reinterpret_cast<uintptr_t>(ptrs[3 * j + 1]),
-                      o = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
-      flo = std::min(flo, f), fhi = std::max(fhi, f + bytes);
-      olo = std::min(olo, o), ohi = std::max(ohi, o + bytes);
-    }
-    return fhi <= olo || ohi <= flo;
-  };
+  // the former, as does every class when tensor maps are switched off; one cube of 128^3
+  // runs separate passes, beside others 89 us where the staged pass takes 100.
   auto form = [&](int n) {
     const int v = get_pass_variant(n, kKindXy);
-    if (v == kXyTwoPass && tma_enabled()) {
-      const uintptr_t bytes = (uintptr_t)n * n * n * sizeof(float2);
-      bool apart = true;
-      for (unsigned j = 0; j < njobs && apart; ++j) {
-        const uintptr_t su = reinterpret_cast<uintptr_t>(ptrs[3 * j]), ou = reinterpret_cast<uintptr_t>(ptrs[3 * j + 2]);
-        if (sizes[j] == n && su < ou + bytes && ou < su + bytes) apart = false;
-      }
-      if (apart) return filters_apart(n) ? kXyTiles : kXyTilesOrdered;
-    }
+    const Class &c = cls[Forms::index(n)];
+    if (v == kXyTwoPass && tma_enabled() && c.apart && in_tiles(n)) return c.filters_apart() ? kXyTiles : kXyTilesOrdered;
     if (n < 128 || (v != 1 && v != kXyTwoPass)) return kXySeparate;
+    if (v == kXyTwoPass && n == 128 && c.jobs == 1) return kXySeparate;
     if (v == kXyTwoPass && prepare_xy_l2(n) != cudaSuccess) {  // no memory for its ring
       cudaGetLastError();
       return kXySeparate;
@@ -261,9 +281,9 @@ int uneven_grouped(const UnevenJob *jobs, unsigned njobs, const void *d_sig, con
   };
   Forms forms;
   for (int n : {32, 64, 128, 256})
-    if (std::find(sizes.begin(), sizes.end(), n) != sizes.end()) forms.of[Forms::index(n)] = form(n);
+    if (of_size(n) > 0) forms.of[Forms::index(n)] = form(n);
   // 16^3 jobs run whole, in any order
-  forms.of[0] = filters_apart(16) ? kWhole : kXySeparate;
+  forms.of[0] = of_size(16) > 0 && cls[0].filters_apart() ? kWhole : kXySeparate;
   int form_key = 0;
   for (XyForm f : forms.of) form_key = 5 * form_key + f;
   auto key = std::make_pair(sizes, (normalize ? 1 : 0) + 2 * form_key);

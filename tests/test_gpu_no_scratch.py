@@ -116,14 +116,17 @@ def test_one_small_cube(fresh, n, real):
 
 @pytest.mark.parametrize("n", [128, 256])
 def test_uneven_in_place_without_the_ring(fresh, n):
+    """Two jobs: one of 128^3 would not ask for it."""
     cg, rng = fresh, np.random.default_rng(n)
-    sig, f = _c64(rng, (n, n, n)), _c64(rng, (n, n, n))
+    sig, f = _c64(rng, (2, n, n, n)), _c64(rng, (2, n, n, n))
     s, d = torch.from_numpy(sig).cuda(), torch.from_numpy(f).cuda()
     cg.debug_fail_allocations(1)
-    cg.conv3d_uneven_device([(n, 0, 0, 0)], s, d, s, cg.NORMALIZE)
+    cg.conv3d_uneven_device([(n, i * n ** 3, i * n ** 3, i * n ** 3) for i in range(2)], s, d, s, cg.NORMALIZE)
     torch.cuda.synchronize()
     assert cg.device_status() == 0
-    assert rel_l2(conv3d(sig[None], f, "fp64", normalize=True, engine="pocketfft")[0], s.cpu().numpy()) < 1e-6
+    for i in range(2):
+        ref = conv3d(sig[i:i + 1], f[i], "fp64", normalize=True, engine="pocketfft")[0]
+        assert rel_l2(ref, s[i].cpu().numpy()) < 1e-6
 
 
 @pytest.mark.parametrize("n,b", [(32, 3), (64, 2), (128, 2), (256, 1)])
