@@ -1397,7 +1397,7 @@ struct TuneRow {
   int n;
   int choice[kPassKinds];
   double us[2][kPassKinds];
-  double us_two_pass;  // two-pass transform of a signal and its filter (N = 128, 256), else 0
+  double us_two_pass;  // two-pass transform of a signal and its filter (N = 32 to 256), else 0
 };
 static std::vector<TuneRow> g_tuned;
 

@@ -9,9 +9,10 @@
 // uploaded only when a job's buffers move. When the plan fuses the x and y passes of
 // N = 256 or 128 (L2-staged pass), that class runs filter x+y, signal x+y, fused z and
 // inverse y+x instead: three table-mode launches of the fused pass around the z launch. With
-// the two-pass transform in the plan (and no job of the class in place) it runs that: filters
-// and signals forward (signals through their outputs), middle pass into the spectra's
-// workspace, inverse.
+// the two-pass transform in the plan, no job of the class in place, and tiles the faster form
+// beside the other classes (uneven_grouped), it runs that: filters and signals forward (signals
+// through their outputs), middle pass into the spectra's workspace, inverse; such classes run
+// in turn.
 #include <cuda.h>
 #include <cuda_runtime.h>
 

@@ -203,7 +203,8 @@ void set_tma_enabled(bool on) { g_use_tma = on; }
 bool tma_enabled() { return g_use_tma; }
 
 // Every size starts with shape variant 0; x and y of N = 32 to 256 with the two-pass
-// transform, which was faster than the other forms on every working set measured.
+// transform, which was faster than the other forms on nearly every working set measured (where it
+// was not, the calls keep to those: enqueue_tp_spectrum, launch_xy_pass, uneven_grouped).
 #define CG_TWO_PASS {0, 0, 0, 0, kXyTwoPass}
 static std::atomic<int> g_variant[6][kPassKinds] = {{}, CG_TWO_PASS, CG_TWO_PASS, CG_TWO_PASS, CG_TWO_PASS, {}};
 #undef CG_TWO_PASS

@@ -138,8 +138,8 @@ __device__ __forceinline__ void tp_step_tw(uint32_t utw, uint32_t lin, int tid, 
 // Programmatic dependent launch: a CTA may start once every CTA of the kernel before it in the
 // stream has started to end, fills its tables and sets up its barriers, and touches nothing
 // that another kernel writes before tp_grid_wait(). It hides the launch and the set-up of
-// every pass but the first: 17 cubes of 32^3 25 us instead of 35, one of 128^3 41 instead of
-// 49. (Letting the next kernel in from the start, launch_dependents, changed nothing there
+// every pass but the first: 17 cubes of 32^3 21.8 us instead of 30.8, one of 128^3 44.7 instead
+// of 52.2, three of 256^3 529 instead of 538. (Letting the next kernel in from the start, launch_dependents, changed nothing there
 // and cost 4 cubes of 256^3 with their filters 909 us instead of 835.)
 __device__ __forceinline__ void tp_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -178,8 +178,8 @@ __device__ __forceinline__ uint32_t tp_tmem_warp(uint32_t tmem, int b) {
 // tiles drift apart. A forward pass of 32 cubes of 256^3 then took 123 us a cube and filter
 // where one of 8 took 91, and the inverse 51 a cube; claimed 85 and 42. At N = 32 and 64 runs
 // are whole lines, and the claims of so many small tiles cost more than they give (17 cubes
-// of 32^3 64 us instead of 25). One counter per size and
-// pass (kernels of one size and pass never run side by side); every tile claims one successor,
+// of 32^3 64 us instead of 25, before those took their stores from the tile's own buffer). One
+// counter per size and pass (kernels of one size and pass never run side by side); every tile claims one successor,
 // so the claim that counts the last tile is the last there is and sets it back to zero. The
 // middle pass between them zeroes both as well, for after a pass that gave up.
 __device__ unsigned g_tp_claims[4];

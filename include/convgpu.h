@@ -119,7 +119,7 @@ typedef struct {
 /* Convolutions of different power-of-two sizes in one call (one filter per job),
  * on device pointers. Extends fpgaf_conv3D_svm_batch to uneven sizes.
  * Default: one CUDA graph, cached per sequence of job sizes, in which every size class is
- * a branch of one to seven launches over all jobs of that size; tensor maps are
+ * one to seven launches over all jobs of that size; tensor maps are
  * rebuilt only when a job's buffers move. CONVGPU_UNEVEN_QUEUE runs the batch as one
  * persistent launch fed by a device work queue of (job, pass, tile) items (at most
  * 4096 jobs), also replayed from a cached graph. Graphs and filter-spectrum workspaces
